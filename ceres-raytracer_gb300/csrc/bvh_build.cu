@@ -701,13 +701,13 @@ __device__ __forceinline__ int ref_count(const CollapseArgs& A, int ref) {
 }
 __device__ __forceinline__ int ref_first(const CollapseArgs& A, int ref) { return ref < 0 ? ~ref : A.range[ref].x; }
 
-// Quantisation grid for a node: p = lo - q, q = 2^e with (hi - lo) / q <= 252 and q >= 4 ulps of the
+// Quantisation grid for a node: p = lo - 2 q, q = 2^e with (hi - lo) / q <= 250 and q >= 4 ulps of the
 // largest coordinate; every child box is widened by one quantum on each side, so the decoded FP32
 // planes enclose the FP32 triangles with a margin of at least 4 ulps.
 __device__ void node_grid(const float lo[3], const float hi[3], float p[3], int ex[3]) {
     for (int k = 0; k < 3; ++k) {
         const double ext = (double)hi[k] - (double)lo[k];
-        int e = ext > 0 ? (int)ceil(log2(ext / 252.0)) : -126;
+        int e = ext > 0 ? (int)ceil(log2(ext / 250.0)) : -126;
         const float m = fmaxf(fabsf(lo[k]), fabsf(hi[k]));
         int em = -126;
         if (m > 0.f) {
@@ -719,7 +719,7 @@ __device__ void node_grid(const float lo[3], const float hi[3], float p[3], int 
         e = max(e, -126);
         e = min(e, 127);
         ex[k] = e;
-        p[k] = __double2float_rd((double)lo[k] - ldexp(1.0, e));
+        p[k] = __double2float_rd((double)lo[k] - ldexp(2.0, e));
     }
 }
 
@@ -862,32 +862,29 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ frontier, ui
     float p[3];
     int ex[3];
     node_grid(lo, hi, p, ex);
-    uint8_t meta[8], qlo[3][8], qhi[3][8];
-    uint32_t rank = 0;
+    uint8_t qlo[3][8], qhi[3][8];
+    uint32_t rank = 0, tri_valid = 0;
     for (int s = 0; s < 8; ++s) {
         const int k = child_in[s];
         if (k < 0) {
-            meta[s] = 0;
             for (int a = 0; a < 3; ++a) { qlo[a][s] = 0xFF; qhi[a][s] = 0; }
             continue;
         }
         for (int a = 0; a < 3; ++a) {
             const double iq = ldexp(1.0, -ex[a]);   // 1 / 2^ex, exact: the products equal the quotients
-            double l = floor(((double)clo[k][a] - (double)p[a]) * iq);
-            double h = ceil(((double)chi[k][a] - (double)p[a]) * iq);
-            l -= 1.0;
-            h += 1.0;
+            // an even child's planes read 0.71875 .. 0.75 quanta above the byte (WideNode)
+            const bool even = !(s & 1);
+            double l = floor(((double)clo[k][a] - (double)p[a]) * iq - (even ? 1.75 : 1.0));
+            double h = ceil(((double)chi[k][a] - (double)p[a]) * iq + (even ? 1.0 - 0.71875 : 1.0));
             if (l < 0 || h > 255) atomicOr(A.err, (uint32_t)DEVERR_QUANT_RANGE);
             qlo[a][s] = (uint8_t)fmax(0.0, fmin(255.0, l));
             qhi[a][s] = (uint8_t)fmax(0.0, fmin(255.0, h));
         }
         if (imask & (1u << s)) {
-            meta[s] = (uint8_t)((1u << 5) | (24u + s));
             next[atomicAdd(&A.counters[2], 1u)] = make_int2(refs[k], (int)(child_base + rank));
             ++rank;
         } else {
-            const uint32_t unary = (1u << cnt[k]) - 1u;
-            meta[s] = (uint8_t)((unary << 5) | (uint32_t)tri_off[s]);
+            tri_valid |= ((1u << cnt[k]) - 1u) << (3 * s);
             for (int m = 0; m < cnt[k]; ++m) {
                 const uint32_t slot = tri_base + tri_off[s] + m;
                 const uint32_t prim = A.sorted[first[k] + m];
@@ -904,19 +901,16 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ frontier, ui
             }
         }
     }
-    auto pack4 = [](const uint8_t* b) {
-        return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
-    };
     WideNode w;
-    const uint32_t eword = ((uint32_t)(uint8_t)(int8_t)ex[0]) | ((uint32_t)(uint8_t)(int8_t)ex[1] << 8) |
-                           ((uint32_t)(uint8_t)(int8_t)ex[2] << 16) | (imask << 24);
+    const uint32_t eword = ((uint32_t)(ex[0] + 127) << 23) | ((uint32_t)(ex[1] + 127) << 15) |
+                           ((uint32_t)(ex[2] + 127) << 7);
     w.w[0] = make_float4(p[0], p[1], p[2], __uint_as_float(eword));
-    w.w[1] = make_float4(__uint_as_float(child_base), __uint_as_float(tri_base), __uint_as_float(pack4(meta)),
-                         __uint_as_float(pack4(meta + 4)));
-    // planes: per axis 8 halves 0x5C00 | q (= 256 + q / 4), lo x/y/z then hi x/y/z
+    w.w[1] = make_float4(__uint_as_float(child_base), __uint_as_float(tri_base),
+                         __uint_as_float(tri_valid | (imask << 24)), 0.f);
+    // planes: per axis 4 words of two children, lo x/y/z then hi x/y/z
     auto pack_h = [](const uint8_t* b) {
         uint32_t v[4];
-        for (int j = 0; j < 4; ++j) v[j] = (0x5C00u | b[2 * j]) | ((0x5C00u | b[2 * j + 1]) << 16);
+        for (int j = 0; j < 4; ++j) v[j] = 0x43800000u | ((uint32_t)b[2 * j] << 15) | 0x5C00u | ((uint32_t)b[2 * j + 1] << 2);
         return make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
     };
     for (int a = 0; a < 3; ++a) {

@@ -148,15 +148,17 @@ int crt_guard(crt_context* ctx, F&& f) {
 
 // ------------------------------------------------------------------ scene
 // 8-wide compressed node, 128 bytes = 8 x float4:
-//  w0: origin p (float x3), exponents ex/ey/ez (int8) + imask (uint8)
-//  w1: child_base (uint32), tri_base (uint32), meta[0..7] (uint8)
-//  w2..w4: qlo_x[8], qlo_y[8], qlo_z[8]     w5..w7: qhi_x[8], qhi_y[8], qhi_z[8]
-//  each plane q (0..255, in quanta 2^e from p) stored as the half 0x5C00 | q = 256 + q / 4: the
-//  traversal converts it with one half-to-float conversion on the FMA pipe, where a byte extraction
-//  (PRMT) would load the ALU pipe that the slab test's min / max already keeps busy.
-// meta per slot: 0 = empty; internal child: (1 << 5) | (24 + slot);
-//                leaf: (unary triangle count << 5) | offset from tri_base (< 24).
-// Internal children are stored contiguously from child_base in slot order.
+//  w0: origin p (float x3), exponents of the quanta 2^e per axis: (e + 127) << 23 | << 15 | << 7 for x, y, z
+//  w1: child_base (uint32), tri_base (uint32), child bits (uint32): bit 3 s + m set when the leaf in slot
+//      s has a triangle m (0..2), bit 24 + s when slot s is an internal child; unused
+//  w2..w4: lo planes x, y, z     w5..w7: hi planes x, y, z
+//  Each row of 8 planes q (0..255, in quanta from p) is four words, word j for the children 2 j (a) and
+//  2 j + 1 (b): 0x43800000 | a << 15 | 0x5C00 | b << 2.  As a float the word is 256 + a + n, where the
+//  low half adds n = 0.71875 .. 0.75 quanta, so a is read without any decoding; the build chooses a for
+//  that value.  The low half, its sign bit (the lowest of a) dropped, is the half 256 + b: one conversion
+//  on the FMA pipe.  Both then take the same fma, t = fma(256 + q, s, d - 256 s).
+// A leaf holds 1..3 triangles, stored contiguously from tri_base in slot order; internal children are stored contiguously from child_base in slot order; an empty slot has no bit and
+// its lo planes lie above its hi planes.
 struct WideNode {
     float4 w[8];
 };

@@ -293,6 +293,7 @@ struct PrimaryJobT {
 };
 
 struct ShadowJob {
+    static constexpr int kMinBlocks = 7;   // trace_min_blocks
     Batch B;
     struct Item {
         uint32_t req, k;
@@ -317,6 +318,7 @@ struct ShadowJob {
 };
 
 struct BounceJob {
+    static constexpr int kMinBlocks = 7;
     Batch B;
     const uint32_t* q;
     struct Item {

@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
 
 // continuing rays of a device stage descriptor's range
 struct SrpBounceJobDev {
+    static constexpr int kMinBlocks = 7;   // trace_min_blocks
     const SrpStage* S;
     const uint32_t* q;
     struct Item {

@@ -6,14 +6,9 @@
 
 #include <type_traits>
 
-#ifndef CRT_TRACE_BLOCK
-#define CRT_TRACE_BLOCK 128
-#endif
-// resident blocks per SM the trace kernel is compiled for (registers per thread: 65536 / (128 x 7),
-// 72 after allocation granularity).  With the half-precision plane rows of the 8-wide node, 8 blocks
-// (64 registers) spill in the traversal loop and lose more than the eighth block's warps bring.
+// resident blocks per SM the trace kernel is compiled for (registers per thread: 65536 / (128 x 8) = 64).
 #ifndef CRT_TRACE_MIN_BLOCKS
-#define CRT_TRACE_MIN_BLOCKS 7
+#define CRT_TRACE_MIN_BLOCKS 8
 #endif
 
 __host__ __device__ __forceinline__ SceneView scene_view(const crt_scene* s) {
@@ -87,9 +82,9 @@ struct JobBase {
 // left so that the last grabs stay small (few atomics on the queue counter while much work is left,
 // balance at the end).
 // Resident blocks per SM for one job type: CRT_TRACE_MIN_BLOCKS unless the job names its own
-// (kMinBlocks).  crt_trace_closest's job runs 5 % faster at 6 blocks (80 registers); the any-hit,
-// LiDAR, pass and render jobs measured the same or slower there.  launch_trace sizes the persistent
-// grid from the occupancy the kernel gets.
+// (kMinBlocks): jobs whose rays come with a scene of their own and a skipped triangle need more
+// registers than 8 blocks leave and spill there (a 2048^2 render with its shadow rays at 8 blocks 1583
+// us, at 7 1560 us).  launch_trace sizes the persistent grid from the occupancy the kernel gets.
 template <class J, class = void>
 struct trace_min_blocks {
     static constexpr int value = CRT_TRACE_MIN_BLOCKS;
@@ -104,7 +99,7 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
                                                             const uint32_t* __restrict__ n_dev,
                                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ err,
                                                             unsigned long long* __restrict__ counters, uint32_t chunk) {
-    extern __shared__ uint2 sstack[];
+    extern __shared__ __align__(16) unsigned char trace_smem[];
     if (n_dev) n_items = *n_dev;   // item count produced by an earlier kernel on the stream
     const int lane = threadIdx.x & 31;
     TravStats st{0u, 0u};
@@ -123,13 +118,13 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
         base = __shfl_sync(0xffffffffu, base, 0);
         take = __shfl_sync(0xffffffffu, take, 0);
         if (base >= n_items) break;
-        for (uint32_t c = 0; c < take; ++c) {
-            const uint32_t i = base + 32u * c + lane;
+        for (const uint32_t end = base + 32u * take; base != end; base += 32u) {
+            const uint32_t i = base + lane;
             TRay r;
             typename Job::Item it;
             const int kind = i < n_items ? (int)job.ray(i, r, it) : 0;
             if (kind == 1) {
-                const THit h = traverse<ANY, COUNT>(job.view(sv, it), r, sstack + threadIdx.x, CRT_TRACE_BLOCK, st, err);
+                const THit h = traverse<ANY, COUNT>(job.view(sv, it), r, trace_smem, st, err);
                 job.write(sv, i, r, h, it);
             }
             if (COUNT) {
@@ -162,7 +157,7 @@ void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
                   const uint32_t* n_dev = nullptr, uint32_t* queue = nullptr, uint32_t chunk_override = 0) {
     if (!queue) queue = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
     CRT_CUDA(cudaMemsetAsync(queue, 0, sizeof(uint32_t), ctx->stream));
-    const size_t smem = (size_t)CRT_STACK_SMEM * CRT_TRACE_BLOCK * sizeof(uint2);
+    const size_t smem = TRACE_SMEM;
     const void* kfn = ctx->counting ? (const void*)k_trace<ANY, true, Job> : (const void*)k_trace<ANY, false, Job>;
     int grid = occupancy_grid(ctx, kfn, CRT_TRACE_BLOCK, smem);
     const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;

@@ -6,8 +6,19 @@
 // (the reference's "eager" leaves); internal children are visited nearest-first by the octant
 // order fixed at build time.  Node groups (base index, hit bits, slot mask) live on a per-thread
 // stack whose first STACK_SMEM entries are in shared memory and the rest in local memory.  The
-// triangle test is watertight (tri_test); the child-box test reads the node's planes as halves
-// (WideNode), so the ray octant picks each axis's entry / exit row by address.
+// triangle test is watertight (tri_test); the child-box test reads the node's planes two to a word
+// (WideNode), and the ray octant picks each axis's entry / exit row by address.
+//
+// What bounds it: instruction issue (and, for incoherent rays, the L1 data pipe and its latency).  The
+// node test is therefore written for few instructions: half of the planes need no decoding, two planes
+// take one packed fma, a child's hit is one sign bit shifted into a mask, and the triangles of all leaf
+// children that were hit come from that mask by four multiplies and masks.  Against planes as halves
+// with one conversion and one fma each, and a byte of slot / triangle bits looked up per child: 18 - 23 %
+// fewer instructions, and the kernel then waits for memory more than for issue slots (0.60 -> 0.53 of a
+// slot used per cycle on incoherent rays), so it runs as many warps as it can (8 blocks per SM, below).
+// Together, before / after: 3 M incoherent closest-hit rays on 2 M triangles 1942 / 1742 us, 333 k any-hit
+// rays on 100 k 125 / 120 us, a 1024^2 beam scan 236 / 211 us, a 2048^2 render 1860 / 1625 us, 12 x 2048^2
+// sun rays 3260 / 3070 us.
 #pragma once
 
 #include "common.cuh"
@@ -15,6 +26,9 @@
 
 #ifndef CRT_STACK_SMEM
 #define CRT_STACK_SMEM 8
+#endif
+#ifndef CRT_TRACE_BLOCK
+#define CRT_TRACE_BLOCK 128   // threads of a trace block (the strides of its shared memory)
 #endif
 #define CRT_STACK_TOTAL 64   // > wide-tree depth bound (binary depth <= 62 with index tie-breaks)
 
@@ -32,84 +46,148 @@ struct TravStats {
     uint32_t nodes, tris;
 };
 
-// barycentrics of a hit from tri_test's weights
-__device__ __forceinline__ THit normalized(THit h, float det) {
-    const float inv = 1.0f / det;
-    h.u *= inv;
-    h.v *= inv;
-    return h;
+// Shared memory of a trace block, every array indexed by thread last (no bank conflicts): the first
+// stack entries (8 bytes each), four float4 of ray constants that only the triangle test reads, and one
+// float4 of the closest hit so far.  Keeping those 18 values out of the registers while nodes are
+// visited is what brings the kernels to 8 blocks per SM (64 registers) with little or no spilling; a
+// triangle group reads them back with four 16-byte loads.  (In registers, the beam scan's kernel spilled
+// even at 7 blocks: 243 us against 211.)
+constexpr uint32_t TRACE_RAY = 8u * CRT_STACK_SMEM * CRT_TRACE_BLOCK;   // byte offsets
+constexpr uint32_t TRACE_ROW = 16u * CRT_TRACE_BLOCK;
+constexpr uint32_t TRACE_HIT = TRACE_RAY + 4u * TRACE_ROW;
+constexpr uint32_t TRACE_SMEM = TRACE_HIT + TRACE_ROW;
+
+// volatile: the values are to live in shared memory, not in registers
+__device__ __forceinline__ void st_shared4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared4(uint32_t a) {
+    float4 r;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                 : "r"(a)
+                 : "memory");
+    return r;
 }
 
-// Plane c (0..3) of half a row (4 halves 256 + q / 4) as an exact float (one half-to-float
-// conversion).  Plane distances are then fma(256 + q / 4, 4 s, a - 1024 s) with s = quantum / d: one
-// conversion and one FFMA per plane, the node-constant offset folded into a - 1024 s, whose rounding
-// adds at most 2^-24 (|a| + 2^10 |s|), well inside the build's one-quantum slack on every child box.
-__device__ __forceinline__ float half_at2(const float2 r, int c) {
-    const float w = (c >> 1) == 0 ? r.x : r.y;
-    const __half2 h = *reinterpret_cast<const __half2*>(&w);
-    return (c & 1) ? __high2float(h) : __low2float(h);
+// A pair of floats in one 64-bit register pair, and fma of both in one instruction (fma.rn.f32x2): each
+// lane's result is that of fmaf.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
+// The planes of two neighbouring words of a row (WideNode): of the even children as the words are, of
+// the odd ones from the words' low halves, whose sign bit belongs to the even child.
+__device__ __forceinline__ f32x2 planes(float w0, float w1, bool odd) {
+    if (!odd) return pack2(w0, w1);
+    const __half h0 = __ushort_as_half((unsigned short)(__float_as_uint(w0) & 0xFFFFu));
+    const __half h1 = __ushort_as_half((unsigned short)(__float_as_uint(w1) & 0xFFFFu));
+    return pack2(__half2float(__habs(h0)), __half2float(__habs(h1)));
+}
+
+// smem: the block's TRACE_SMEM bytes.  An any-hit traversal returns the slot only.
 template <bool ANY, bool COUNT>
-__device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, uint2* __restrict__ sstack, int sstride,
-                                         TravStats& st, uint32_t* __restrict__ err) {
+__device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned char* smem, TravStats& st,
+                                         uint32_t* __restrict__ err) {
     THit hit;
     hit.slot = CRT_MISS;
     hit.t = hit.u = hit.v = 0.f;
+    uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
     // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
     // -0.0 counts as negative, consistent with safe_rcp(-0.0) < 0
     const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
                          ((__float_as_uint(ray.d.z) >> 31) << 2);
     const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
+    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
     // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative direction enters at hi)
     const int offx = (oct & 1u) ? 3 : 0, offy = (oct & 2u) ? 3 : 0, offz = (oct & 4u) ? 3 : 0;
-    TShear shear = make_shear(ray.d);
-    shear.ox = shear_proj(ray.o, shear.bx);
-    shear.oy = shear_proj(ray.o, shear.by);
+    // the internal child to visit next is the pending one whose slot differs most from the octant: per
+    // slot bit, the slots that differ from the octant in it (in the group's top byte)
+    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
+                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
+    {
+        const TShear sh = make_shear(ray.d);
+        st_shared4(own + TRACE_RAY, sh.bx.x, sh.bx.y, sh.bx.z, shear_proj(ray.o, sh.bx));
+        st_shared4(own + TRACE_RAY + TRACE_ROW, sh.by.x, sh.by.y, sh.by.z, shear_proj(ray.o, sh.by));
+        st_shared4(own + TRACE_RAY + 2 * TRACE_ROW, ray.o.x, ray.o.y, ray.o.z, __uint_as_float(ray.skip));
+        st_shared4(own + TRACE_RAY + 3 * TRACE_ROW, ray.d.x, ray.d.y, ray.d.z, ray.tmin);
+        if (!ANY) st_shared4(own + TRACE_HIT, 0.f, 0.f, 1.f, __uint_as_float(CRT_MISS));
+    }
     uint2 lstack[CRT_STACK_TOTAL - CRT_STACK_SMEM];
     int sp = 0;
     // root = slot 0 of a virtual parent whose children start at node 0
-    uint2 ngroup = make_uint2(0u, (1u << (24u + oct)) | 1u);
-    float hit_det = 1.0f;   // weight sum of the hit's barycentrics (tri_test)
-    uint2 tgroup = make_uint2(0u, 0u);
+    uint2 ngroup = make_uint2(0u, 0x01000001u);
+    uint32_t tmask = 0, tvalid = 0, tbase = 0;
     while (true) {
         // ---- leaf triangles of the last visited node
-        while (tgroup.y) {
-            const int b = __ffs(tgroup.y) - 1;
-            tgroup.y &= tgroup.y - 1;
-            const uint32_t slot = tgroup.x + (uint32_t)b;
-            if (slot == ray.skip) continue;
-            const float4* tp = sv.tris + 3ull * slot;
-            const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
-            if (COUNT) st.tris++;
-            float t, wv, ww, det;
-            if (tri_test(a, bb, c, ray, shear, t, wv, ww, det)) {
-                hit.t = t;
-                hit.u = wv;
-                hit.v = ww;
-                hit_det = det;
-                hit.slot = slot;
-                if (ANY) return normalized(hit, hit_det);
-                ray.tmax = t;
-            }
+        if (tmask) {
+            TRay r;
+            TShear shear;
+            const float4 q0 = ld_shared4(own + TRACE_RAY), q1 = ld_shared4(own + TRACE_RAY + TRACE_ROW);
+            const float4 q2 = ld_shared4(own + TRACE_RAY + 2 * TRACE_ROW), q3 = ld_shared4(own + TRACE_RAY + 3 * TRACE_ROW);
+            shear.bx = f3(q0.x, q0.y, q0.z);
+            shear.ox = q0.w;
+            shear.by = f3(q1.x, q1.y, q1.z);
+            shear.oy = q1.w;
+            r.o = f3(q2.x, q2.y, q2.z);
+            r.skip = __float_as_uint(q2.w);
+            r.d = f3(q3.x, q3.y, q3.z);
+            r.tmin = q3.w;
+            do {
+                const uint32_t low = tmask & (0u - tmask);
+                tmask ^= low;
+                const uint32_t slot = tbase + __popc(tvalid & (low - 1u));
+                if (slot == r.skip) continue;
+                const float4* tp = sv.tris + 3ull * slot;
+                const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                if (COUNT) st.tris++;
+                r.tmax = ray.tmax;
+                float t, wv, ww, det;
+                if (tri_test(a, bb, c, r, shear, t, wv, ww, det)) {
+                    if (ANY) {
+                        hit.slot = slot;
+                        return hit;
+                    }
+                    ray.tmax = t;
+                    st_shared4(own + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
+                }
+            } while (tmask);
         }
         // ---- next internal node
         if (ngroup.y <= 0x00FFFFFFu) {
             if (sp == 0) break;
             --sp;
-            ngroup = sp < CRT_STACK_SMEM ? sstack[sp * sstride] : lstack[sp - CRT_STACK_SMEM];
+            ngroup = sp < CRT_STACK_SMEM ? sstack[sp * CRT_TRACE_BLOCK] : lstack[sp - CRT_STACK_SMEM];
         }
-        const uint32_t bit = 31u - __clz(ngroup.y);
-        const uint32_t cslot = (bit - 24u) ^ oct;
-        const uint32_t pmask = ngroup.y & 0xFFu;
-        const uint32_t node = ngroup.x + __popc(pmask & ((1u << cslot) - 1u));
-        ngroup.y &= ~(1u << bit);
+        uint32_t cb = ngroup.y & 0xFF000000u;   // pending children; ends as the one taken
+        uint32_t pr = cb & pick2;
+        cb = pr ? pr : cb;
+        pr = cb & pick1;
+        cb = pr ? pr : cb;
+        pr = cb & pick0;
+        cb = pr ? pr : cb;
+        const uint32_t node = ngroup.x + __popc(ngroup.y & ((cb >> 24) - 1u));
+        ngroup.y ^= cb;
         if (ngroup.y > 0x00FFFFFFu) {
-            if (sp < CRT_STACK_SMEM) sstack[sp * sstride] = ngroup;
+            if (sp < CRT_STACK_SMEM) sstack[sp * CRT_TRACE_BLOCK] = ngroup;
             else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
             else {
                 atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
-                return normalized(hit, hit_det);
+                break;
             }
             ++sp;
         }
@@ -118,43 +196,61 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, uint2* _
         const float4 w0 = __ldg(np), w1 = __ldg(np + 1);
         if (COUNT) st.nodes++;
         const uint32_t ew = __float_as_uint(w0.w);
-        // 4 x quantum x 1/d per axis (the planes are stored as 256 + q / 4)
-        const float sx4 = __uint_as_float((uint32_t)(((int)(int8_t)(ew & 0xFF) + 129) << 23)) * idir.x;
-        const float sy4 = __uint_as_float((uint32_t)(((int)(int8_t)((ew >> 8) & 0xFF) + 129) << 23)) * idir.y;
-        const float sz4 = __uint_as_float((uint32_t)(((int)(int8_t)((ew >> 16) & 0xFF) + 129) << 23)) * idir.z;
-        const float ax = fmaf(-256.0f, sx4, (w0.x - ray.o.x) * idir.x);
-        const float ay = fmaf(-256.0f, sy4, (w0.y - ray.o.y) * idir.y);
-        const float az = fmaf(-256.0f, sz4, (w0.z - ray.o.z) * idir.z);
-        const uint32_t imask = ew >> 24;
-        const uint32_t meta0 = __float_as_uint(w1.z), meta1 = __float_as_uint(w1.w);
-        // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address; each half
-        // of a row (children 0-3, 4-7) is loaded when its children are tested
-        const float2* rp = reinterpret_cast<const float2*>(np);
-        uint32_t hitmask = 0;
+        const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
+        const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
+        const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
+        const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
+        const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
+        const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
+        const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+        const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+        // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
+        const float4 xn = __ldg(np + 2 + offx), xf = __ldg(np + 5 - offx), yn = __ldg(np + 3 + offy),
+                     yf = __ldg(np + 6 - offy), zn = __ldg(np + 4 + offz), zf = __ldg(np + 7 - offz);
+        // exit minus entry distance of each child: its sign bit is set where the ray misses the child
+        // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
+        // into `miss` in turn.
+        uint32_t miss = 0;
 #pragma unroll
-        for (int hlf = 0; hlf < 2; ++hlf) {
-            const float2 xl = __ldg(rp + 2 * (2 + offx) + hlf), xh = __ldg(rp + 2 * (5 - offx) + hlf);
-            const float2 yl = __ldg(rp + 2 * (3 + offy) + hlf), yh = __ldg(rp + 2 * (6 - offy) + hlf);
-            const float2 zl = __ldg(rp + 2 * (4 + offz) + hlf), zh = __ldg(rp + 2 * (7 - offz) + hlf);
+        for (int half = 1; half >= 0; --half) {   // children 4 half .. 4 half + 3: two words of each row
+            float2 gap[2];
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                const int c = 4 * hlf + cc;
-                const int k = c & 3;
-                const float tx0 = fmaf(half_at2(xl, cc), sx4, ax), tx1 = fmaf(half_at2(xh, cc), sx4, ax);
-                const float ty0 = fmaf(half_at2(yl, cc), sy4, ay), ty1 = fmaf(half_at2(yh, cc), sy4, ay);
-                const float tz0 = fmaf(half_at2(zl, cc), sz4, az), tz1 = fmaf(half_at2(zh, cc), sz4, az);
-                const float tmin = fmaxf(fmaxf(tx0, ty0), fmaxf(tz0, ray.tmin));
-                const float tmax = fminf(fminf(tx1, ty1), fminf(tz1, ray.tmax));
-                if (tmin <= tmax) {
-                    const uint32_t meta = ((c < 4 ? meta0 : meta1) >> (8 * k)) & 0xFFu;
-                    uint32_t shift = meta & 31u;
-                    if ((imask >> c) & 1u) shift ^= oct;
-                    hitmask |= (meta >> 5) << shift;
-                }
+            for (int odd = 1; odd >= 0; --odd) {
+                auto dist = [&](const float4& r, f32x2 s, f32x2 a) {
+                    return unpack2(fma2(half ? planes(r.z, r.w, odd) : planes(r.x, r.y, odd), s, a));
+                };
+                const float2 tx0 = dist(xn, sx2, ax2), tx1 = dist(xf, sx2, ax2);
+                const float2 ty0 = dist(yn, sy2, ay2), ty1 = dist(yf, sy2, ay2);
+                const float2 tz0 = dist(zn, sz2, az2), tz1 = dist(zf, sz2, az2);
+                gap[odd].x = fminf(fminf(tx1.x, ty1.x), fminf(tz1.x, ray.tmax)) -
+                             fmaxf(fmaxf(tx0.x, ty0.x), fmaxf(tz0.x, ray.tmin));
+                gap[odd].y = fminf(fminf(tx1.y, ty1.y), fminf(tz1.y, ray.tmax)) -
+                             fmaxf(fmaxf(tx0.y, ty0.y), fmaxf(tz0.y, ray.tmin));
             }
+            miss = __funnelshift_l(__float_as_uint(gap[1].y), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[0].y), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[1].x), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[0].x), miss, 1);
         }
-        ngroup = make_uint2(__float_as_uint(w1.x), (hitmask & 0xFF000000u) | imask);
-        tgroup = make_uint2(__float_as_uint(w1.y), hitmask & 0x00FFFFFFu);
+        // internal children that were hit, and the triangles of the leaf children that were hit: each
+        // child's bit spread to three, one per triangle of a leaf (ascending bits are ascending slots)
+        const uint32_t vm = __float_as_uint(w1.z);   // 24 bits of triangles, 8 of internal children
+        const uint32_t hits = ~miss;
+        uint32_t leaf3 = hits & 0xFFu;
+        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
+        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
+        leaf3 = (leaf3 * 0x5u) & 0x249249u;
+        tvalid = vm & 0x00FFFFFFu;
+        tmask = (leaf3 * 7u) & tvalid;
+        tbase = __float_as_uint(w1.y);
+        ngroup = make_uint2(__float_as_uint(w1.x), ((hits << 24) & vm) | (vm >> 24));
     }
-    return normalized(hit, hit_det);
+    if (ANY) return hit;
+    const float4 h = ld_shared4(own + TRACE_HIT);   // weights of p1 and p2, their sum with p0's, slot
+    hit.slot = __float_as_uint(h.w);
+    const float inv = 1.0f / h.z;
+    hit.t = hit.slot != CRT_MISS ? ray.tmax : 0.0f;
+    hit.u = h.x * inv;
+    hit.v = h.y * inv;
+    return hit;
 }
