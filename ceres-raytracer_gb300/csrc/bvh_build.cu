@@ -917,7 +917,8 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ frontier, ui
         w.w[2 + a] = pack_h(qlo[a]);
         w.w[5 + a] = pack_h(qhi[a]);
     }
-    A.nodes[wnode] = w;
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) A.nodes[wnode].w[r ^ (wnode & 7u)] = w.w[r];   // rows permuted (WideNode)
 }
 
 // ---------------------------------------------------------------- binned-SAH topology

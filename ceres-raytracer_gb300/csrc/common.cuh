@@ -157,6 +157,11 @@ int crt_guard(crt_context* ctx, F&& f) {
 //  low half adds n = 0.71875 .. 0.75 quanta, so a is read without any decoding; the build chooses a for
 //  that value.  The low half, its sign bit (the lowest of a) dropped, is the half 256 + b: one conversion
 //  on the FMA pipe.  Both then take the same fma, t = fma(256 + q, s, d - 256 s).
+// Row r of node i is stored at w[r ^ (i & 7)]: lanes of a warp read the same row of different nodes, and
+// in one place those rows would all lie in the same four of the L1 data pipe's 32 banks, a pass per
+// node.  Spread over the banks: 12 % fewer data-pipe passes and 13 % less time on 3 M incoherent rays
+// (1742 -> 1519 us), 333 k any-hit rays 120 -> 105 us, a 2048^2 render 1625 -> 1554 us; the permutation
+// costs no instruction per row (the row's offset is xored to the address instead of added).
 // A leaf holds 1..3 triangles, stored contiguously from tri_base in slot order; internal children are stored contiguously from child_base in slot order; an empty slot has no bit and
 // its lo planes lie above its hi planes.
 struct WideNode {

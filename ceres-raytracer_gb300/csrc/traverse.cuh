@@ -114,7 +114,8 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
     const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
     const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
     // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative direction enters at hi)
-    const int offx = (oct & 1u) ? 3 : 0, offy = (oct & 2u) ? 3 : 0, offz = (oct & 4u) ? 3 : 0;
+    // (byte offsets; the exit row is the entry row's partner, an exclusive or away)
+    const uint32_t rowx = (oct & 1u) ? 0x50u : 0x20u, rowy = (oct & 2u) ? 0x60u : 0x30u, rowz = (oct & 4u) ? 0x70u : 0x40u;
     // the internal child to visit next is the pending one whose slot differs most from the octant: per
     // slot bit, the slots that differ from the octant in it (in the group's top byte)
     const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
@@ -192,8 +193,9 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
             ++sp;
         }
         // ---- visit: test the 8 quantised child boxes
-        const float4* np = reinterpret_cast<const float4*>(sv.nodes + node);
-        const float4 w0 = __ldg(np), w1 = __ldg(np + 1);
+        const uintptr_t np = reinterpret_cast<uintptr_t>(sv.nodes + node) ^ ((node & 7u) << 4);   // rows permuted
+        auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
+        const float4 w0 = row(0x00u), w1 = row(0x10u);
         if (COUNT) st.nodes++;
         const uint32_t ew = __float_as_uint(w0.w);
         const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
@@ -205,8 +207,8 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
         const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
         const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
         // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
-        const float4 xn = __ldg(np + 2 + offx), xf = __ldg(np + 5 - offx), yn = __ldg(np + 3 + offy),
-                     yf = __ldg(np + 6 - offy), zn = __ldg(np + 4 + offz), zf = __ldg(np + 7 - offz);
+        const float4 xn = row(rowx), xf = row(rowx ^ 0x70u), yn = row(rowy), yf = row(rowy ^ 0x50u), zn = row(rowz),
+                     zf = row(rowz ^ 0x30u);
         // exit minus entry distance of each child: its sign bit is set where the ray misses the child
         // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
         // into `miss` in turn.
