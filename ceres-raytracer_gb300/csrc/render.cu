@@ -202,6 +202,7 @@ __device__ __forceinline__ bool tile_px(uint32_t i, uint32_t W, uint32_t H, uint
 // of the wave's SRP request.  Batches without SRP requests use the SRP = false instantiation.
 template <bool SRP>
 struct PrimaryJobT {
+    static constexpr bool kDeviceGroup = SRP;   // trace_device_group: waves may hold one small query only
     Batch B;
     struct Item {
         uint32_t req;

@@ -104,6 +104,7 @@ struct SrpPrimaryJob : JobBase {
 
 // continuing rays: a compacted queue of item indices (hits still land at the item's own slot)
 struct SrpBounceJob {
+    static constexpr bool kDeviceGroup = true;   // trace_device_group
     SrpWave W;
     const uint32_t* q;
     struct Item {
@@ -293,6 +294,7 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
 // continuing rays of a device stage descriptor's range
 struct SrpBounceJobDev {
     static constexpr int kMinBlocks = 7;   // trace_min_blocks
+    static constexpr bool kDeviceGroup = true;
     const SrpStage* S;
     const uint32_t* q;
     struct Item {

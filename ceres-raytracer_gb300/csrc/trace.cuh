@@ -77,10 +77,6 @@ struct JobBase {
     __device__ __forceinline__ const SceneView& view(const SceneView& sv, const Item&) const { return sv; }
 };
 
-// Persistent ray-queue kernel.  Each warp takes groups of 32 consecutive items per atomic grab: with
-// chunk == 1 one group, otherwise a guided size of up to `chunk` groups, shrinking with the work
-// left so that the last grabs stay small (few atomics on the queue counter while much work is left,
-// balance at the end).
 // Resident blocks per SM for one job type: CRT_TRACE_MIN_BLOCKS unless the job names its own
 // (kMinBlocks): jobs whose rays come with a scene of their own and a skipped triangle need more
 // registers than 8 blocks leave and spill there (a 2048^2 render with its shadow rays at 8 blocks 1583
@@ -94,35 +90,66 @@ struct trace_min_blocks<J, std::void_t<decltype(J::kMinBlocks)>> {
     static constexpr int value = J::kMinBlocks;
 };
 
+// Whether a job's launches take the group size from the item count on the device (kDeviceGroup) instead
+// of the bound known to the host: jobs whose bound is far above the usual count (specular
+// continuations of a sun-ray grid; waves of a mixed batch that hold nothing but one small query).
+// The group size then is a register of every thread, which cost 1.7 % of a 2048^2 render's traces, so
+// the other jobs go by the bound.
+template <class J, class = void>
+struct trace_device_group {
+    static constexpr bool value = false;
+};
+template <class J>
+struct trace_device_group<J, std::void_t<decltype(J::kDeviceGroup)>> {
+    static constexpr bool value = J::kDeviceGroup;
+};
+
+// Items a warp takes at a time in a launch of n items on `warps` warps: 32, one per lane, unless that
+// would leave more than half of the warps without work; then fewer, the other lanes idle.  A small
+// launch lasts as long as its slowest warp, and a warp of 32 rays is slower than its slowest ray by
+// every node and triangle that only other lanes visit.  256 rays on 20 k triangles 37 -> 21.5 us,
+// a 128^2 render 167 -> 142 us, one 250^2 sun-ray grid with two bounces 181 -> 137 us.  (Groups that also
+// shrink at the end of a large launch cost it 1 - 3 %: its last rays then take more issue slots.)
+__host__ __device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t warps) {
+    const uint32_t per = n / warps;
+    return per >= 16u ? 32u : per >= 8u ? 16u : per >= 4u ? 4u : per >= 2u ? 2u : 1u;
+}
+
+// Persistent ray-queue kernel.  Each warp takes one group of consecutive items per atomic grab, or,
+// with chunk > 1 and full groups, a guided number of up to `chunk` groups, shrinking with the work left
+// so that the last grabs stay small (few atomics on the queue counter while much work is left, balance
+// at the end).  grab: group size | chunk << 8.
 template <bool ANY, bool COUNT, class Job>
 __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value) k_trace(SceneView sv, Job job, uint32_t n_items,
                                                             const uint32_t* __restrict__ n_dev,
                                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ err,
-                                                            unsigned long long* __restrict__ counters, uint32_t chunk) {
+                                                            unsigned long long* __restrict__ counters, uint32_t grab) {
     extern __shared__ __align__(16) unsigned char trace_smem[];
     if (n_dev) n_items = *n_dev;   // item count produced by an earlier kernel on the stream
-    const int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31u;
     TravStats st{0u, 0u};
     uint32_t nrays = 0, nres = 0;
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
+    const uint32_t chunk = grab >> 8;
+    const uint32_t group = trace_device_group<Job>::value ? group_size(n_items, warps_total) : grab & 0xFFu;
     while (true) {
-        uint32_t base = 0, take = 1;
+        uint32_t base = 0, take = group;
         if (lane == 0) {
-            if (chunk > 1) {
+            if (chunk > 1 && group == 32u) {
                 const uint32_t cur = *reinterpret_cast<volatile uint32_t*>(queue);
                 const uint32_t left = cur < n_items ? (n_items - cur) >> 5 : 0u;
-                take = min(chunk, max(1u, left / (4u * warps_total)));
+                take = 32u * min(chunk, max(1u, left / (4u * warps_total)));
             }
-            base = atomicAdd(queue, 32u * take);
+            base = atomicAdd(queue, take);
         }
         base = __shfl_sync(0xffffffffu, base, 0);
         take = __shfl_sync(0xffffffffu, take, 0);
         if (base >= n_items) break;
-        for (const uint32_t end = base + 32u * take; base != end; base += 32u) {
+        for (const uint32_t end = base + ((take + 31u) & ~31u); base != end; base += 32u) {
             const uint32_t i = base + lane;
             TRay r;
             typename Job::Item it;
-            const int kind = i < n_items ? (int)job.ray(i, r, it) : 0;
+            const int kind = lane < group && i < n_items ? (int)job.ray(i, r, it) : 0;
             if (kind == 1) {
                 const THit h = traverse<ANY, COUNT>(job.view(sv, it), r, trace_smem, st, err);
                 job.write(sv, i, r, h, it);
@@ -160,15 +187,17 @@ void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
     const size_t smem = TRACE_SMEM;
     const void* kfn = ctx->counting ? (const void*)k_trace<ANY, true, Job> : (const void*)k_trace<ANY, false, Job>;
     int grid = occupancy_grid(ctx, kfn, CRT_TRACE_BLOCK, smem);
-    const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
-    if ((uint32_t)grid > need) grid = (int)std::max<uint32_t>(need, 1u);
+    // one warp per item at most (group_size)
+    const uint32_t need = std::max<uint32_t>((n_items + CRT_TRACE_BLOCK / 32 - 1) / (CRT_TRACE_BLOCK / 32), 1u);
+    if ((uint32_t)grid > need) grid = (int)need;
     const uint32_t chunk = chunk_override ? chunk_override : (ctx->queue_chunk ? ctx->queue_chunk : 1u);
+    const uint32_t grab = group_size(n_items, (uint32_t)grid * (CRT_TRACE_BLOCK / 32)) | chunk << 8;
     if (ctx->counting)
         k_trace<ANY, true, Job><<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, queue,
-                                                                             ctx->d_error, ctx->d_counters, chunk);
+                                                                             ctx->d_error, ctx->d_counters, grab);
     else
         k_trace<ANY, false, Job><<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, queue,
-                                                                              ctx->d_error, ctx->d_counters, chunk);
+                                                                              ctx->d_error, ctx->d_counters, grab);
     check_launch(ctx, "k_trace");
 }
 
