@@ -337,10 +337,16 @@ __device__ __forceinline__ void dp_child(const float* __restrict__ dp, int ref, 
         for (int i = 1; i <= 8; ++i) out[i] = v;
         return;
     }
-    const float* d = dp + 8ull * ref;
-    const float single = __ldcg(d);
-    out[1] = single;
-    for (int i = 2; i <= 8; ++i) out[i] = fminf(single, __ldcg(d + i - 1));
+    const float4* d = reinterpret_cast<const float4*>(dp + 8ull * ref);
+    const float4 a = __ldcg(d), b = __ldcg(d + 1);
+    out[1] = a.x;
+    out[2] = fminf(a.x, a.y);
+    out[3] = fminf(a.x, a.z);
+    out[4] = fminf(a.x, a.w);
+    out[5] = fminf(a.x, b.x);
+    out[6] = fminf(a.x, b.y);
+    out[7] = fminf(a.x, b.z);
+    out[8] = fminf(a.x, b.w);
 }
 
 // node boxes: 2 float4 per node; internal nodes [0, n-1), leaves [n-1, 2n-1)
@@ -414,112 +420,192 @@ constexpr int TL_WARPS = 4;
 
 __device__ __forceinline__ size_t tl_index(int n, int ref) { return ref >= 0 ? (size_t)ref : (size_t)(n - 1 + ~ref); }
 
-// depth of every internal node (root 0), by walking up the parent links
-__global__ void k_tl_depth(const int* __restrict__ parent, int n, uint8_t* __restrict__ depth) {
+// Treelet roots of one launch: the internal nodes whose depth (root 0, found by walking up the parent
+// links) is = cls (mod 7) and that hold at least three leaves, listed in any order (treelets of a launch
+// are independent).
+__global__ void k_tl_roots(const int* __restrict__ parent, const int2* __restrict__ child, int n, int cls,
+                           int* __restrict__ list, uint32_t* __restrict__ count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    int d = 0, node = i;
-    while (true) {
-        const int p = parent[node];
-        if (p < 0 || d >= 255) break;
-        node = p;
-        ++d;
+    bool root = false;
+    if (i < n - 1) {
+        int d = 0, node = i;
+        while (true) {
+            const int p = parent[node];
+            if (p < 0 || d >= 255) break;
+            node = p;
+            ++d;
+        }
+        const int2 c = child[i];
+        root = d < 255 && d % 7 == cls && (c.x >= 0 || c.y >= 0);   // 255: deeper than tracked
     }
-    depth[i] = (uint8_t)d;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, root);
+    const int lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == 0 && m) base = atomicAdd(count, (uint32_t)__popc(m));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (root) list[base + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
+// The subsets of 7 leaves by size (ascending within a size), sizes 2 .. 5, and where each size begins.
+__constant__ uint8_t TL_SUBSETS[112] = {
+    3,  5,  6,  9,  10, 12, 17, 18, 20, 24, 33, 34, 36, 40, 48, 65, 66, 68, 72, 80, 96,   // 2
+    7,  11, 13, 14, 19, 21, 22, 25, 26, 28, 35, 37, 38, 41, 42, 44, 49, 50, 52, 56, 67, 69, 70, 73, 74, 76, 81, 82,
+    84, 88, 97, 98, 100, 104, 112,   // 3
+    15, 23, 27, 29, 30, 39, 43, 45, 46, 51, 53, 54, 57, 58, 60, 71, 75, 77, 78, 83, 85, 86, 89, 90, 92, 99, 101, 102,
+    105, 106, 108, 113, 114, 116, 120,   // 4
+    31, 47, 55, 59, 61, 62, 79, 87, 91, 93, 94, 103, 107, 109, 110, 115, 117, 118, 121, 122, 124};   // 5
+
+// keeps the cheaper partition; of equal ones the larger subset
+__device__ __forceinline__ void tl_better(float& best, uint32_t& bp, float c, uint32_t P) {
+    if (c < best || (c == best && P > bp)) {
+        best = c;
+        bp = P;
+    }
+}
+
+// One warp per treelet.  What bounds it: the chain of dependent loads that grows the treelet (each
+// opened node gives the next two boxes) and the dynamic program's 1,093 partitions, both of which one
+// lane walked before; now the leaves sit in lanes, and the partitions of a size are spread over lanes
+// (one lane a subset up to size 5, four lanes a subset of 6, all lanes for 7).  500 k triangles, seven
+// launches: 2516 -> 632 us.
 __global__ void __launch_bounds__(32 * TL_WARPS) k_treelet(int2* __restrict__ child, int* __restrict__ parent,
-                                                          float4* __restrict__ nbox,
-                                                          const uint8_t* __restrict__ depth, int n, int cls,
-                                                          uint32_t* __restrict__ stats) {
+                                                          float4* __restrict__ nbox, const int* __restrict__ list,
+                                                          const uint32_t* __restrict__ count, int n) {
     __shared__ float s_area[TL_WARPS][128];
     __shared__ float s_cost[TL_WARPS][128];
     __shared__ uint8_t s_part[TL_WARPS][128];
     __shared__ float s_box[TL_WARPS][TL_LEAVES][6];
     __shared__ int s_leaf[TL_WARPS][TL_LEAVES];
     __shared__ int s_int[TL_WARPS][TL_LEAVES - 1];
-    __shared__ int s_nl[TL_WARPS];
-    __shared__ float s_old[TL_WARPS];
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int warps = gridDim.x * TL_WARPS;
-    uint32_t improved = 0;
-    for (int R = blockIdx.x * TL_WARPS + w; R < n - 1; R += warps) {
-        if (depth[R] == 255 || (int)depth[R] % 7 != cls) continue;   // warp-uniform; 255: deeper than tracked
-        if (lane == 0) {
-            // grow the treelet: open the leaf of largest area that is an internal node
-            int leaf[TL_LEAVES], nl = 2, ni = 1;
-            float area[TL_LEAVES];
-            const int2 c = child[R];
-            leaf[0] = c.x;
-            leaf[1] = c.y;
-            s_int[w][0] = R;
-            float old = box_area(nbox[2 * (size_t)R], nbox[2 * (size_t)R + 1]);
-            for (int k = 0; k < 2; ++k) area[k] = leaf[k] >= 0 ? box_area(nbox[2 * tl_index(n, leaf[k])], nbox[2 * tl_index(n, leaf[k]) + 1]) : -1.f;
-            while (nl < TL_LEAVES) {
-                int best = -1;
-                float ba = -1.f;
-                for (int k = 0; k < nl; ++k)
-                    if (leaf[k] >= 0 && area[k] > ba) { ba = area[k]; best = k; }
-                if (best < 0) break;
-                const int L = leaf[best];
-                s_int[w][ni++] = L;
-                old += ba;
-                const int2 cc = child[L];
-                leaf[best] = cc.x;
-                leaf[nl] = cc.y;
-                area[best] = cc.x >= 0 ? box_area(nbox[2 * tl_index(n, cc.x)], nbox[2 * tl_index(n, cc.x) + 1]) : -1.f;
-                area[nl] = cc.y >= 0 ? box_area(nbox[2 * tl_index(n, cc.y)], nbox[2 * tl_index(n, cc.y) + 1]) : -1.f;
-                ++nl;
+    const uint32_t warps = gridDim.x * TL_WARPS, todo = *count;
+    for (uint32_t item = blockIdx.x * TL_WARPS + w; item < todo; item += warps) {
+        const int R = list[item];
+        // grow the treelet: open the leaf of largest area that is an internal node (of equal ones the
+        // first); lane k holds leaf k
+        const int2 c = child[R];
+        int ref = lane == 0 ? c.x : c.y, nl = 2;
+        float4 lo, hi;
+        uint32_t key = 0;   // area of an internal leaf as an ordered integer, 0: none
+        auto load = [&]() {
+            const size_t bi = tl_index(n, ref);
+            lo = nbox[2 * bi];
+            hi = nbox[2 * bi + 1];
+            key = ref >= 0 ? __float_as_uint(box_area(lo, hi)) + 1u : 0u;
+        };
+        if (lane < 2) load();
+        float old = box_area(nbox[2 * (size_t)R], nbox[2 * (size_t)R + 1]);
+        if (lane == 0) s_int[w][0] = R;
+        while (nl < TL_LEAVES) {
+            const uint32_t top = __reduce_max_sync(ALL, key);
+            if (!top) break;
+            const int best = __ffs(__ballot_sync(ALL, key == top)) - 1;
+            const int L = __shfl_sync(ALL, ref, best);
+            old += __uint_as_float(top - 1u);
+            const int2 cc = child[L];
+            if (lane == 0) s_int[w][nl - 1] = L;
+            if (lane == best || lane == nl) {
+                ref = lane == best ? cc.x : cc.y;
+                load();
             }
-            for (int k = 0; k < nl; ++k) {
-                s_leaf[w][k] = leaf[k];
-                const size_t bi = tl_index(n, leaf[k]);
-                const float4 lo = nbox[2 * bi], hi = nbox[2 * bi + 1];
-                s_box[w][k][0] = lo.x; s_box[w][k][1] = lo.y; s_box[w][k][2] = lo.z;
-                s_box[w][k][3] = hi.x; s_box[w][k][4] = hi.y; s_box[w][k][5] = hi.z;
-            }
-            s_nl[w] = nl;
-            s_old[w] = old;
+            ++nl;
+        }
+        if (nl < 3) continue;   // uniform: two triangles
+        if (lane < nl) {
+            s_leaf[w][lane] = ref;
+            s_box[w][lane][0] = lo.x; s_box[w][lane][1] = lo.y; s_box[w][lane][2] = lo.z;
+            s_box[w][lane][3] = hi.x; s_box[w][lane][4] = hi.y; s_box[w][lane][5] = hi.z;
         }
         __syncwarp();
-        const int nl = s_nl[w];
-        if (nl < 3) {
-            __syncwarp();
-            continue;
-        }
         const uint32_t full = (1u << nl) - 1u;
-        // surface area of the union of each subset's boxes
-        for (uint32_t S = lane + 1; S <= full; S += 32) {
-            float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-            for (int k = 0; k < nl; ++k)
-                if ((S >> k) & 1u)
-                    for (int a = 0; a < 3; ++a) {
-                        lo[a] = fminf(lo[a], s_box[w][k][a]);
-                        hi[a] = fmaxf(hi[a], s_box[w][k][3 + a]);
+        {   // surface area of the union of each subset's boxes: lane takes subsets lane, lane + 32, ...
+            float ulo[4][3], uhi[4][3];
+            for (int q = 0; q < 4; ++q)
+                for (int a = 0; a < 3; ++a) {
+                    ulo[q][a] = 3.0e38f;
+                    uhi[q][a] = -3.0e38f;
+                }
+            for (int k = 0; k < nl; ++k) {
+                const float b0 = s_box[w][k][0], b1 = s_box[w][k][1], b2 = s_box[w][k][2];
+                const float b3 = s_box[w][k][3], b4 = s_box[w][k][4], b5 = s_box[w][k][5];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (((uint32_t)(lane + 32 * q) >> k) & 1u) {
+                        ulo[q][0] = fminf(ulo[q][0], b0); ulo[q][1] = fminf(ulo[q][1], b1); ulo[q][2] = fminf(ulo[q][2], b2);
+                        uhi[q][0] = fmaxf(uhi[q][0], b3); uhi[q][1] = fmaxf(uhi[q][1], b4); uhi[q][2] = fmaxf(uhi[q][2], b5);
                     }
-            const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-            s_area[w][S] = dx * dy + dy * dz + dz * dx;
-            s_cost[w][S] = 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float dx = uhi[q][0] - ulo[q][0], dy = uhi[q][1] - ulo[q][1], dz = uhi[q][2] - ulo[q][2];
+                s_area[w][lane + 32 * q] = dx * dy + dy * dz + dz * dx;
+                s_cost[w][lane + 32 * q] = 0.f;
+            }
         }
         __syncwarp();
-        // cost of the best subtree over each subset, by subset size
-        for (int size = 2; size <= nl; ++size) {
-            for (uint32_t S = lane + 1; S <= full; S += 32) {
-                if (__popc(S) != size) continue;
-                const uint32_t low = S & (0u - S);
+        // cost of the best subtree over each subset, by subset size.  A partition is (P, S ^ P) with P
+        // holding the lowest leaf of S.
+        const float* cost = s_cost[w];
+        constexpr int begin[4] = {0, 21, 56, 91}, end[4] = {21, 56, 91, 112};
+#pragma unroll 1
+        for (int size = 2; size <= min(nl, 5); ++size) {
+            for (int t = begin[size - 2] + lane; t < end[size - 2]; t += 32) {
+                const uint32_t S = TL_SUBSETS[t];
+                if (S > full) continue;
+                const uint32_t low = S & (0u - S), rest = S ^ low;
                 float best = 3.0e38f;
                 uint32_t bp = low;
-                for (uint32_t P = (S - 1) & S; P; P = (P - 1) & S) {
-                    if (!(P & low)) continue;
-                    const float c = s_cost[w][P] + s_cost[w][S ^ P];
-                    if (c < best) { best = c; bp = P; }
+                for (uint32_t Q = rest; Q;) {
+                    Q = (Q - 1) & rest;
+                    const float v = cost[Q | low] + cost[rest ^ Q];
+                    if (v < best) {
+                        best = v;
+                        bp = Q | low;
+                    }
                 }
                 s_cost[w][S] = s_area[w][S] + best;
                 s_part[w][S] = (uint8_t)bp;
             }
             __syncwarp();
         }
-        if (lane == 0 && s_cost[w][full] < s_old[w] * (1.0f - 1e-5f)) {
+        if (nl >= 6) {   // subsets of 6: all leaves but leaf m; four lanes each
+            const uint32_t m = (uint32_t)lane >> 2, S = 127u ^ (1u << m);
+            const bool on = lane < 28 && S <= full;
+            float best = 3.0e38f;
+            uint32_t bp = S & (0u - S);
+            if (on) {
+                const uint32_t low = bp, rest = S ^ low;
+                const int sh = m == 0 ? 2 : 1;
+                for (uint32_t j = lane & 3; j < 31u; j += 4) {   // the j-th proper subset of rest
+                    uint32_t Q = j << sh;
+                    if (m > 0) Q = (Q & ((1u << m) - 1u)) | ((Q >> m) << (m + 1));
+                    tl_better(best, bp, cost[Q | low] + cost[rest ^ Q], Q | low);
+                }
+            }
+            for (int o = 1; o < 4; o <<= 1) tl_better(best, bp, __shfl_xor_sync(ALL, best, o), __shfl_xor_sync(ALL, bp, o));
+            __syncwarp();
+            if (on && (lane & 3) == 0) {
+                s_cost[w][S] = s_area[w][S] + best;
+                s_part[w][S] = (uint8_t)bp;
+            }
+            __syncwarp();
+        }
+        if (nl == 7) {   // all leaves: 63 partitions over the warp
+            float best = 3.0e38f;
+            uint32_t bp = 1u;
+            for (uint32_t j = lane; j < 63u; j += 32) {
+                const uint32_t Q = j << 1;
+                tl_better(best, bp, cost[Q | 1u] + cost[126u ^ Q], Q | 1u);
+            }
+            for (int o = 1; o < 32; o <<= 1) tl_better(best, bp, __shfl_xor_sync(ALL, best, o), __shfl_xor_sync(ALL, bp, o));
+            if (lane == 0) {
+                s_cost[w][127] = s_area[w][127] + best;
+                s_part[w][127] = (uint8_t)bp;
+            }
+            __syncwarp();
+        }
+        if (lane == 0 && s_cost[w][full] < old * (1.0f - 1e-5f)) {
             // rebuild: internal nodes reuse the treelet's indices (R stays the root)
             uint32_t stk_s[TL_LEAVES], ord_s[TL_LEAVES];
             int stk_n[TL_LEAVES], ord_n[TL_LEAVES];
@@ -559,11 +645,9 @@ __global__ void __launch_bounds__(32 * TL_WARPS) k_treelet(int2* __restrict__ ch
                 nbox[2 * (size_t)ord_n[k]] = make_float4(lo[0], lo[1], lo[2], 0.f);
                 nbox[2 * (size_t)ord_n[k] + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
             }
-            ++improved;
         }
         __syncwarp();
     }
-    if (stats && lane == 0 && improved) atomicAdd(stats, improved);
 }
 
 // boxes only (the treelet pass reads node areas): second arrival at each node does the union
@@ -686,7 +770,7 @@ struct CollapseArgs {
     uint32_t* leaf_prim;
     float4* leaf_vn;
     uint32_t* leaf_entity;
-    uint32_t* counters;           // [0] wide nodes used, [1] triangles placed, [2] next frontier size
+    uint32_t* counters;           // [0] wide nodes used, [1] triangles placed
     uint32_t node_cap;
     uint32_t* err;
     const float* dp;              // collapse costs from k_refit
@@ -694,231 +778,276 @@ struct CollapseArgs {
 };
 
 __device__ __forceinline__ size_t box_index(int n, int ref) { return ref >= 0 ? (size_t)ref : (size_t)(n - 1 + ~ref); }
-__device__ __forceinline__ int ref_count(const CollapseArgs& A, int ref) {
-    if (ref < 0) return 1;
-    int2 r = A.range[ref];
-    return r.y - r.x + 1;
-}
-__device__ __forceinline__ int ref_first(const CollapseArgs& A, int ref) { return ref < 0 ? ~ref : A.range[ref].x; }
 
-// Quantisation grid for a node: p = lo - 2 q, q = 2^e with (hi - lo) / q <= 250 and q >= 4 ulps of the
-// largest coordinate; every child box is widened by one quantum on each side, so the decoded FP32
-// planes enclose the FP32 triangles with a margin of at least 4 ulps.
-__device__ void node_grid(const float lo[3], const float hi[3], float p[3], int ex[3]) {
-    for (int k = 0; k < 3; ++k) {
-        const double ext = (double)hi[k] - (double)lo[k];
-        int e = ext > 0 ? (int)ceil(log2(ext / 250.0)) : -126;
-        const float m = fmaxf(fabsf(lo[k]), fabsf(hi[k]));
-        int em = -126;
-        if (m > 0.f) {
-            int fe;
-            frexpf(m, &fe);          // m in [2^(fe-1), 2^fe)
-            em = fe - 1 - 23 + 2;    // 4 ulps
-        }
-        e = max(e, em);
-        e = max(e, -126);
-        e = min(e, 127);
-        ex[k] = e;
-        p[k] = __double2float_rd((double)lo[k] - ldexp(2.0, e));
+// Quantisation grid of a node along one axis: p = lo - 2 q, q = 2^e with (hi - lo) / q <= 250 and q >= 4
+// ulps of the largest coordinate; every child box is widened by one quantum on each side, so the decoded
+// FP32 planes enclose the FP32 triangles with a margin of at least 4 ulps.
+__device__ __forceinline__ void node_grid(float lo, float hi, float& p, int& ex) {
+    const double ext = ((double)hi - (double)lo) / 250.0;
+    int e = -126;
+    if (ext > 0) {   // the least e with 2^e >= ext
+        const double f = frexp(ext, &e);   // ext = f 2^e, f in [0.5, 1)
+        if (f == 0.5) --e;
     }
+    const float m = fmaxf(fabsf(lo), fabsf(hi));
+    int em = -126;
+    if (m > 0.f) {
+        int fe;
+        frexpf(m, &fe);          // m in [2^(fe-1), 2^fe)
+        em = fe - 1 - 23 + 2;    // 4 ulps
+    }
+    ex = min(max(max(e, em), -126), 127);
+    p = __double2float_rd((double)lo - ldexp(2.0, ex));
 }
 
-__global__ void k_collapse(CollapseArgs A, const int2* __restrict__ frontier, uint32_t fcount,
-                           int2* __restrict__ next) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= fcount) return;
-    const int bnode = frontier[t].x;       // binary internal node (or ~0 for the 1-leaf root)
-    const uint32_t wnode = (uint32_t)frontier[t].y;
+// One level of the collapse: eight lanes per wide node (fcount[0] nodes in `frontier`; the next level's are
+// appended to `next` and counted in fcount[1]).  What bounds it: the chain of dependent loads of the cost
+// decisions and the copies of leaf triangles; the first levels are too small to fill the GPU, so a
+// node's own latency counts.  With one thread per node (736 bytes of local arrays) a level took 133 us
+// on 500 k triangles, 1061 us in all; with eight lanes 205 us in all.
+constexpr int COLLAPSE_BLOCK = 128;
+constexpr uint32_t COLLAPSE_MAX_LEVELS = 200;
+constexpr int ALL_TRIS = 0x7FFFFFFF;   // frontier entry of a scene of at most 3 triangles: one leaf
+
+__global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, const int2* __restrict__ frontier,
+                                                             uint32_t* __restrict__ fcount, int2* __restrict__ next) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    __shared__ int2 s_open[COLLAPSE_BLOCK];        // subtree and slots handed to another lane
+    __shared__ int s_child[COLLAPSE_BLOCK];        // lane of the child that a slot takes
+    const int lane = threadIdx.x & 31, oct0 = lane & 24, sub = lane & 7;
+    const int tid0 = threadIdx.x & ~7;
+    const uint32_t octs = gridDim.x * (COLLAPSE_BLOCK / 8), todo = *fcount;
     const int n = A.n;
+    auto oct_ballot = [&](bool b) { return (__ballot_sync(ALL, b) >> oct0) & 0xFFu; };
+    auto from = [&](auto v, int k) { return __shfl_sync(ALL, v, oct0 + k); };
+    // the warp's four nodes go through every step together (the trip count is uniform over the warp)
+    const uint32_t t0 = (blockIdx.x * COLLAPSE_BLOCK + threadIdx.x) / 32u * 4u;
+    for (uint32_t tw = t0; tw < todo; tw += octs) {
+        const uint32_t t = tw + (uint32_t)(lane >> 3);
+        const bool live = t < todo;
+        const int2 job = live ? frontier[t] : make_int2(0, 0);
+        const uint32_t wnode = (uint32_t)job.y;
 
-    int refs[8];
-    int nc = 0;
-    if (bnode == 0x7FFFFFFF) {
-        // tiny scene: the root holds one leaf with all (<= 3) triangles
-        nc = n > 0 ? 1 : 0;
-        refs[0] = 0x7FFFFFFF;
-    } else {
-        // expand by the cost decisions: a child given k slots stays one root (a leaf or an 8-wide
-        // node) unless spreading its k slots over its own children is cheaper
-        int sr[8], sk[8], sp = 0;
-        sr[sp] = bnode;
-        sk[sp++] = 8;
-        while (sp) {
-            --sp;
-            const int r = sr[sp], k = sk[sp];
-            if (r != bnode && (r < 0 || k == 1 || !(__ldg(A.dp + 8ull * r + k - 1) < __ldg(A.dp + 8ull * r)))) {
-                refs[nc++] = r;
-                continue;
-            }
-            const int2 c = A.child[r];
-            float cl[9], cr[9];
-            dp_child(A.dp, c.x, c.x < 0 ? box_area(A.nbox[2 * box_index(n, c.x)], A.nbox[2 * box_index(n, c.x) + 1]) : 0.f,
-                     A.cost_tri, cl);
-            dp_child(A.dp, c.y, c.y < 0 ? box_area(A.nbox[2 * box_index(n, c.y)], A.nbox[2 * box_index(n, c.y) + 1]) : 0.f,
-                     A.cost_tri, cr);
-            int bk = 1;
-            float best = 3.0e38f;
-            for (int kk = 1; kk < k; ++kk) {
-                const float v = cl[kk] + cr[k - kk];
-                if (v < best) {
-                    best = v;
-                    bk = kk;
+        // expand by the cost decisions: lane `sub` holds subtree `ref` with k slots (k 0: none), which
+        // occupies slots sub .. sub + k - 1; a subtree stays one child (a leaf or an 8-wide node) unless
+        // spreading its k slots over its own children is cheaper
+        int ref = job.x, k = live && sub == 0 && n > 0 ? 8 : 0;
+        bool open = k > 0 && ref != ALL_TRIS;   // the node itself is always opened
+        while (__any_sync(ALL, open)) {
+            s_open[threadIdx.x] = make_int2(0, 0);
+            __syncwarp();
+            if (open) {
+                const int2 c = A.child[ref];
+                float cl[9], cr[9];
+                dp_child(A.dp, c.x, c.x < 0 ? box_area(A.nbox[2 * box_index(n, c.x)], A.nbox[2 * box_index(n, c.x) + 1]) : 0.f,
+                         A.cost_tri, cl);
+                dp_child(A.dp, c.y, c.y < 0 ? box_area(A.nbox[2 * box_index(n, c.y)], A.nbox[2 * box_index(n, c.y) + 1]) : 0.f,
+                         A.cost_tri, cr);
+                int bk = 1;
+                float best = 3.0e38f;
+#pragma unroll
+                for (int kt = 2; kt <= 8; ++kt) {   // k as a constant, so that cl and cr stay in registers
+                    if (kt != k) continue;
+#pragma unroll
+                    for (int kk = 1; kk < kt; ++kk) {
+                        const float v = cl[kk] + cr[kt - kk];
+                        if (v < best) {
+                            best = v;
+                            bk = kk;
+                        }
+                    }
                 }
+                s_open[tid0 + sub + bk] = make_int2(c.y, k - bk);
+                ref = c.x;
+                k = bk;
             }
-            sr[sp] = c.y;
-            sk[sp++] = k - bk;
-            sr[sp] = c.x;
-            sk[sp++] = bk;
+            __syncwarp();
+            const int2 given = s_open[threadIdx.x];
+            if (given.y) {
+                ref = given.x;
+                k = given.y;
+            }
+            open = (open || given.y) && ref >= 0 && k > 1 && __ldg(A.dp + 8ull * ref + k - 1) < __ldg(A.dp + 8ull * ref);
+            __syncwarp();
         }
-    }
 
-    // child boxes, counts, first sorted positions
-    float clo[8][3], chi[8][3];
-    int cnt[8], first[8];
-    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-    for (int k = 0; k < nc; ++k) {
-        if (refs[k] == 0x7FFFFFFF) {   // all triangles
-            cnt[k] = n;
-            first[k] = 0;
-            const size_t bi = n > 1 ? 0 : (size_t)(n - 1);   // root box (internal 0) or the single leaf
-            const float4 a = A.nbox[2 * bi], b = A.nbox[2 * bi + 1];
-            clo[k][0] = a.x; clo[k][1] = a.y; clo[k][2] = a.z;
-            chi[k][0] = b.x; chi[k][1] = b.y; chi[k][2] = b.z;
-        } else {
-            cnt[k] = ref_count(A, refs[k]);
-            first[k] = ref_first(A, refs[k]);
-            if (cnt[k] < 1 || first[k] < 0 || first[k] + cnt[k] > n) {   // damaged ranges: report, read nothing
-                atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
-                return;
+        // the lane's child: box, number of triangles, first sorted position
+        const bool child = k > 0;
+        const uint32_t cmask = oct_ballot(child);
+        const int rank = __popc(cmask & ((1u << sub) - 1u));
+        float clo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, chi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+        int cnt = 0, first = 0;
+        bool bad = false;
+        if (child) {
+            size_t bi;
+            if (ref == ALL_TRIS) {
+                cnt = n;
+                bi = n > 1 ? 0 : (size_t)(n - 1);   // root box (internal 0) or the single leaf
+            } else {
+                const int2 r = ref >= 0 ? A.range[ref] : make_int2(~ref, ~ref);
+                cnt = r.y - r.x + 1;
+                first = r.x;
+                bi = box_index(n, ref);
+                bad = cnt < 1 || first < 0 || first + cnt > n;   // damaged ranges: report, read nothing
             }
-            const size_t bi = box_index(n, refs[k]);
-            const float4 a = A.nbox[2 * bi], b = A.nbox[2 * bi + 1];
-            clo[k][0] = a.x; clo[k][1] = a.y; clo[k][2] = a.z;
-            chi[k][0] = b.x; chi[k][1] = b.y; chi[k][2] = b.z;
+            if (!bad) {
+                const float4 a = A.nbox[2 * bi], b = A.nbox[2 * bi + 1];
+                clo[0] = a.x; clo[1] = a.y; clo[2] = a.z;
+                chi[0] = b.x; chi[1] = b.y; chi[2] = b.z;
+            }
         }
+        const bool node_bad = oct_ballot(bad) != 0u;
+        if (node_bad && sub == 0) atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
+        float lo[3], hi[3];
         for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], clo[k][a]);
-            hi[a] = fmaxf(hi[a], chi[k][a]);
+            lo[a] = clo[a];
+            hi[a] = chi[a];
+            for (int o = 1; o < 8; o <<= 1) {
+                lo[a] = fminf(lo[a], __shfl_xor_sync(ALL, lo[a], o));
+                hi[a] = fmaxf(hi[a], __shfl_xor_sync(ALL, hi[a], o));
+            }
+            if (!cmask) lo[a] = hi[a] = 0.f;
         }
-    }
-    if (nc == 0) {
-        for (int a = 0; a < 3; ++a) lo[a] = hi[a] = 0.f;
-    }
 
-    // slot assignment: slot s takes the child whose centroid lies farthest along
-    // D(s) = (s&1 ? -1 : 1, s&2 ? -1 : 1, s&4 ? -1 : 1) from the node centre (greedy)
-    int slot_of[8];
-    int child_in[8];
-    for (int s = 0; s < 8; ++s) child_in[s] = -1;
-    {
-        float score[8][8];
-        const float cxn = 0.5f * (lo[0] + hi[0]), cyn = 0.5f * (lo[1] + hi[1]), czn = 0.5f * (lo[2] + hi[2]);
-        for (int k = 0; k < nc; ++k) {
-            const float ox = 0.5f * (clo[k][0] + chi[k][0]) - cxn;
-            const float oy = 0.5f * (clo[k][1] + chi[k][1]) - cyn;
-            const float oz = 0.5f * (clo[k][2] + chi[k][2]) - czn;
-            for (int s = 0; s < 8; ++s)
-                score[k][s] = ((s & 1) ? -ox : ox) + ((s & 2) ? -oy : oy) + ((s & 4) ? -oz : oz);
-            slot_of[k] = -1;
-        }
-        for (int it = 0; it < nc; ++it) {
-            float best = -3.0e38f;
-            int bk = -1, bs = -1;
-            for (int k = 0; k < nc; ++k) {
-                if (slot_of[k] >= 0) continue;
+        // slot assignment: slot s takes the child whose centroid lies farthest along
+        // D(s) = (s&1 ? -1 : 1, s&2 ? -1 : 1, s&4 ? -1 : 1) from the node centre (greedy; of equal scores
+        // the first child, then the first slot)
+        const float ox = 0.5f * (clo[0] + chi[0]) - 0.5f * (lo[0] + hi[0]);
+        const float oy = 0.5f * (clo[1] + chi[1]) - 0.5f * (lo[1] + hi[1]);
+        const float oz = 0.5f * (clo[2] + chi[2]) - 0.5f * (lo[2] + hi[2]);
+        uint32_t free_slots = 0xFFu;
+        int slot = -1;
+        s_child[threadIdx.x] = -1;
+        __syncwarp();
+        for (int it = 0; it < 8; ++it) {
+            float best = -3.4e38f;
+            int what = 64;   // child's rank x 8 + slot
+            if (child && slot < 0) {
+                int bs = __ffs(free_slots) - 1;
+#pragma unroll
                 for (int s = 0; s < 8; ++s) {
-                    if (child_in[s] >= 0) continue;
-                    if (score[k][s] > best) { best = score[k][s]; bk = k; bs = s; }
+                    const float v = ((s & 1) ? -ox : ox) + ((s & 2) ? -oy : oy) + ((s & 4) ? -oz : oz);
+                    if (((free_slots >> s) & 1u) && v > best) {
+                        best = v;
+                        bs = s;
+                    }
+                }
+                what = rank * 8 + bs;
+            }
+            for (int o = 1; o < 8; o <<= 1) {
+                const float v = __shfl_xor_sync(ALL, best, o);
+                const int w = __shfl_xor_sync(ALL, what, o);
+                if (v > best || (v == best && w < what)) {
+                    best = v;
+                    what = w;
                 }
             }
-            slot_of[bk] = bs;
-            child_in[bs] = bk;
+            if (what < 64) {
+                free_slots &= ~(1u << (what & 7));
+                if (child && slot < 0 && rank == (what >> 3)) slot = what & 7;
+            }
         }
-    }
+        if (slot >= 0) s_child[tid0 + slot] = sub;
+        __syncwarp();
 
-    // leaves (<= 3 triangles) vs internal children; allocation
-    uint32_t imask = 0, n_int = 0, n_tri = 0;
-    int tri_off[8];
-    for (int s = 0; s < 8; ++s) {
-        tri_off[s] = 0;
-        const int k = child_in[s];
-        if (k < 0) continue;
-        if (cnt[k] <= 3) {
-            tri_off[s] = (int)n_tri;
-            n_tri += cnt[k];
-        } else {
-            imask |= 1u << s;
-            ++n_int;
-        }
-    }
-    uint32_t child_base = 0, tri_base = 0;
-    if (n_int) child_base = atomicAdd(&A.counters[0], n_int);
-    if (n_tri) tri_base = atomicAdd(&A.counters[1], n_tri);
-    if (child_base + n_int > A.node_cap || tri_base + n_tri > (uint32_t)n) {
-        atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
-        return;
-    }
-
-    float p[3];
-    int ex[3];
-    node_grid(lo, hi, p, ex);
-    uint8_t qlo[3][8], qhi[3][8];
-    uint32_t rank = 0, tri_valid = 0;
-    for (int s = 0; s < 8; ++s) {
-        const int k = child_in[s];
-        if (k < 0) {
-            for (int a = 0; a < 3; ++a) { qlo[a][s] = 0xFF; qhi[a][s] = 0; }
-            continue;
-        }
+        // from here lane `sub` is slot `sub`
+        const int src = s_child[threadIdx.x];
+        const bool full = src >= 0 && !node_bad;
+        const int from_lane = max(src, 0);
+        ref = from(ref, from_lane);
+        cnt = from(cnt, from_lane);
+        if (!full) cnt = 0;
+        first = from(first, from_lane);
         for (int a = 0; a < 3; ++a) {
+            clo[a] = from(clo[a], from_lane);
+            chi[a] = from(chi[a], from_lane);
+        }
+        const bool leaf = full && cnt <= 3, inner = full && cnt > 3;
+        const uint32_t imask = oct_ballot(inner);
+        const int irank = __popc(imask & ((1u << sub) - 1u));
+        const uint32_t n_int = __popc(imask);
+        uint32_t tri_off = leaf ? (uint32_t)cnt : 0u;   // triangles of the leaves in lower slots
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(ALL, tri_off, o, 8);
+            if (sub >= o) tri_off += v;
+        }
+        const uint32_t n_tri = from(tri_off, 7);
+        tri_off -= leaf ? (uint32_t)cnt : 0u;
+        uint32_t child_base = 0, tri_base = 0, next_base = 0;
+        if (sub == 0) {
+            if (n_int) {
+                child_base = atomicAdd(&A.counters[0], n_int);
+                next_base = atomicAdd(&fcount[1], n_int);
+            }
+            if (n_tri) tri_base = atomicAdd(&A.counters[1], n_tri);
+        }
+        child_base = from(child_base, 0);
+        next_base = from(next_base, 0);
+        tri_base = from(tri_base, 0);
+        const bool fits = child_base + n_int <= A.node_cap && next_base + n_int <= A.node_cap && tri_base + n_tri <= (uint32_t)n;
+        if (!fits && sub == 0) atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
+        const bool write = live && fits && !node_bad;
+
+        // child planes in quanta; lane a finds the grid of axis a
+        float p[3];
+        int ex[3];
+        {
+            float pa = 0.f;
+            int ea = 0;
+            if (sub < 3) node_grid(sub == 0 ? lo[0] : sub == 1 ? lo[1] : lo[2], sub == 0 ? hi[0] : sub == 1 ? hi[1] : hi[2], pa, ea);
+            for (int a = 0; a < 3; ++a) {
+                p[a] = from(pa, a);
+                ex[a] = from(ea, a);
+            }
+        }
+        uint32_t q[6];   // lo x, y, z, hi x, y, z
+        for (int a = 0; a < 3; ++a) {
+            q[a] = 0xFFu;
+            q[3 + a] = 0u;
+            if (!full) continue;
             const double iq = ldexp(1.0, -ex[a]);   // 1 / 2^ex, exact: the products equal the quotients
             // an even child's planes read 0.71875 .. 0.75 quanta above the byte (WideNode)
-            const bool even = !(s & 1);
-            double l = floor(((double)clo[k][a] - (double)p[a]) * iq - (even ? 1.75 : 1.0));
-            double h = ceil(((double)chi[k][a] - (double)p[a]) * iq + (even ? 1.0 - 0.71875 : 1.0));
+            const bool even = !(sub & 1);
+            const double l = floor(((double)clo[a] - (double)p[a]) * iq - (even ? 1.75 : 1.0));
+            const double h = ceil(((double)chi[a] - (double)p[a]) * iq + (even ? 1.0 - 0.71875 : 1.0));
             if (l < 0 || h > 255) atomicOr(A.err, (uint32_t)DEVERR_QUANT_RANGE);
-            qlo[a][s] = (uint8_t)fmax(0.0, fmin(255.0, l));
-            qhi[a][s] = (uint8_t)fmax(0.0, fmin(255.0, h));
+            q[a] = (uint32_t)fmax(0.0, fmin(255.0, l));
+            q[3 + a] = (uint32_t)fmax(0.0, fmin(255.0, h));
         }
-        if (imask & (1u << s)) {
-            next[atomicAdd(&A.counters[2], 1u)] = make_int2(refs[k], (int)(child_base + rank));
-            ++rank;
-        } else {
-            tri_valid |= ((1u << cnt[k]) - 1u) << (3 * s);
-            for (int m = 0; m < cnt[k]; ++m) {
-                const uint32_t slot = tri_base + tri_off[s] + m;
-                const uint32_t prim = A.sorted[first[k] + m];
-                A.tris[3ull * slot + 0] = A.geo[3ull * prim + 0];
-                A.tris[3ull * slot + 1] = A.geo[3ull * prim + 1];
-                A.tris[3ull * slot + 2] = A.geo[3ull * prim + 2];
-                A.leaf_prim[slot] = prim;
-                A.leaf_entity[slot] = A.prim_ent[prim];
+        uint32_t valid = leaf ? ((1u << cnt) - 1u) << (3 * sub) : 0u;
+        for (int o = 1; o < 8; o <<= 1) valid |= __shfl_xor_sync(ALL, valid, o);
+        uint32_t* const words = reinterpret_cast<uint32_t*>(A.nodes + wnode);
+        auto put = [&](uint32_t row, uint32_t word, uint32_t v) {   // rows permuted by node (WideNode)
+            if (write) words[4u * (row ^ (wnode & 7u)) + word] = v;
+        };
+        for (int r = 0; r < 6; ++r) {
+            const uint32_t odd = __shfl_xor_sync(ALL, q[r], 1);
+            if (!(sub & 1)) put(2u + r, (uint32_t)sub >> 1, 0x43800000u | (q[r] << 15) | 0x5C00u | (odd << 2));
+        }
+        const uint32_t eword = ((uint32_t)(ex[0] + 127) << 23) | ((uint32_t)(ex[1] + 127) << 15) |
+                               ((uint32_t)(ex[2] + 127) << 7);
+        const uint32_t head = sub == 0 ? __float_as_uint(p[0]) : sub == 1 ? __float_as_uint(p[1]) : sub == 2 ? __float_as_uint(p[2])
+                              : sub == 3 ? eword : sub == 4 ? child_base : sub == 5 ? tri_base : sub == 6 ? valid | (imask << 24) : 0u;
+        put((uint32_t)sub >> 2, (uint32_t)sub & 3u, head);
+        if (write && inner) next[next_base + irank] = make_int2(ref, (int)(child_base + irank));
+        if (write && leaf) {
+            for (int m = 0; m < cnt; ++m) {
+                const uint32_t at = tri_base + tri_off + m;
+                const uint32_t prim = A.sorted[first + m];
+                A.tris[3ull * at + 0] = A.geo[3ull * prim + 0];
+                A.tris[3ull * at + 1] = A.geo[3ull * prim + 1];
+                A.tris[3ull * at + 2] = A.geo[3ull * prim + 2];
+                A.leaf_prim[at] = prim;
+                A.leaf_entity[at] = A.prim_ent[prim];
                 if (A.vn) {
-                    A.leaf_vn[3ull * slot + 0] = A.vn[3ull * prim + 0];
-                    A.leaf_vn[3ull * slot + 1] = A.vn[3ull * prim + 1];
-                    A.leaf_vn[3ull * slot + 2] = A.vn[3ull * prim + 2];
+                    A.leaf_vn[3ull * at + 0] = A.vn[3ull * prim + 0];
+                    A.leaf_vn[3ull * at + 1] = A.vn[3ull * prim + 1];
+                    A.leaf_vn[3ull * at + 2] = A.vn[3ull * prim + 2];
                 }
             }
         }
+        __syncwarp();
     }
-    WideNode w;
-    const uint32_t eword = ((uint32_t)(ex[0] + 127) << 23) | ((uint32_t)(ex[1] + 127) << 15) |
-                           ((uint32_t)(ex[2] + 127) << 7);
-    w.w[0] = make_float4(p[0], p[1], p[2], __uint_as_float(eword));
-    w.w[1] = make_float4(__uint_as_float(child_base), __uint_as_float(tri_base),
-                         __uint_as_float(tri_valid | (imask << 24)), 0.f);
-    // planes: per axis 4 words of two children, lo x/y/z then hi x/y/z
-    auto pack_h = [](const uint8_t* b) {
-        uint32_t v[4];
-        for (int j = 0; j < 4; ++j) v[j] = 0x43800000u | ((uint32_t)b[2 * j] << 15) | 0x5C00u | ((uint32_t)b[2 * j + 1] << 2);
-        return make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
-    };
-    for (int a = 0; a < 3; ++a) {
-        w.w[2 + a] = pack_h(qlo[a]);
-        w.w[5 + a] = pack_h(qhi[a]);
-    }
-#pragma unroll
-    for (uint32_t r = 0; r < 8; ++r) A.nodes[wnode].w[r ^ (wnode & 7u)] = w.w[r];   // rows permuted (WideNode)
 }
 
 // ---------------------------------------------------------------- binned-SAH topology
@@ -1519,10 +1648,9 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     uint32_t *prim_ent = nullptr, *code_a = nullptr, *idx_a = nullptr, *code_b = nullptr, *idx_b = nullptr;
     uint32_t* code_prim = nullptr;
     float* dpc = nullptr;
-    uint32_t *hist = nullptr, *flags = nullptr, *keys = nullptr;
+    uint32_t *hist = nullptr, *flags = nullptr, *keys = nullptr, *level_count = nullptr;
     int2 *child = nullptr, *range = nullptr, *front = nullptr, *front_b = nullptr;
     int* parent = nullptr;
-    uint8_t* tl_depth = nullptr;
     int *tl_cnt = nullptr, *tl_pos = nullptr, *tl_par = nullptr;
     uint32_t* tl_sorted = nullptr;
     const size_t nb_sort = (nn + SORT_TILE - 1) / SORT_TILE;
@@ -1552,9 +1680,9 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
         nbox = (float4*)take(nn * 64);        // 2n - 1 nodes x (lo, hi)
         dpc = (float*)take(nn * 32);          // collapse costs: 8 per internal node
         keys = (uint32_t*)take(64 * 4);
+        level_count = (uint32_t*)take((COLLAPSE_MAX_LEVELS + 1) * 4);
         front = (int2*)take(nn * 8 + 8);
         front_b = (int2*)take(nn * 8 + 8);
-        tl_depth = (uint8_t*)take(nn);
         tl_cnt = (int*)take(nn * 4);
         tl_pos = (int*)take(nn * 8);          // 2n - 1 nodes
         tl_par = (int*)take(nn * 4);
@@ -1603,13 +1731,17 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
             k_tl_boxes<<<cdiv(n, BLOCK), BLOCK, 0, st>>>(va, tbox, (int)n, child, parent, nbox, flags, ctx->d_error);
             check_launch(ctx, "k_tl_boxes");
             const uint32_t tl_grid = std::min<uint32_t>(cdiv(n - 1, TL_WARPS), (uint32_t)ctx->sm_count * 16);
-            for (uint32_t pass = 0; pass < ctx->treelet_passes; ++pass)
+            // root lists (tl_pos, filled later, has room) and their lengths, one per launch
+            uint32_t* tl_count = keys + 32;
+            for (uint32_t pass = 0; pass < ctx->treelet_passes; ++pass) {
+                CRT_CUDA(cudaMemsetAsync(tl_count, 0, 7 * sizeof(uint32_t), st));
                 for (int cls = 0; cls < 7; ++cls) {
-                    k_tl_depth<<<cdiv(n - 1, BLOCK), BLOCK, 0, st>>>(parent, (int)n, tl_depth);
-                    check_launch(ctx, "k_tl_depth");
-                    k_treelet<<<tl_grid, 32 * TL_WARPS, 0, st>>>(child, parent, nbox, tl_depth, (int)n, cls, nullptr);
+                    k_tl_roots<<<cdiv(n - 1, BLOCK), BLOCK, 0, st>>>(parent, child, (int)n, cls, tl_pos, tl_count + cls);
+                    check_launch(ctx, "k_tl_roots");
+                    k_treelet<<<tl_grid, 32 * TL_WARPS, 0, st>>>(child, parent, nbox, tl_pos, tl_count + cls, (int)n);
                     check_launch(ctx, "k_treelet");
                 }
+            }
             CRT_CUDA(cudaMemsetAsync(flags, 0, nn * 4, st));
             k_tl_count<<<cdiv(n, BLOCK), BLOCK, 0, st>>>((int)n, child, parent, tl_cnt, flags, ctx->d_error);
             check_launch(ctx, "k_tl_count");
@@ -1637,9 +1769,11 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     CRT_CUDA(cudaMalloc(&s->leaf_entity, sizeof(uint32_t) * nn));
     if (any_vn) CRT_CUDA(cudaMalloc(&s->leaf_vn, sizeof(float4) * 3 * nn));
     uint32_t* counters = keys + 16;
-    const uint32_t c0[3] = {1, 0, 0};
+    const uint32_t c0[2] = {1, 0};
     CRT_CUDA(cudaMemcpyAsync(counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
-    int2 root = make_int2(n > 3 ? root_index : 0x7FFFFFFF, 0);
+    CRT_CUDA(cudaMemsetAsync(level_count, 0, sizeof(uint32_t) * (COLLAPSE_MAX_LEVELS + 1), st));
+    CRT_CUDA(cudaMemcpyAsync(level_count, c0, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    int2 root = make_int2(n > 3 ? root_index : ALL_TRIS, 0);
     CRT_CUDA(cudaMemcpyAsync(front, &root, sizeof(root), cudaMemcpyHostToDevice, st));
 
     CollapseArgs A;
@@ -1662,18 +1796,29 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     A.dp = dpc;
     A.cost_tri = ctx->collapse_tri_cost;
 
-    uint32_t fcount = 1, depth = 0;
+    // The levels are launched without waiting for their sizes, which stay on the device (level d of the
+    // tree has at most 8^d nodes): as many as a tree of this size usually has, then a look at the counts,
+    // then two at a time.
+    uint32_t depth = 0;
     int2 *cur = front, *nxt = front_b;
-    while (fcount) {
-        CRT_CUDA(cudaMemsetAsync(counters + 2, 0, sizeof(uint32_t), st));
-        k_collapse<<<cdiv(fcount, 128), 128, 0, st>>>(A, cur, fcount, nxt);
-        check_launch(ctx, "k_collapse");
-        ++depth;
-        CRT_CUDA(cudaMemcpyAsync(&fcount, counters + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    uint32_t lc_h[COLLAPSE_MAX_LEVELS + 1];
+    uint32_t launched = 0, batch = 4;
+    for (uint32_t m = n / 3; m; m /= 8) ++batch;
+    for (uint64_t bound = 1;;) {
+        CRT_CHECK(launched + batch <= COLLAPSE_MAX_LEVELS, CRT_ERR_DEVICE, "BVH collapse did not terminate");
+        for (uint32_t b = 0; b < batch; ++b, ++launched) {
+            const uint32_t grid = std::min<uint32_t>(cdiv(bound, COLLAPSE_BLOCK / 8), (uint32_t)ctx->sm_count * 16);
+            k_collapse<<<grid, COLLAPSE_BLOCK, 0, st>>>(A, cur, level_count + launched, nxt);
+            check_launch(ctx, "k_collapse");
+            std::swap(cur, nxt);
+            bound = std::min<uint64_t>(bound * 8, cap);
+        }
+        CRT_CUDA(cudaMemcpyAsync(lc_h, level_count, sizeof(uint32_t) * (launched + 1), cudaMemcpyDeviceToHost, st));
         CRT_CUDA(cudaStreamSynchronize(st));
-        std::swap(cur, nxt);
-        CRT_CHECK(depth < 200, CRT_ERR_DEVICE, "BVH collapse did not terminate");
+        if (!lc_h[launched]) break;
+        batch = 2;
     }
+    while (depth < launched && lc_h[depth]) ++depth;
     uint32_t used[2];
     CRT_CUDA(cudaMemcpyAsync(used, counters, sizeof(used), cudaMemcpyDeviceToHost, st));
     uint32_t kb_h[6] = {0, 0, 0, 0, 0, 0};
