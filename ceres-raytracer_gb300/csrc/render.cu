@@ -202,8 +202,9 @@ __device__ __forceinline__ bool tile_px(uint32_t i, uint32_t W, uint32_t H, uint
 // of the wave's SRP request.  Batches without SRP requests use the SRP = false instantiation.
 template <bool SRP>
 struct PrimaryJobT {
-    static constexpr bool kDeviceGroup = SRP;   // trace_device_group: waves may hold one small query only
+    static constexpr int kGroups = SRP ? GROUPS_DEVICE : GROUPS_HOST;   // SRP: a wave may hold one small query only
     Batch B;
+    __device__ __forceinline__ bool full_groups() const { return B.cur->n_lidar_items != 0; }
     struct Item {
         uint32_t req;
         uint32_t lidar;   // 0 camera path, 1 LiDAR beam, 2 SRP sun ray
@@ -792,12 +793,13 @@ inline uint32_t tiles_items(uint32_t W, uint32_t H) { return ((W + 7) / 8) * ((H
 // srp_items: bound on the wave's SRP items (crt_batch_mixed, serving); when non-zero the primary
 // trace also traces the wave's SRP sun rays and srp_stages (launches of the SRP shade and specular
 // segments) runs right after it.  srp_mask (when given): the SRP hit mask, zeroed before the primary
-// trace.  With srp_stages reading the wave's range from the device descriptor (srp_wave_stages_dev)
+// trace.  small_scenes: every scene of the wave has fewer than SMALL_SCENE triangles (group_size).
+// With srp_stages reading the wave's range from the device descriptor (srp_wave_stages_dev)
 // the sequence is the same for every wave and can be captured and replayed.
 void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, uint32_t lidar_items,
                          int max_bounces, uint32_t* qa, uint32_t* qb, uint32_t* tqueue, uint32_t srp_items = 0,
                          const std::function<void()>* srp_stages = nullptr, uint32_t* srp_mask = nullptr,
-                         size_t srp_mask_len = 0) {
+                         size_t srp_mask_len = 0, bool small_scenes = false) {
     cudaStream_t st = ctx->stream;
     const uint32_t g_shade = grid_for(ctx, k_shade, P), g_accum = grid_for(ctx, k_accum, P);
     const uint32_t g_update = max_bounces <= 1 ? grid_for(ctx, k_update<true>, P) : grid_for(ctx, k_update<false>, P);
@@ -807,11 +809,12 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
     if (srp_items) {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<true>{B},
                             (uint32_t)std::min<size_t>(P + lidar_items + srp_items, 0xFFFFFF00u), &B.cur->n_primary,
-                            tqueue);
+                            tqueue, small_scenes);
         if (srp_stages) (*srp_stages)();
     } else {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<false>{B},
-                            (uint32_t)std::min<size_t>(P + lidar_items, 0xFFFFFF00u), &B.cur->n_primary, tqueue);
+                            (uint32_t)std::min<size_t>(P + lidar_items, 0xFFFFFF00u), &B.cur->n_primary, tqueue,
+                            small_scenes || lidar_items > 0);
     }
     const uint32_t* q_in = nullptr;
     uint32_t* q_out = qa;
@@ -821,13 +824,13 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
                                          ctx->counting ? ctx->d_counters : nullptr);
         check_launch(ctx, "k_shade");
         launch_trace<true>(ctx, SceneView{}, ShadowJob{B}, (uint32_t)std::min<size_t>(P * NL, 0xFFFFFF00u),
-                           &B.counts[2], tqueue);
+                           &B.counts[2], tqueue, small_scenes);
         if (!fuse) {
             k_accum<<<g_accum, 256, 0, st>>>(B, b, q_in);
             check_launch(ctx, "k_accum");
         }
         if (b < max_bounces - 1) {
-            launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[1], tqueue);
+            launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[1], tqueue, small_scenes);
             k_queue_rotate<<<1, 1, 0, st>>>(B.counts);
             check_launch(ctx, "k_queue_rotate");
             q_in = q_out;
@@ -1201,7 +1204,11 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
 
     // ---- one wave: every launch reads the wave from B.cur (graph-capturable)
     uint32_t* tqueue = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
-    auto launch_wave = [&]() { launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, tqueue); };
+    bool small_scenes = n_srp == 0;
+    for (size_t i = 0; i < n; ++i) small_scenes = small_scenes && reqs[i].scene->n_tris < SMALL_SCENE;
+    auto launch_wave = [&]() {
+        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, tqueue, 0, nullptr, nullptr, 0, small_scenes);
+    };
 
     size_t waves_run = 0;
     const bool graph_ok = ctx->use_graphs && !ctx->counting && plan.size() > 1;

@@ -104,7 +104,8 @@ struct SrpPrimaryJob : JobBase {
 
 // continuing rays: a compacted queue of item indices (hits still land at the item's own slot)
 struct SrpBounceJob {
-    static constexpr bool kDeviceGroup = true;   // trace_device_group
+    static constexpr int kGroups = GROUPS_DEVICE;   // trace_groups
+    __device__ __forceinline__ bool full_groups() const { return false; }
     SrpWave W;
     const uint32_t* q;
     struct Item {
@@ -294,7 +295,8 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
 // continuing rays of a device stage descriptor's range
 struct SrpBounceJobDev {
     static constexpr int kMinBlocks = 7;   // trace_min_blocks
-    static constexpr bool kDeviceGroup = true;
+    static constexpr int kGroups = GROUPS_DEVICE;
+    __device__ __forceinline__ bool full_groups() const { return false; }
     const SrpStage* S;
     const uint32_t* q;
     struct Item {

@@ -63,6 +63,7 @@ __device__ __forceinline__ bool tile_pixel(uint32_t i, uint32_t W, uint32_t H, u
 }
 
 struct PassJob : JobBase {
+    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
     CamBasis cam;
     double* xyz;
     uint32_t* ids;
@@ -133,6 +134,7 @@ struct PassJob : JobBase {
 };
 
 struct LidarBatchJob : JobBase {
+    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
     const double* pos;
     const double* rot;
     float zsign;
@@ -163,6 +165,7 @@ struct LidarBatchJob : JobBase {
 };
 
 struct LidarGridJob : JobBase {
+    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
     double o[3];
     double rt[9];         // R^T row-major (world = rt * sensor direction)
     double zsign;

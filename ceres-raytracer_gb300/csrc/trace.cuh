@@ -90,18 +90,21 @@ struct trace_min_blocks<J, std::void_t<decltype(J::kMinBlocks)>> {
     static constexpr int value = J::kMinBlocks;
 };
 
-// Whether a job's launches take the group size from the item count on the device (kDeviceGroup) instead
-// of the bound known to the host: jobs whose bound is far above the usual count (specular
-// continuations of a sun-ray grid; waves of a mixed batch that hold nothing but one small query).
-// The group size then is a register of every thread, which cost 1.7 % of a 2048^2 render's traces, so
-// the other jobs go by the bound.
+// How a job's launches choose the items per warp (group_size): by the bound on the item count known to the
+// host, the default; by the count on the device (kGroups = GROUPS_DEVICE), for jobs whose bound is far
+// above the usual count (specular continuations of a sun-ray grid; waves of a mixed batch that hold
+// nothing but one small query; the job's full_groups() says where it has FP64 items); or always 32 (GROUPS_FULL), for jobs with FP64 work per item, which
+// takes the same time for a warp with one active lane (a 229 x 128 beam scan: 34 us, in small groups 53).
+// A group size from the device is a register of every thread, which cost 1.7 % of a 2048^2 render's
+// traces, so it is not the default.
+enum { GROUPS_HOST, GROUPS_DEVICE, GROUPS_FULL };
 template <class J, class = void>
-struct trace_device_group {
-    static constexpr bool value = false;
+struct trace_groups {
+    static constexpr int value = GROUPS_HOST;
 };
 template <class J>
-struct trace_device_group<J, std::void_t<decltype(J::kDeviceGroup)>> {
-    static constexpr bool value = J::kDeviceGroup;
+struct trace_groups<J, std::void_t<decltype(J::kGroups)>> {
+    static constexpr int value = J::kGroups;
 };
 
 // Items a warp takes at a time in a launch of n items on `warps` warps: 32, one per lane, unless that
@@ -110,15 +113,19 @@ struct trace_device_group<J, std::void_t<decltype(J::kDeviceGroup)>> {
 // every node and triangle that only other lanes visit.  256 rays on 20 k triangles 37 -> 21.5 us,
 // a 128^2 render 167 -> 142 us, one 250^2 sun-ray grid with two bounces 181 -> 137 us.  (Groups that also
 // shrink at the end of a large launch cost it 1 - 3 %: its last rays then take more issue slots.)
+// Scenes of fewer than SMALL_SCENE triangles always get 32: their rays are done in a few nodes, and the
+// work per ray outside the traversal, repeated per warp, is what they wait for (27 k camera paths in a
+// box of 36 triangles: 64 us, in groups of 8 67 us).
+constexpr size_t SMALL_SCENE = 1024;
 __host__ __device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t warps) {
     const uint32_t per = n / warps;
-    return per >= 16u ? 32u : per >= 8u ? 16u : per >= 4u ? 4u : per >= 2u ? 2u : 1u;
+    return per >= 16u ? 32u : per >= 8u ? 16u : per >= 4u ? 8u : per >= 2u ? 4u : per >= 1u ? 2u : 1u;
 }
 
 // Persistent ray-queue kernel.  Each warp takes one group of consecutive items per atomic grab, or,
 // with chunk > 1 and full groups, a guided number of up to `chunk` groups, shrinking with the work left
 // so that the last grabs stay small (few atomics on the queue counter while much work is left, balance
-// at the end).  grab: group size | chunk << 8.
+// at the end).  grab: group size (0: from the count, GROUPS_DEVICE) | chunk << 8.
 template <bool ANY, bool COUNT, class Job>
 __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value) k_trace(SceneView sv, Job job, uint32_t n_items,
                                                             const uint32_t* __restrict__ n_dev,
@@ -131,7 +138,9 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
     uint32_t nrays = 0, nres = 0;
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
     const uint32_t chunk = grab >> 8;
-    const uint32_t group = trace_device_group<Job>::value ? group_size(n_items, warps_total) : grab & 0xFFu;
+    uint32_t group = grab & 0xFFu;
+    if constexpr (trace_groups<Job>::value == GROUPS_DEVICE)
+        if (!group) group = job.full_groups() ? 32u : group_size(n_items, warps_total);
     while (true) {
         uint32_t base = 0, take = group;
         if (lane == 0) {
@@ -178,20 +187,24 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
 }
 
 // Launches the persistent trace kernel over n_items work items (or over *n_dev items when n_dev is
-// given: n_items is then the upper bound used to size the grid).
+// given: n_items is then the upper bound used to size the grid).  full_groups: 32 items per warp whatever
+// the count (launches with FP64 items among others).
 template <bool ANY, class Job>
 void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items,
-                  const uint32_t* n_dev = nullptr, uint32_t* queue = nullptr, uint32_t chunk_override = 0) {
+                  const uint32_t* n_dev = nullptr, uint32_t* queue = nullptr, bool full_groups = false) {
     if (!queue) queue = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
     CRT_CUDA(cudaMemsetAsync(queue, 0, sizeof(uint32_t), ctx->stream));
     const size_t smem = TRACE_SMEM;
     const void* kfn = ctx->counting ? (const void*)k_trace<ANY, true, Job> : (const void*)k_trace<ANY, false, Job>;
     int grid = occupancy_grid(ctx, kfn, CRT_TRACE_BLOCK, smem);
-    // one warp per item at most (group_size)
-    const uint32_t need = std::max<uint32_t>((n_items + CRT_TRACE_BLOCK / 32 - 1) / (CRT_TRACE_BLOCK / 32), 1u);
+    constexpr int groups = trace_groups<Job>::value;
+    full_groups = full_groups || groups == GROUPS_FULL || (sv.nodes && sv.n_tris < SMALL_SCENE);
+    // at most one warp per group (per item where groups may be smaller than 32)
+    const uint32_t per_block = full_groups ? CRT_TRACE_BLOCK : CRT_TRACE_BLOCK / 32;
+    const uint32_t need = std::max<uint32_t>((n_items + per_block - 1) / per_block, 1u);
     if ((uint32_t)grid > need) grid = (int)need;
-    const uint32_t chunk = chunk_override ? chunk_override : (ctx->queue_chunk ? ctx->queue_chunk : 1u);
-    const uint32_t grab = group_size(n_items, (uint32_t)grid * (CRT_TRACE_BLOCK / 32)) | chunk << 8;
+    const uint32_t group = full_groups ? 32u : groups == GROUPS_DEVICE ? 0u : group_size(n_items, (uint32_t)grid * (CRT_TRACE_BLOCK / 32));
+    const uint32_t grab = group | (ctx->queue_chunk ? ctx->queue_chunk : 1u) << 8;
     if (ctx->counting)
         k_trace<ANY, true, Job><<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, queue,
                                                                              ctx->d_error, ctx->d_counters, grab);
