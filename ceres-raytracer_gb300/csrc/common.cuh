@@ -40,7 +40,7 @@ enum : uint32_t {
 
 // ------------------------------------------------------------------ context
 enum ScratchSlot {
-    SCR_QUEUE = 0,      // persistent-kernel work counters
+    SCR_QUEUE = 0,      // persistent-kernel work counters (k_trace: zero between launches)
     SCR_RAYS,           // staged rays / hits
     SCR_OUT0,
     SCR_OUT1,

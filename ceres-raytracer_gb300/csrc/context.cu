@@ -199,6 +199,9 @@ int crt_context_create(int device, crt_context** out) {
         CRT_CUDA(cudaMemset(ctx->d_counters, 0, 4 * sizeof(unsigned long long)));
         CRT_CUDA(cudaMalloc(&ctx->d_error, sizeof(uint32_t)));
         CRT_CUDA(cudaMemset(ctx->d_error, 0, sizeof(uint32_t)));
+        // the trace queue's counters start at zero and every trace leaves them so (k_trace)
+        CRT_CUDA(cudaMemset(ctx_scratch(ctx, SCR_QUEUE, 256), 0, 256));
+        CRT_CUDA(cudaDeviceSynchronize());
     });
     if (rc != CRT_OK) {
         crt_context_destroy(ctx);
@@ -270,7 +273,7 @@ int crt_measure_read(crt_context* ctx, const void* buf, size_t bytes, uint32_t r
         CRT_CHECK(is_device_ptr(buf) && ((uintptr_t)buf & 15) == 0, CRT_ERR_INVALID,
                   "crt_measure_read needs a 16-byte aligned device buffer");
         CRT_CUDA(cudaSetDevice(ctx->device));
-        uint32_t* sink = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
+        uint32_t* sink = (uint32_t*)ctx_scratch(ctx, SCR_OUT0, 256);
         const int grid = occupancy_grid(ctx, (const void*)k_read_stream, 256, 0);
         const uint4* p = (const uint4*)buf;
         const size_t n16 = bytes / 16;

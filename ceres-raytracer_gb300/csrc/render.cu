@@ -3,7 +3,8 @@
 // queues that serve many requests (renders and LiDAR grids, possibly on different resident scenes)
 // per launch:
 //
-//   begin     copy this wave's descriptor, reset the queue counters          (k_wave_begin)
+//   begin     copy this wave's descriptor, reset the queue counters (k_wave_begin; a call of a single
+//             wave reads the uploaded descriptor instead)
 //   primary   LiDAR beams of the batch + camera ray per (pixel, sample)       (persistent trace)
 //             (+ the sun rays of one SRP range in crt_batch_mixed waves, whose shade and specular
 //             segments follow: srp_wave_stages)
@@ -115,7 +116,10 @@ struct Batch {
     const WaveDesc* descs;
     WaveDesc* cur;
     uint32_t* wave_idx;
-    uint32_t* counts;          // [0] |bounce queue in| [1] |bounce queue out| [2] |shadow queue|
+    uint32_t* counts;          // queue lengths of bounce b at 2 (b mod 3): paths continuing out of it, its shadow
+                               // rays; k_shade of a bounce zeroes the next bounce's (last read two bounces ago).
+                               // [6] [7] [8]: work counters of the primary, shadow and bounce traces (the first
+                               // zeroed with the wave's descriptor, the others by every k_shade)
     uint32_t L;                // light stride per path
     float4* ray;
     uint32_t* skip;
@@ -369,15 +373,9 @@ __global__ void k_wave_begin(Batch B) {
     const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
     uint32_t* d = reinterpret_cast<uint32_t*>(B.cur);
     for (uint32_t k = threadIdx.x; k < sizeof(WaveDesc) / 4; k += blockDim.x) d[k] = s[k];
-    if (threadIdx.x == 0) B.counts[0] = B.counts[1] = B.counts[2] = 0;
+    if (threadIdx.x < 9) B.counts[threadIdx.x] = 0;
 }
 __global__ void k_wave_end(Batch B) { *B.wave_idx += 1; }
-__global__ void k_queue_rotate(uint32_t* counts) {
-    counts[0] = counts[1];
-    counts[1] = 0;
-    counts[2] = 0;
-}
-
 // Path weight at bounce b: Color(2*M_PI) at the camera vertex (unidirectional.hpp:38), then
 // multiplied by (1 - r1) per bounce (k_shade)
 __device__ __forceinline__ float4 path_weight(const Batch& B, uint32_t p, int bounce) {
@@ -580,7 +578,9 @@ __device__ __forceinline__ uint32_t shade_path(const Batch& B, int bounce, uint3
 __global__ void __launch_bounds__(256) k_shade(Batch B, int bounce, const uint32_t* __restrict__ q_in,
                                                uint32_t* __restrict__ q_out, bool any_cont,
                                                unsigned long long* __restrict__ counters) {
-    const uint32_t n = bounce == 0 ? B.cur->n_paths : B.counts[0];
+    const uint32_t n = bounce == 0 ? B.cur->n_paths : B.counts[2 * ((bounce - 1) % 3)];
+    uint32_t* const n_out = B.counts + 2 * (bounce % 3);   // continuing paths, shadow rays
+    if (blockIdx.x == 0 && threadIdx.x < 2) B.counts[2 * ((bounce + 1) % 3) + threadIdx.x] = B.counts[7 + threadIdx.x] = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
         uint32_t p = 0, req = 0;
@@ -607,13 +607,13 @@ __global__ void __launch_bounds__(256) k_shade(Batch B, int bounce, const uint32
             const uint32_t wsum = __reduce_add_sync(0xFFFFFFFFu, resolved);
             if ((threadIdx.x & 31) == 0 && wsum) atomicAdd(counters + 3, (unsigned long long)wsum);
         }
-        const uint2 at = block_append2(&B.counts[2], __popc(keep), &B.counts[1], 0u);
+        const uint2 at = block_append2(n_out + 1, __popc(keep), n_out, 0u);
         uint32_t e = at.x;
         for (uint32_t m = keep; m; m &= m - 1) B.sidx[e++] = make_uint2(p * B.L + (uint32_t)(__ffs(m) - 1), req);
         // bounce queue grouped by ray octant within the block: warps of the bounce trace take rays
         // with one near-to-far child order
         if (any_cont) {   // false at the wave's last bounce: no path continues
-            const uint32_t qi = block_append_buckets8(&B.counts[1], cont ? (sp >> 16) & 7u : 8u);
+            const uint32_t qi = block_append_buckets8(n_out, cont ? (sp >> 16) & 7u : 8u);
             if (cont) q_out[qi] = p;
         }
     }
@@ -641,7 +641,7 @@ __device__ __forceinline__ float4 add_light(const Batch& B, uint32_t p, uint32_t
 }
 
 __global__ void k_accum(Batch B, int bounce, const uint32_t* __restrict__ q_in) {
-    const uint32_t n = bounce == 0 ? B.cur->n_paths : B.counts[0];
+    const uint32_t n = bounce == 0 ? B.cur->n_paths : B.counts[2 * ((bounce - 1) % 3)];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t p = bounce == 0 ? i : q_in[i];
         const bool hit = __float_as_uint(B.hit[p].w) != CRT_MISS;
@@ -684,10 +684,12 @@ __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
         const RReq& R = B.rr[S.req];
         const uint32_t pixel = S.active ? S.active[a] : tile_slot_pixel(a, R.c.W, R.c.H);
         const size_t g = (size_t)R.pix_base + pixel;
-        // a slice that starts at sample 0 holds the pixel's first samples: its state is still the
-        // zeroed one (running mean, count and done flag), so it is not read
+        // a slice that starts at sample 0 holds the pixel's first samples: its state (running mean, count
+        // and done flag) is not set yet and not read
         const bool fresh = S.s0 == 0;
         if (!fresh && B.done[g]) continue;
+        const bool last = R.fin_update && S.s0 + S.ns == (uint32_t)R.c.max_samples;
+        bool done = false;
         float4 m = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : B.pix[g];
         uint32_t t = fresh ? 0u : B.taken[g];
         for (uint32_t k = 0; k < S.ns; ++k) {
@@ -711,14 +713,18 @@ __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
             if ((int)sample >= R.c.min_samples) {
                 const float noise = sqrtf(dx * dx + dy * dy + dz * dz);
                 if (noise < R.c.noise_threshold) {
-                    B.done[g] = 1;
+                    done = true;
                     break;
                 }
             }
         }
-        B.pix[g] = m;
-        B.taken[g] = t;
-        if (R.fin_update && S.s0 + S.ns == (uint32_t)R.c.max_samples) store_pixel(R, pixel, m);
+        if (last) {   // nothing reads the pixel's state after this
+            store_pixel(R, pixel, m);
+        } else {
+            B.pix[g] = m;
+            B.taken[g] = t;
+            if (fresh || done) B.done[g] = done;
+        }
     }
 }
 
@@ -794,27 +800,30 @@ inline uint32_t tiles_items(uint32_t W, uint32_t H) { return ((W + 7) / 8) * ((H
 // trace also traces the wave's SRP sun rays and srp_stages (launches of the SRP shade and specular
 // segments) runs right after it.  srp_mask (when given): the SRP hit mask, zeroed before the primary
 // trace.  small_scenes: every scene of the wave has fewer than SMALL_SCENE triangles (group_size).
-// With srp_stages reading the wave's range from the device descriptor (srp_wave_stages_dev)
+// direct: B.cur already is the wave's descriptor and the counters are zero (a call of a single wave):
+// no k_wave_begin and k_wave_end (8 us).  With srp_stages reading the wave's range from the device descriptor (srp_wave_stages_dev)
 // the sequence is the same for every wave and can be captured and replayed.
 void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, uint32_t lidar_items,
-                         int max_bounces, uint32_t* qa, uint32_t* qb, uint32_t* tqueue, uint32_t srp_items = 0,
+                         int max_bounces, uint32_t* qa, uint32_t* qb, uint32_t srp_items = 0,
                          const std::function<void()>* srp_stages = nullptr, uint32_t* srp_mask = nullptr,
-                         size_t srp_mask_len = 0, bool small_scenes = false) {
+                         size_t srp_mask_len = 0, bool small_scenes = false, bool direct = false) {
     cudaStream_t st = ctx->stream;
     const uint32_t g_shade = grid_for(ctx, k_shade, P), g_accum = grid_for(ctx, k_accum, P);
     const uint32_t g_update = max_bounces <= 1 ? grid_for(ctx, k_update<true>, P) : grid_for(ctx, k_update<false>, P);
-    k_wave_begin<<<1, 128, 0, st>>>(B);
-    check_launch(ctx, "k_wave_begin");
+    if (!direct) {
+        k_wave_begin<<<1, 512, 0, st>>>(B);
+        check_launch(ctx, "k_wave_begin");
+    }
     if (srp_mask) CRT_CUDA(cudaMemsetAsync(srp_mask, 0, srp_mask_len, st));
     if (srp_items) {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<true>{B},
                             (uint32_t)std::min<size_t>(P + lidar_items + srp_items, 0xFFFFFF00u), &B.cur->n_primary,
-                            tqueue, small_scenes);
+                            B.counts + 6, small_scenes);
         if (srp_stages) (*srp_stages)();
     } else {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<false>{B},
-                            (uint32_t)std::min<size_t>(P + lidar_items, 0xFFFFFF00u), &B.cur->n_primary, tqueue,
-                            small_scenes || lidar_items > 0);
+                            (uint32_t)std::min<size_t>(P + lidar_items, 0xFFFFFF00u), &B.cur->n_primary,
+                            B.counts + 6, small_scenes || lidar_items > 0);
     }
     const uint32_t* q_in = nullptr;
     uint32_t* q_out = qa;
@@ -824,15 +833,14 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
                                          ctx->counting ? ctx->d_counters : nullptr);
         check_launch(ctx, "k_shade");
         launch_trace<true>(ctx, SceneView{}, ShadowJob{B}, (uint32_t)std::min<size_t>(P * NL, 0xFFFFFF00u),
-                           &B.counts[2], tqueue, small_scenes);
+                           &B.counts[2 * (b % 3) + 1], B.counts + 7, small_scenes);
         if (!fuse) {
             k_accum<<<g_accum, 256, 0, st>>>(B, b, q_in);
             check_launch(ctx, "k_accum");
         }
         if (b < max_bounces - 1) {
-            launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[1], tqueue, small_scenes);
-            k_queue_rotate<<<1, 1, 0, st>>>(B.counts);
-            check_launch(ctx, "k_queue_rotate");
+            launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[2 * (b % 3)],
+                                B.counts + 8, small_scenes);
             q_in = q_out;
             q_out = (q_out == qa) ? qb : qa;
         }
@@ -840,6 +848,7 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
     if (fuse) k_update<true><<<g_update, 256, 0, st>>>(B);
     else k_update<false><<<g_update, 256, 0, st>>>(B);
     check_launch(ctx, "k_update");
+    if (direct) return;
     k_wave_end<<<1, 1, 0, st>>>(B);
     check_launch(ctx, "k_wave_end");
 }
@@ -1064,6 +1073,9 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
     char* s_state = nullptr;
     uint32_t* s_bq = nullptr;
     uint32_t* s_bcount = nullptr;
+    // a single wave reads its descriptor where it was uploaded (launch_wave_kernels)
+    const bool direct = plan.size() == 1 && !any_adaptive;
+    size_t up_bytes = 0;
     auto carve = [&](char* b) {
         size_t off = 0;
         auto take = [&](size_t bytes) {
@@ -1072,14 +1084,17 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
             off += bytes;
             return q;
         };
+        // first what is uploaded, in one copy
         B.rr = (const RReq*)take(sizeof(RReq) * std::max<size_t>(rr.size(), 1));
         B.lr = (const LReq*)take(sizeof(LReq) * std::max<size_t>(lr.size(), 1));
         B.lights = (const LightDev*)take(sizeof(LightDev) * std::max<size_t>(lights.size(), 1));
-        B.tan = (const double*)take(8 * std::max<uint32_t>(tan_total, 1));
         B.descs = (const WaveDesc*)take(WD * plan.size());
-        B.cur = (WaveDesc*)take(WD);
         B.wave_idx = (uint32_t*)take(64);
         B.counts = (uint32_t*)take(64);
+        for (size_t j = 0; j < n_srp; ++j) s_att[j] = (SrpAtt*)take(sizeof(SrpAtt) * std::max<size_t>(splans[j].n_att(), 1));
+        up_bytes = off;
+        B.cur = direct ? (WaveDesc*)B.descs : (WaveDesc*)take(WD);
+        B.tan = (const double*)take(8 * std::max<uint32_t>(tan_total, 1));
         B.ray = (float4*)take(P * 32);
         B.skip = (uint32_t*)take(P * 4);
         B.hit = (float4*)take(P * 16);
@@ -1096,10 +1111,9 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         B.pix = (float4*)take((size_t)std::max<uint32_t>(pix_total, 1) * 16);
         B.taken = (uint32_t*)take((size_t)std::max<uint32_t>(pix_total, 1) * 4);
         B.done = (uint8_t*)take(std::max<uint32_t>(pix_total, 1));
-        for (size_t j = 0; j < n_srp; ++j) {   // SRP: attitude table, partial sums, staged outputs
+        for (size_t j = 0; j < n_srp; ++j) {   // SRP: partial sums, staged outputs
             const SrpPlan& SP = splans[j];
             const size_t na = std::max<size_t>(SP.n_att(), 1);
-            s_att[j] = (SrpAtt*)take(sizeof(SrpAtt) * na);
             s_partial[j] = (double*)take(sizeof(double) * 6 * std::max<uint64_t>(SP.blocks_per_att, 1) * na);
             s_force[j] = is_device_ptr(srps[j]->force) ? srps[j]->force : (double*)take(24 * na);
             s_torque[j] = is_device_ptr(srps[j]->torque) ? srps[j]->torque : (double*)take(24 * na);
@@ -1107,7 +1121,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         if (n_srp) {   // one wave's SRP item state, shared by the requests' ranges
             s_state = (char*)take(srp_state_bytes(std::max<uint64_t>(srp_max, 1), srp_nb));
             s_bq = srp_nb ? (uint32_t*)take(srp_max * 4 + 256) : nullptr;
-            s_bcount = (uint32_t*)take(256);
+            s_bcount = (uint32_t*)(s_state + srp_mask_offset(srp_max, srp_nb));
         }
         return off;
     };
@@ -1157,36 +1171,27 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
     }
 
     // ---- uploads (pinned staging ring: no wait for the previous call's kernels)
-    size_t srp_up = 0;
-    for (const SrpPlan& SP : splans) srp_up += sizeof(SrpAtt) * SP.n_att() + 256;
-    const size_t up_bytes = sizeof(RReq) * rr.size() + sizeof(LReq) * lr.size() + sizeof(LightDev) * lights.size() +
-                            WD * plan.size() + srp_up + 1024;
-    PinnedStaging staging(ctx, up_bytes);
+    PinnedStaging staging(ctx, std::max(up_bytes, WD));
     char* pin = staging.p;
-    size_t po = 0;
     auto up = [&](const void* dst, const void* src, size_t bytes) {
-        if (!bytes) return;
-        std::memcpy(pin + po, src, bytes);
-        CRT_CUDA(cudaMemcpyAsync((void*)dst, pin + po, bytes, cudaMemcpyHostToDevice, st));
-        po += (bytes + 255) & ~size_t(255);
+        if (bytes) std::memcpy(pin + ((const char*)dst - base), src, bytes);
     };
     up(B.rr, rr.data(), sizeof(RReq) * rr.size());
     up(B.lr, lr.data(), sizeof(LReq) * lr.size());
     up(B.lights, lights.data(), sizeof(LightDev) * lights.size());
     up(B.descs, plan.data(), WD * plan.size());
+    std::memset(pin + ((char*)B.wave_idx - base), 0, 64);
+    std::memset(pin + ((char*)B.counts - base), 0, 64);
     for (size_t j = 0; j < n_srp; ++j) up(s_att[j], splans[j].att.data(), sizeof(SrpAtt) * splans[j].n_att());
+    CRT_CUDA(cudaMemcpyAsync(base, pin, up_bytes, cudaMemcpyHostToDevice, st));
     staging.release();   // the adaptive loop below rewrites `pin` only after synchronising the stream
-    CRT_CUDA(cudaMemsetAsync(B.wave_idx, 0, 4, st));
-    if (pix_total) {
-        // every pixel of a request that takes samples gets its mean and count from its first slice
-        // (k_update); only requests without samples (max_samples 0) read the zeroed state
-        bool unsampled = false;
-        for (const HostReq& h : hreq) unsampled |= h.total == 0;
-        if (unsampled) {
-            CRT_CUDA(cudaMemsetAsync(B.pix, 0, (size_t)pix_total * 16, st));
-            CRT_CUDA(cudaMemsetAsync(B.taken, 0, (size_t)pix_total * 4, st));
-        }
-        CRT_CUDA(cudaMemsetAsync(B.done, 0, pix_total, st));
+    // every pixel of a request that takes samples gets its mean, count and flag from its first slice
+    // (k_update); only requests without samples (max_samples 0) read the zeroed state
+    bool unsampled = false;
+    for (const HostReq& h : hreq) unsampled |= h.total == 0;
+    if (unsampled) {
+        CRT_CUDA(cudaMemsetAsync(B.pix, 0, (size_t)pix_total * 16, st));
+        CRT_CUDA(cudaMemsetAsync(B.taken, 0, (size_t)pix_total * 4, st));
     }
     for (size_t k = 0; k < lr.size(); ++k) {
         const crt_lidar_grid_desc& g = *([&]() {
@@ -1203,15 +1208,18 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
     B.L = (uint32_t)NL;
 
     // ---- one wave: every launch reads the wave from B.cur (graph-capturable)
-    uint32_t* tqueue = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
     bool small_scenes = n_srp == 0;
     for (size_t i = 0; i < n; ++i) small_scenes = small_scenes && reqs[i].scene->n_tris < SMALL_SCENE;
     auto launch_wave = [&]() {
-        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, tqueue, 0, nullptr, nullptr, 0, small_scenes);
+        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, 0, nullptr, nullptr, 0, small_scenes, direct);
     };
 
     size_t waves_run = 0;
-    const bool graph_ok = ctx->use_graphs && !ctx->counting && plan.size() > 1;
+    // waves that hold nothing but SRP items take no render stages (max_bounces 0), and a single wave with
+    // render or LiDAR work is launched once, not captured
+    size_t full_waves = 0;
+    for (const WaveDesc& w : plan) full_waves += w.n_paths || w.n_lidar_items;
+    const bool graph_ok = ctx->use_graphs && !ctx->counting && full_waves > 1;
     const bool with_srp = n_srp && srp_max > 0;
     if (graph_ok) {
         // waves carrying SRP items run their SRP stages from the wave descriptor (B.cur->srp), for
@@ -1221,7 +1229,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         if (with_srp) {
             const SrpStage* d_stage = &B.cur->srp;
             srp_stages = [&, d_stage]() {
-                srp_wave_stages_dev(ctx, d_stage, (uint32_t)srp_max, srp_nb, s_bq, s_bcount, tqueue);
+                srp_wave_stages_dev(ctx, d_stage, (uint32_t)srp_max, srp_nb, s_bq, s_bcount);
             };
             srp_mask = (uint32_t*)(s_state + srp_mask_offset(srp_max, srp_nb));
         }
@@ -1239,8 +1247,8 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         const uint64_t before = ctx->launches;
         try {
             if (with_srp)
-                launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, tqueue, (uint32_t)srp_max,
-                                    &srp_stages, srp_mask, srp_mask_bytes(srp_max));
+                launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, (uint32_t)srp_max,
+                                    &srp_stages, srp_mask, srp_zero_bytes(srp_max));
             else
                 launch_wave();
         } catch (...) {
@@ -1252,8 +1260,13 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         CRT_CUDA(cudaGraphInstantiate(&gh.ge, gh.g, 0));
         ctx->launches = before;
         for (size_t w = 0; w < plan.size(); ++w) {
-            CRT_CUDA(cudaGraphLaunch(gh.ge, st));
-            ctx->launches += per_wave;
+            if (plan[w].n_paths || plan[w].n_lidar_items) {
+                CRT_CUDA(cudaGraphLaunch(gh.ge, st));
+                ctx->launches += per_wave;
+            } else {
+                launch_wave_kernels(ctx, B, 1, NL, 0, 0, qa, qb, plan[w].n_srp_items, &srp_stages, srp_mask,
+                                    srp_zero_bytes(srp_max));
+            }
         }
         waves_run = plan.size();
     } else if (with_srp) {
@@ -1264,14 +1277,15 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
             if (w < sranges.size()) {
                 const SrpRange& R = sranges[w];
                 crt_scene* sc = srps[R.req]->base.scene;
-                CRT_CUDA(cudaMemsetAsync(plan[w].srp.W.hitmask, 0, srp_mask_bytes(R.n), st));   // before the trace
+                CRT_CUDA(cudaMemsetAsync(s_bcount, 0, srp_zero_bytes(R.n), st));   // counters, hit mask
                 stages = [&, w, sc]() {
                     srp_wave_stages(ctx, scene_view(sc), plan[w].srp.W, (uint32_t)R.n, splans[R.req], s_partial[R.req],
                                     nullptr, (uint32_t)sc->n_tris, s_bq, s_bcount);
                 };
             }
-            launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, tqueue,
-                                (uint32_t)std::max<uint64_t>(srp_max, 1), stages ? &stages : nullptr);
+            const WaveDesc& wd = plan[w];
+            launch_wave_kernels(ctx, B, std::max<uint32_t>(wd.n_paths, 1), NL, wd.n_lidar_items, wd.n_paths ? max_bounces : 0, qa,
+                                qb, std::max<uint32_t>(wd.n_srp_items, 1), stages ? &stages : nullptr, nullptr, 0, false, direct);
         }
         waves_run = plan.size();
     } else {
@@ -1281,7 +1295,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
 
     // ---- adaptive requests: one sample per wave over the still-active pixels
     if (any_adaptive) {
-        uint32_t* acount = B.counts + 8;
+        uint32_t* acount = B.counts + 12;
         uint32_t offs = 0;
         for (HostReq& h : hreq) {
             if (!h.adaptive) continue;
@@ -1510,7 +1524,6 @@ struct WaveEngine {
     uint32_t* d_wave_idx = nullptr;
     uint32_t* d_counts = nullptr;
     uint32_t* d_acount = nullptr;
-    uint32_t* d_tqueue = nullptr;
     // SRP items of one wave (allocated at the first SRP admission): state, continuation queue, counters
     uint64_t srp_cap = 0;
     char* srp_state = nullptr;
@@ -1667,7 +1680,7 @@ WaveEngine* engine_create(crt_context* ctx, size_t budget_bytes) {
     try {
         CRT_CUDA(cudaSetDevice(ctx->device));
         const size_t fixed = up256(sizeof(RReq) * ENGINE_SLOTS) + up256(sizeof(LightDev) * ENGINE_SLOTS * MAX_LIGHTS) +
-                             up256(sizeof(LReq) * MAX_LIDAR) + 2 * up256(sizeof(WaveDesc)) + 4 * 256 +
+                             up256(sizeof(LReq) * MAX_LIDAR) + 2 * up256(sizeof(WaveDesc)) + 2 * 256 +
                              up256(4 * ENGINE_SLOTS);
         CRT_CUDA(cudaMalloc(&e->fixed, fixed));
         char* f = e->fixed;
@@ -1679,8 +1692,6 @@ WaveEngine* engine_create(crt_context* ctx, size_t budget_bytes) {
         e->d_cur = (WaveDesc*)take(sizeof(WaveDesc));
         e->d_wave_idx = (uint32_t*)take(256);
         e->d_counts = (uint32_t*)take(256);
-        e->d_tqueue = (uint32_t*)take(256);
-        take(256);
         e->d_acount = (uint32_t*)take(4 * ENGINE_SLOTS);
         for (uint32_t s = ENGINE_SLOTS; s > 0; --s) e->free_slots.push_back(s - 1);
         CRT_CUDA(cudaMallocHost(&e->err_pin, 2 * sizeof(uint32_t)));
@@ -1799,11 +1810,10 @@ bool engine_admit(WaveEngine* e, const crt_request& q, uint64_t tag) {
         }
         engine_upload(e, e->d_rr + r.slot, &R, sizeof(R));
         if (q.n_lights) engine_upload(e, e->d_lights + R.light_base, lights, sizeof(LightDev) * q.n_lights);
-        if (r.total == 0) {   // otherwise the first slice writes the mean and count (k_update)
+        if (r.total == 0) {   // otherwise the first slice writes the mean, count and flag (k_update)
             CRT_CUDA(cudaMemsetAsync(e->pix() + r.unit_off, 0, (size_t)r.npix * 16, st));
             CRT_CUDA(cudaMemsetAsync(e->taken() + r.unit_off, 0, (size_t)r.npix * 4, st));
         }
-        CRT_CUDA(cudaMemsetAsync(e->done() + r.unit_off, 0, r.npix, st));
         e->want_P = std::max(e->want_P, r.npix);
         e->want_NL = std::max(e->want_NL, std::max<uint32_t>(q.n_lights, 1));
     } else {
@@ -1851,10 +1861,10 @@ bool engine_admit_srp(WaveEngine* e, crt_scene* scene, const crt_srp_desc& desc,
     if (!e->srp_state) {
         const uint64_t cap = std::max<uint64_t>((uint64_t)e->want_P / SRP_BLOCK_ITEMS * SRP_BLOCK_ITEMS, SRP_BLOCK_ITEMS);
         const size_t b_state = up256(srp_state_bytes(cap, 1)), b_q = up256(cap * 4);
-        CRT_CUDA(cudaMalloc(&e->srp_state, b_state + b_q + 256));
+        CRT_CUDA(cudaMalloc(&e->srp_state, b_state + b_q));
         e->srp_cap = cap;
         e->srp_bq = (uint32_t*)(e->srp_state + b_state);
-        e->srp_bcount = (uint32_t*)(e->srp_state + b_state + b_q);
+        e->srp_bcount = (uint32_t*)(e->srp_state + srp_mask_offset(cap, 1));
     }
     EReq r;
     std::memset(&r.q, 0, sizeof(r.q));
@@ -2137,7 +2147,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
                 const SrpStage* d_stage = &e->d_cur->srp;
                 stages = [&, d_stage]() {
                     srp_wave_stages_dev(ctx, d_stage, (uint32_t)e->srp_cap, (uint32_t)srp_nb, e->srp_bq,
-                                        e->srp_bcount, e->d_tqueue);
+                                        e->srp_bcount);
                 };
                 mask = (uint32_t*)(e->srp_state + srp_mask_offset(e->srp_cap, 1));
             }
@@ -2146,9 +2156,9 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
             CRT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             const uint64_t before = ctx->launches;
             try {
-                launch_wave_kernels(ctx, B, P, NL, 0xF0000000u, max_bounces, qa, qb, e->d_tqueue,
+                launch_wave_kernels(ctx, B, P, NL, 0xF0000000u, max_bounces, qa, qb,
                                     srp_nb >= 0 ? (uint32_t)e->srp_cap : 0u, srp_nb >= 0 ? &stages : nullptr, mask,
-                                    srp_nb >= 0 ? srp_mask_bytes(e->srp_cap) : 0);
+                                    srp_nb >= 0 ? srp_zero_bytes(e->srp_cap) : 0);
             } catch (...) {
                 cudaStreamEndCapture(st, &cg);
                 if (cg) cudaGraphDestroy(cg);
@@ -2170,13 +2180,13 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
         std::function<void()> stages;
         if (sq) {
             const SrpWave W = w.srp.W;
-            CRT_CUDA(cudaMemsetAsync(W.hitmask, 0, srp_mask_bytes(srp_n), st));   // before the trace
+            CRT_CUDA(cudaMemsetAsync(e->srp_bcount, 0, srp_zero_bytes(srp_n), st));   // counters, hit mask
             stages = [&, W]() {
                 srp_wave_stages(ctx, scene_view(sq->q.scene), W, (uint32_t)srp_n, *sq->splan, sq->partial, nullptr,
                                 (uint32_t)sq->q.scene->n_tris, e->srp_bq, e->srp_bcount);
             };
         }
-        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, e->d_tqueue,
+        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb,
                             sq ? (uint32_t)e->srp_cap : 0u, sq ? &stages : nullptr);
     }
     // an SRP query whose last range ran in this wave: per-attitude totals, outputs staged

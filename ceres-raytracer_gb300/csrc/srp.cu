@@ -150,6 +150,7 @@ struct SrpShadeArgs {
     uint32_t n_tris;
     uint32_t* q_out;          // continuing items of the next segment
     uint32_t* q_count;
+    uint32_t* counts;         // the wave's counters (srp_wave_stages): the next segment's are zeroed
 };
 
 // Sums: each thread adds its (at most 4) rays in FP32, the warp tree is FP32 (at most 128 terms, so
@@ -159,6 +160,7 @@ struct SrpShadeArgs {
 template <bool FIRST>
 __device__ __forceinline__ void srp_shade(const SceneView& sv, const SrpWave& W, const SrpShadeArgs& A) {
     __shared__ double red[SRP_SHADE_THREADS / 32][6];
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.counts[(A.seg + 1) % 3] = A.counts[4] = 0u;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     bool any_hit = false;
@@ -272,9 +274,13 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade(SceneView sv, S
 // request's, return at once: the condition is uniform over the block)
 template <bool FIRST>
 __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpStage* __restrict__ S, uint32_t seg,
-                                                                    uint32_t* q_out, uint32_t* q_count) {
+                                                                    uint32_t* q_out, uint32_t* q_count,
+                                                                    uint32_t* counts) {
     const uint32_t n = S->n, nb = S->nb;
-    if (seg > nb || blockIdx.x * SRP_BLOCK_ITEMS >= n) return;
+    if (seg > nb || blockIdx.x * SRP_BLOCK_ITEMS >= n) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) counts[(seg + 1) % 3] = counts[4] = 0u;
+        return;
+    }
     SrpShadeArgs A;
     A.n_items = n;
     A.seg = seg;
@@ -287,6 +293,7 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
     A.n_tris = S->n_tris;
     A.q_out = q_out;
     A.q_count = q_count;
+    A.counts = counts;
     const SceneView sv = S->sv;
     const SrpWave W = S->W;
     srp_shade<FIRST>(sv, W, A);
@@ -440,7 +447,7 @@ SrpWave srp_wave(const SrpPlan& P, const SrpAtt* d_att, char* state, uint64_t ca
         W.box_hi[k] = P.box_hi[k];
     }
     W.hit = (float4*)state;
-    W.hitmask = (uint32_t*)(state + srp_mask_offset(cap, nb));
+    W.hitmask = (uint32_t*)(state + srp_mask_offset(cap, nb) + SRP_COUNTS);
     W.st_o = nb ? (float4*)(state + cap * 16) : nullptr;
     W.st_d = nb ? (float4*)(state + cap * 32) : nullptr;
     W.alive = nb ? (uint8_t*)(state + cap * 48) : nullptr;
@@ -449,7 +456,7 @@ SrpWave srp_wave(const SrpPlan& P, const SrpAtt* d_att, char* state, uint64_t ca
 
 void srp_wave_stages(crt_context* ctx, const SceneView& sv, const SrpWave& W, uint32_t n, const SrpPlan& P,
                      double* partial, double* facet, uint32_t n_tris, uint32_t* bq, uint32_t* bcount,
-                     uint64_t partial_block0, uint32_t* trace_queue) {
+                     uint64_t partial_block0) {
     cudaStream_t st = ctx->stream;
     SrpShadeArgs A;
     A.n_items = n;
@@ -464,8 +471,8 @@ void srp_wave_stages(crt_context* ctx, const SceneView& sv, const SrpWave& W, ui
     const uint32_t nblk = (n + SRP_BLOCK_ITEMS - 1) / SRP_BLOCK_ITEMS;
     for (uint32_t seg = 0; seg <= P.nb; ++seg) {
         A.seg = seg;
-        A.q_count = bcount + (seg & 1);          // filled by this segment's shade
-        if (seg < P.nb) CRT_CUDA(cudaMemsetAsync(A.q_count, 0, sizeof(uint32_t), st));
+        A.q_count = bcount + seg % 3;            // filled by this segment's shade
+        A.counts = bcount;
         if (seg == 0) {
             k_srp_shade<true><<<nblk, SRP_SHADE_THREADS, 0, st>>>(sv, W, A);
         } else {
@@ -473,7 +480,7 @@ void srp_wave_stages(crt_context* ctx, const SceneView& sv, const SrpWave& W, ui
             SrpBounceJob J;
             J.W = W;
             J.q = bq;
-            launch_trace<false>(ctx, sv, J, n, bcount + ((seg - 1) & 1), trace_queue);
+            launch_trace<false>(ctx, sv, J, n, bcount + (seg - 1) % 3, bcount + 4);
             k_srp_shade<false><<<nblk, SRP_SHADE_THREADS, 0, st>>>(sv, W, A);
         }
         check_launch(ctx, "k_srp_shade");
@@ -496,20 +503,19 @@ SrpStage srp_stage(const SceneView& sv, const SrpWave& W, uint32_t n, const SrpP
 }
 
 void srp_wave_stages_dev(crt_context* ctx, const SrpStage* d_stage, uint32_t n_max, uint32_t nb_max, uint32_t* bq,
-                         uint32_t* bcount, uint32_t* trace_queue) {
+                         uint32_t* bcount) {
     cudaStream_t st = ctx->stream;
     const uint32_t nblk = std::max<uint32_t>(1, (n_max + SRP_BLOCK_ITEMS - 1) / SRP_BLOCK_ITEMS);
     for (uint32_t seg = 0; seg <= nb_max; ++seg) {
-        uint32_t* q_count = bcount + (seg & 1);   // filled by this segment's shade
-        if (seg < nb_max) CRT_CUDA(cudaMemsetAsync(q_count, 0, sizeof(uint32_t), st));
+        uint32_t* q_count = bcount + seg % 3;   // filled by this segment's shade
         if (seg == 0) {
-            k_srp_shade_dev<true><<<nblk, SRP_SHADE_THREADS, 0, st>>>(d_stage, 0, bq, q_count);
+            k_srp_shade_dev<true><<<nblk, SRP_SHADE_THREADS, 0, st>>>(d_stage, 0, bq, q_count, bcount);
         } else {
             SrpBounceJobDev J;
             J.S = d_stage;
             J.q = bq;
-            launch_trace<false>(ctx, SceneView{}, J, n_max, bcount + ((seg - 1) & 1), trace_queue);
-            k_srp_shade_dev<false><<<nblk, SRP_SHADE_THREADS, 0, st>>>(d_stage, seg, bq, q_count);
+            launch_trace<false>(ctx, SceneView{}, J, n_max, bcount + (seg - 1) % 3, bcount + 4);
+            k_srp_shade_dev<false><<<nblk, SRP_SHADE_THREADS, 0, st>>>(d_stage, seg, bq, q_count, bcount);
         }
         check_launch(ctx, "k_srp_shade");
     }
@@ -542,7 +548,7 @@ void srp_run(crt_context* ctx, crt_scene* s, const crt_srp_desc* desc, const dou
         double* d_partial = (double*)ctx_scratch(ctx, SCR_WAVE3, sizeof(double) * 6 * P.blocks_per_att * n_att);
         char* state = (char*)ctx_scratch(ctx, SCR_WAVE4, srp_state_bytes(wave_items, P.nb));
         uint32_t* bq = P.nb ? (uint32_t*)ctx_scratch(ctx, SCR_WAVE5, wave_items * 4 + 256) : nullptr;
-        uint32_t* bcount = (uint32_t*)ctx_scratch(ctx, SCR_WAVE6, 256);
+        uint32_t* bcount = (uint32_t*)(state + srp_mask_offset(wave_items, P.nb));
         double* d_force = (double*)out_device(ctx, force, n_att * 24, SCR_OUT0);
         double* d_torque = (double*)out_device(ctx, torque, n_att * 24, SCR_OUT1);
         double* d_facet = facet_power ? (double*)out_device(ctx, facet_power, n_att * s->n_tris * 8, SCR_OUT2) : nullptr;
@@ -556,8 +562,8 @@ void srp_run(crt_context* ctx, crt_scene* s, const crt_srp_desc* desc, const dou
             // from L1/L2 (measured: larger grabs were slower on the 2M asteroid)
             SrpPrimaryJob J;
             J.W = W;
-            CRT_CUDA(cudaMemsetAsync(W.hitmask, 0, srp_mask_bytes(n), st));
-            launch_trace<false>(ctx, sv, J, n);
+            CRT_CUDA(cudaMemsetAsync(bcount, 0, srp_zero_bytes(n), st));   // counters and hit mask
+            launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5);
             srp_wave_stages(ctx, sv, W, n, P, d_partial, d_facet, (uint32_t)s->n_tris, bq, bcount);
         }
         srp_reduce(ctx, d_partial, P, d_force, d_torque);
@@ -582,7 +588,7 @@ extern "C" int crt_srp(crt_scene* s, const crt_srp_desc* desc, const double* qua
 // components embedded in a host application that owns the CUDA allocator.  Every GPU that loads the
 // library holds this array until the process exits.
 //
-// Layout: work counters, the attitude table and the staging of host outputs, then the state of one
+// Layout: the attitude table and the staging of host outputs, then the state of one
 // wave of at most SS_WAVE items (per-item hits and continuation rays, hit mask, continuation queue)
 // and the partial sums of that wave's blocks.  Waves hold whole attitudes when an attitude has at
 // most SS_WAVE items (their totals are reduced right after the wave); a larger attitude runs as
@@ -597,9 +603,7 @@ namespace {
 
 constexpr uint64_t SS_WAVE = 1u << 20;                            // items per wave
 constexpr size_t ss_align(size_t x) { return (x + 255) & ~size_t(255); }
-constexpr size_t SS_QUEUE = 0;                                    // trace work counter
-constexpr size_t SS_BCOUNT = 128;                                 // 2 continuation-queue counters
-constexpr size_t SS_ATT = 256;                                    // SrpAtt table
+constexpr size_t SS_ATT = 0;                                      // SrpAtt table
 constexpr size_t SS_OUT = ss_align(SS_ATT + sizeof(SrpAtt) * CRT_SRP_STATIC_MAX_ATT);   // force | torque staging
 constexpr size_t SS_RUN = ss_align(SS_OUT + 48ull * CRT_SRP_STATIC_MAX_ATT);          // running totals 256 x 6
 constexpr size_t SS_PART = ss_align(SS_RUN + 6ull * 8 * SRP_REDUCE_THREADS);          // one wave's block sums
@@ -646,13 +650,12 @@ extern "C" int crt_srp_static(crt_scene* s, const crt_srp_desc* desc, const doub
         if (!n_att) return;
         CRT_CUDA(cudaSetDevice(ctx->device));
         char* base = (char*)static_scratch(ctx->device);
-        uint32_t* queue = (uint32_t*)(base + SS_QUEUE);
-        uint32_t* bcount = (uint32_t*)(base + SS_BCOUNT);
         SrpAtt* d_att = (SrpAtt*)(base + SS_ATT);
         double* run = (double*)(base + SS_RUN);
         double* d_partial = (double*)(base + SS_PART);
         uint32_t* bq = (uint32_t*)(base + SS_BQ);
         char* state = base + SS_STATE;
+        uint32_t* bcount = (uint32_t*)(state + srp_mask_offset(SS_WAVE, P.nb));
         cudaStream_t st = ctx->stream;
 
         // attitude table: computed on the host in chunks held on the stack, copied into the scratch;
@@ -686,11 +689,11 @@ extern "C" int crt_srp_static(crt_scene* s, const crt_srp_desc* desc, const doub
                 const SrpWave W = srp_wave(G, d_att + a0, state, SS_WAVE, i0, n);
                 SrpPrimaryJob J;
                 J.W = W;
-                CRT_CUDA(cudaMemsetAsync(W.hitmask, 0, srp_mask_bytes(n), st));
-                launch_trace<false>(ctx, sv, J, n, nullptr, queue);
+                CRT_CUDA(cudaMemsetAsync(bcount, 0, srp_zero_bytes(n), st));   // counters and hit mask
+                launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5);
                 // block sums of this wave only: slot = (block of the attitude group) - (wave's first block)
                 const uint64_t block0 = i0 / SRP_BLOCK_ITEMS;
-                srp_wave_stages(ctx, sv, W, n, G, d_partial, nullptr, (uint32_t)s->n_tris, bq, bcount, block0, queue);
+                srp_wave_stages(ctx, sv, W, n, G, d_partial, nullptr, (uint32_t)s->n_tris, bq, bcount, block0);
                 if (split) {
                     k_srp_fold<<<1, SRP_REDUCE_THREADS, 0, st>>>(d_partial, block0, n / SRP_BLOCK_ITEMS, run);
                     check_launch(ctx, "k_srp_fold");

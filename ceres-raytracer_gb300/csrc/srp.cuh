@@ -119,14 +119,17 @@ struct SrpStage {
 };
 
 // Per-wave SRP state for waves of at most `cap` items: hits (16 B per item), continuation state when
-// there are specular segments (33 B per item), then the primary segment's hit mask (1 bit per item).
+// there are specular segments (33 B per item), then, zeroed together before the wave's primary trace, the
+// counters of the continuation queue and the primary segment's hit mask (1 bit per item).
 constexpr size_t srp_mask_offset(uint64_t cap, uint32_t nb) {
     return ((size_t)cap * (nb ? 49 : 16) + 255) & ~size_t(255);
 }
+constexpr size_t SRP_COUNTS = 256;   // bytes of the continuation queue's counters, before the mask
 constexpr size_t srp_state_bytes(uint64_t cap, uint32_t nb) {
-    return srp_mask_offset(cap, nb) + ((((size_t)cap + 31) / 32 * 4 + 255) & ~size_t(255)) + 256;
+    return srp_mask_offset(cap, nb) + SRP_COUNTS + ((((size_t)cap + 31) / 32 * 4 + 255) & ~size_t(255)) + 256;
 }
-inline size_t srp_mask_bytes(uint64_t n) { return ((size_t)n + 31) / 32 * 4; }
+// bytes to zero before the primary trace of a wave of n items, from srp_mask_offset on
+inline size_t srp_zero_bytes(uint64_t n) { return SRP_COUNTS + ((size_t)n + 31) / 32 * 4; }
 
 // Primary-segment result of wave item i: hits are stored and flagged in the mask; misses leave both
 __device__ __forceinline__ void srp_store_primary(const SrpWave& W, uint32_t i, const THit& h) {
@@ -156,13 +159,15 @@ SrpWave srp_wave(const SrpPlan& P, const SrpAtt* d_att, char* state, uint64_t ca
 // else the rest of the current attitude
 uint64_t srp_wave_items(const SrpPlan& P, uint64_t cap, uint64_t i0);
 // After the primary segment's hits are in W.hit: its shade, then the specular segments (trace of
-// the compacted continuation queue + shade).  bq: room for n entries; bcount: 2 counters.  Block b
+// the compacted continuation queue + shade).  bq: room for n entries; bcount: 3 counters, segment s
+// appending to counter s mod 3 (the state's SRP_COUNTS bytes, zeroed with the hit mask; each segment's
+// shade zeroes the next one's), bcount[4] the specular traces' work counter (zeroed by the shade before
+// each), bcount[5] free for the primary trace's.  Block b
 // of the wave sums into partial slot W.i0 / SRP_BLOCK_ITEMS + b - partial_block0 (0: the request's
 // whole partial array; the wave's first block: an array holding this wave's blocks only).
-// trace_queue: work counter of the continuation traces (null: the context's scratch counter).
 void srp_wave_stages(crt_context* ctx, const SceneView& sv, const SrpWave& W, uint32_t n, const SrpPlan& P,
                      double* partial, double* facet, uint32_t n_tris, uint32_t* bq, uint32_t* bcount,
-                     uint64_t partial_block0 = 0, uint32_t* trace_queue = nullptr);
+                     uint64_t partial_block0 = 0);
 // The stage descriptor of items [W.i0, W.i0 + n) of a request (plan P, partial sums `partial`)
 SrpStage srp_stage(const SceneView& sv, const SrpWave& W, uint32_t n, const SrpPlan& P, double* partial,
                    uint32_t n_tris);
@@ -170,6 +175,6 @@ SrpStage srp_stage(const SceneView& sv, const SrpWave& W, uint32_t n, const SrpP
 // nb_max specular segments over n_max items; segments and blocks beyond the range's own do nothing.
 // No argument depends on the range, so the launches can be captured once and replayed per wave.
 void srp_wave_stages_dev(crt_context* ctx, const SrpStage* d_stage, uint32_t n_max, uint32_t nb_max, uint32_t* bq,
-                         uint32_t* bcount, uint32_t* trace_queue);
+                         uint32_t* bcount);
 // Per-attitude force and torque from the request's partial sums (device outputs)
 void srp_reduce(crt_context* ctx, const double* partial, const SrpPlan& P, double* force, double* torque);
