@@ -36,7 +36,7 @@ struct SrpWave {
     uint32_t* hitmask;        // primary segment: one bit per wave item that hit (zeroed before the trace)
     float4* st_o;             // continuing ray: origin, power
     float4* st_d;             // continuing ray: direction, triangle it leaves
-    uint8_t* alive;           // continuing ray present
+    uint32_t* alive;          // continuing ray present: one bit per wave item
 };
 
 // attitude of wave item i (32-bit arithmetic: a wave is whole attitudes or a part of one)
