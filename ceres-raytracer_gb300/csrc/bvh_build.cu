@@ -2,12 +2,14 @@
 // NodeLayoutOptimizer of the reference, lib/bvh/sweep_sah_builder.hpp:43-111,
 // parallel_reinsertion_optimizer.hpp:140-211, node_layout_optimizer.hpp:30-92).
 //
-// Pipeline, one stream, no host round trips except one frontier count per collapse level:
+// Pipeline, one stream; the host waits once for the SAH levels and once for the collapse levels (more
+// only for trees much deeper than balanced ones):
 //   k_transform      entity transform in FP64 (transform.hpp:43-85), FP32 triangle records
 //                    (p0, p1, p2, n), exact FP32 boxes, centroids, normals
 //   k_bounds         scene and centroid bounds (order-preserving integer atomics)
 //   k_morton         30-bit Morton codes of centroids in the centroid bounds
 //   radix_sort       stable LSD radix sort, 8-bit digits, 4 passes (histogram / scan / scatter)
+//   sah_topology     binned-SAH tree over the Morton order (the default; else k_karras)
 //   k_karras         binary radix tree (Karras, "Maximizing parallelism in the construction of
 //                    BVHs, octrees, and k-d trees", HPG 2012); ties broken by index
 //   k_refit          bottom-up boxes and collapse costs, second arrival at each node does the
@@ -212,26 +214,41 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_hist(const uint32_t* __r
     hist[threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// exclusive scan of m values with one block of 1024 threads
+// exclusive scan of m values with one block of 1024 threads, 8 consecutive values per thread at a time
+// (one thread per contiguous part of the array took 25 us for 31 k values, this takes 8)
 __global__ void __launch_bounds__(1024) k_scan(uint32_t* __restrict__ a, uint32_t m) {
-    __shared__ uint32_t part[1024];
-    const uint32_t per = (m + 1023) / 1024;
-    const uint32_t b = threadIdx.x * per, e = min(m, b + per);
-    uint32_t s = 0;
-    for (uint32_t i = b; i < e; ++i) s += a[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        uint32_t v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
+    __shared__ uint32_t part[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < m; base += 8192u) {
+        const uint32_t b = base + threadIdx.x * 8u;
+        uint32_t v[8], s = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            v[k] = b + k < m ? a[b + k] : 0u;
+            s += v[k];
+        }
+        uint32_t x = s;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) part[warp] = x;
         __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - s;
-    for (uint32_t i = b; i < e; ++i) {
-        uint32_t v = a[i];
-        a[i] = run;
-        run += v;
+        uint32_t w = part[lane];   // every warp scans the 32 warp totals
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+            if (lane >= o) w += y;
+        }
+        const uint32_t before = warp ? __shfl_sync(0xFFFFFFFFu, w, warp - 1) : 0u;
+        uint32_t run = carry + before + x - s;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (b + k < m) a[b + k] = run;
+            run += v[k];
+        }
+        carry += __shfl_sync(0xFFFFFFFFu, w, 31);
+        __syncthreads();   // `part` is rewritten by the next round
     }
 }
 
@@ -1051,19 +1068,30 @@ __global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, con
 }
 
 // ---------------------------------------------------------------- binned-SAH topology
-// Top-down, level-synchronous binned SAH (16 bins on each axis over the centroid bounds) down to
+// Top-down binned SAH (16 bins on each axis over the centroid bounds; surface area x count) down to
 // segments of at most SAH_T triangles, which Karras' construction then builds (its prefix function
-// restricted to the segment).  Partitions are stable, so every segment keeps the Morton order of
-// the global sort.  Node numbering follows the binary radix tree: a segment [f, l] uses internal
+// restricted to the segment).  Partitions are stable, so every segment keeps the Morton order of the
+// global sort.  Node numbering follows the binary radix tree: a segment [f, l] uses internal
 // indices f .. l - 1, and the split that puts [first, p) left and [p, last] right gets index p - 1,
 // the last position of its left part, which no segment uses; together that is exactly n - 1 nodes,
 // so the collapse consumes the tree unchanged (its root is passed explicitly).
+//
+// Tasks of more than SAH_SUB triangles are split level by level over the whole GPU (k_sah_bin, k_sah_split,
+// k_sah_flags, k_scan, k_sah_scatter per level; the number of a level's tasks stays on the device); a task
+// of at most SAH_SUB triangles is taken to its segments by one block (k_sah_subtree).  What bounded the
+// build before was latency and atomics: twenty levels of thirteen launches and a host round trip each,
+// one thread per task reading 2.5 KB of bins, 39 shared-memory atomics per triangle on the few bins that
+// Morton neighbours share.  500 k triangles, levels and segments: about 4.6 -> 1.4 ms with the host's waits (kernels alone 3.6 ->
+// 1.05 ms).
 constexpr int SAH_BINS = 16;
 constexpr int SAH_T = 4;
 constexpr int SAH_W = 13;                               // count, box lo/hi, centroid lo/hi (fkeys)
 constexpr int SAH_TASK_WORDS = 3 * SAH_BINS * SAH_W;
-constexpr int SAH_BLOCK_ITEMS = 2048;
-constexpr int SAH_SMALL = 2048;                         // tasks of at most this many triangles: k_sah_bin_small
+constexpr int SAH_TILE = 1024;                          // positions per block of the flag and scatter kernels
+constexpr int SAH_BIN_TILE = 512;                       // positions per block of the binning kernel
+constexpr int SAH_SUB = 512;                            // tasks of at most this many triangles: k_sah_subtree
+constexpr int SAH_MAX_LEVELS = 256;
+constexpr uint32_t WARP = 0xFFFFFFFFu;
 
 struct SahTask {
     int first, count;
@@ -1074,11 +1102,22 @@ struct SahTask {
 struct SahSplit {
     int nl;                  // triangles of the left child
     int axis, bin;           // axis < 0: split by position (no usable centroid extent)
-    float lclo[3], lchi[3], rclo[3], rchi[3];
+    float clo[2][3], chi[2][3];   // centroid bounds of the left and right child
 };
 
-struct SahSeg {
-    int first, count, parent, side;
+// what the level kernels share on the device
+struct SahState {
+    uint32_t n_sub;                        // tasks of k_sah_subtree
+    int root;                              // internal index of the root
+    uint32_t n_tasks[SAH_MAX_LEVELS + 1];  // tasks of each level
+};
+
+struct SahTree {
+    int n;
+    int2* child;
+    int2* range;
+    int* parent;
+    int *seg_lo, *seg_hi;                  // per position: its segment
 };
 
 __device__ __forceinline__ int sah_bin(float c, float lo, float hi) {
@@ -1088,7 +1127,17 @@ __device__ __forceinline__ int sah_bin(float c, float lo, float hi) {
     return max(0, min(SAH_BINS - 1, b));
 }
 
-__global__ void k_sah_root(const uint32_t* __restrict__ keys, int n, SahTask* __restrict__ t) {
+// value of bin word w without triangles
+__device__ __forceinline__ uint32_t sah_empty(int w) {
+    const int k = w % SAH_W;
+    return k == 0 ? 0u : (((k - 1) % 6) < 3 ? 0xFFFFFFFFu : 0u);
+}
+
+__global__ void k_sah_root(const uint32_t* __restrict__ keys, int n, SahTask* __restrict__ tasks,
+                           SahTask* __restrict__ sub, uint32_t* __restrict__ bins, SahState* __restrict__ state) {
+    for (int w = threadIdx.x; w < SAH_TASK_WORDS; w += blockDim.x) bins[w] = sah_empty(w);
+    for (int l = threadIdx.x; l <= SAH_MAX_LEVELS; l += blockDim.x) state->n_tasks[l] = l == 0 && n > SAH_SUB ? 1u : 0u;
+    if (threadIdx.x) return;
     SahTask r;
     r.first = 0;
     r.count = n;
@@ -1098,99 +1147,110 @@ __global__ void k_sah_root(const uint32_t* __restrict__ keys, int n, SahTask* __
     }
     r.parent = -1;
     r.side = 0;
-    t[0] = r;
+    (n > SAH_SUB ? tasks : sub)[0] = r;
+    state->n_sub = n > SAH_SUB ? 0u : 1u;
+    state->root = -1;
 }
 
-__global__ void k_sah_clear(uint32_t* __restrict__ bins, size_t words) {
-    for (size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(w % SAH_W);
-        bins[w] = k == 0 ? 0u : (((k - 1) % 6) < 3 ? 0xFFFFFFFFu : 0u);
+__device__ __forceinline__ void sah_add(uint32_t* b, uint32_t cnt, const uint32_t key[12]) {
+    atomicAdd(&b[0], cnt);
+    for (int k = 0; k < 3; ++k) {
+        atomicMin(&b[1 + k], key[k]);
+        atomicMax(&b[4 + k], key[3 + k]);
+        atomicMin(&b[7 + k], key[6 + k]);
+        atomicMax(&b[10 + k], key[9 + k]);
     }
 }
 
-__device__ __forceinline__ void sah_add(uint32_t* b, const float4& lo, const float4& hi, const float4& c) {
-    atomicAdd(&b[0], 1u);
-    atomicMin(&b[1], fkey(lo.x)); atomicMin(&b[2], fkey(lo.y)); atomicMin(&b[3], fkey(lo.z));
-    atomicMax(&b[4], fkey(hi.x)); atomicMax(&b[5], fkey(hi.y)); atomicMax(&b[6], fkey(hi.z));
-    atomicMin(&b[7], fkey(c.x)); atomicMin(&b[8], fkey(c.y)); atomicMin(&b[9], fkey(c.z));
-    atomicMax(&b[10], fkey(c.x)); atomicMax(&b[11], fkey(c.y)); atomicMax(&b[12], fkey(c.z));
-}
-
-// One warp per task of at most SAH_SMALL triangles: the warp bins its task's positions (a contiguous
-// range) into warp-private shared memory, where only its own lanes contend, and stores the task's
-// bins, which no other kernel writes (k_sah_bin skips these tasks).  Counts, minima and maxima do not
-// depend on the order of the additions, so the bins equal those of k_sah_bin.
-__global__ void __launch_bounds__(256) k_sah_bin_small(const uint32_t* __restrict__ perm,
-                                                       const SahTask* __restrict__ tasks, int n_tasks,
-                                                       const float4* __restrict__ tbox, const float4* __restrict__ cen,
-                                                       uint32_t* __restrict__ bins) {
-    __shared__ uint32_t sb[8][SAH_TASK_WORDS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * 8 + warp;
-    if (t >= n_tasks) return;            // warp-uniform; the kernel has no block-wide barrier
-    const SahTask T = tasks[t];
-    if (T.count > SAH_SMALL) return;     // warp-uniform: binned by k_sah_bin
-    uint32_t* b = sb[warp];
-    for (int w = lane; w < SAH_TASK_WORDS; w += 32) {
-        const int k = w % SAH_W;
-        b[w] = k == 0 ? 0u : (((k - 1) % 6) < 3 ? 0xFFFFFFFFu : 0u);
+// Adds the warp's triangles (lanes in `on`) to the bins of their task in shared memory.  Morton neighbours
+// share bins: where the warp's lanes fall into few combinations of bins, the lanes of each are first
+// reduced to one (counts, minima and maxima do not depend on the order of the additions); past
+// SAH_GROUPS combinations, which run one after the other, the lanes' own atomics are faster.
+constexpr int SAH_GROUPS = 3;
+__device__ __forceinline__ void sah_bin_warp(uint32_t* bins, bool on, const float lo[3], const float hi[3],
+                                             const float c[3], const float clo[3], const float chi[3]) {
+    const uint32_t active = __ballot_sync(WARP, on);
+    if (on) {
+        int b[3];
+        uint32_t key[12];
+        for (int a = 0; a < 3; ++a) {
+            b[a] = sah_bin(c[a], clo[a], chi[a]);
+            key[a] = fkey(lo[a]);
+            key[3 + a] = fkey(hi[a]);
+            key[6 + a] = key[9 + a] = fkey(c[a]);
+        }
+        const uint32_t peers = __match_any_sync(active, b[0] | b[1] << 8 | b[2] << 16);
+        const bool leader = (int)(threadIdx.x & 31) == __ffs(peers) - 1;
+        uint32_t cnt = 1;
+        bool add = true;
+        if (__popc(__ballot_sync(active, leader)) <= SAH_GROUPS) {
+            for (int k = 0; k < 12; ++k)
+                key[k] = k % 6 < 3 ? __reduce_min_sync(peers, key[k]) : __reduce_max_sync(peers, key[k]);
+            cnt = (uint32_t)__popc(peers);
+            add = leader;
+        }
+        if (add)
+            for (int a = 0; a < 3; ++a) sah_add(bins + (a * SAH_BINS + b[a]) * SAH_W, cnt, key);
     }
     __syncwarp();
-    for (int i = T.first + lane; i < T.first + T.count; i += 32) {
-        const uint32_t p = perm[i];
-        const float4 lo = tbox[2ull * p], hi = tbox[2ull * p + 1], c = cen[p];
-        const float cv[3] = {c.x, c.y, c.z};
-        for (int a = 0; a < 3; ++a) sah_add(b + (a * SAH_BINS + sah_bin(cv[a], T.clo[a], T.chi[a])) * SAH_W, lo, hi, c);
-    }
-    __syncwarp();
-    uint32_t* g = bins + (size_t)t * SAH_TASK_WORDS;
-    for (int w = lane; w < SAH_TASK_WORDS; w += 32) g[w] = b[w];
 }
 
-// One block per SAH_BLOCK_ITEMS positions; a block whose positions all belong to one task (tasks
-// are contiguous ranges) bins into shared memory first.  Positions of tasks of at most SAH_SMALL
-// triangles are left to k_sah_bin_small.
-__global__ void __launch_bounds__(256) k_sah_bin(const uint32_t* __restrict__ perm, const int* __restrict__ task_of,
-                                                 const SahTask* __restrict__ tasks, const float4* __restrict__ tbox,
+// One block per SAH_BIN_TILE positions: each task with positions in the tile (a contiguous range) is binned in
+// shared memory, then added to the task's bins.
+__global__ void __launch_bounds__(SAH_BIN_TILE / 2) k_sah_bin(const uint32_t* __restrict__ perm, const int* __restrict__ task_of,
+                                                 const SahTask* __restrict__ tasks,
+                                                 const uint32_t* __restrict__ n_tasks, const float4* __restrict__ tbox,
                                                  const float4* __restrict__ cen, int n, uint32_t* __restrict__ bins) {
     __shared__ uint32_t sb[SAH_TASK_WORDS];
-    const int b0 = blockIdx.x * SAH_BLOCK_ITEMS, b1 = min(n, b0 + SAH_BLOCK_ITEMS);
-    if (b0 >= n) return;
-    const int t0 = task_of[b0], t1 = task_of[b1 - 1];
-    const bool priv = t0 >= 0 && t0 == t1;
-    if (priv && tasks[t0].count <= SAH_SMALL) return;   // block-uniform, before any barrier
-    if (priv) {
-        for (int w = threadIdx.x; w < SAH_TASK_WORDS; w += blockDim.x) {
-            const int k = w % SAH_W;
-            sb[w] = k == 0 ? 0u : (((k - 1) % 6) < 3 ? 0xFFFFFFFFu : 0u);
+    __shared__ int s_next;
+    if (!*n_tasks) return;
+    const int b0 = blockIdx.x * SAH_BIN_TILE, b1 = min(n, b0 + SAH_BIN_TILE);
+    for (int p = b0; p < b1;) {
+        const int t = task_of[p];   // the same for every thread
+        if (t < 0) {                // finished positions: to the next one with a task
+            __syncthreads();
+            if (threadIdx.x == 0) s_next = b1;
+            __syncthreads();
+            int q = b1;
+            for (int i = p + threadIdx.x; i < b1; i += blockDim.x)
+                if (task_of[i] >= 0) {
+                    q = i;
+                    break;
+                }
+            if (q < b1) atomicMin(&s_next, q);
+            __syncthreads();
+            p = s_next;
+            continue;
+        }
+        const SahTask T = tasks[t];
+        const int e = min(b1, T.first + T.count);
+        for (int w = threadIdx.x; w < SAH_TASK_WORDS; w += blockDim.x) sb[w] = sah_empty(w);
+        __syncthreads();
+        for (int i0 = p; i0 < e; i0 += blockDim.x) {
+            const int i = i0 + threadIdx.x;
+            const bool on = i < e;
+            float lo[3], hi[3], c[3];
+            if (on) {
+                const uint32_t q = perm[i];
+                const float4 l = tbox[2ull * q], h = tbox[2ull * q + 1], m = cen[q];
+                lo[0] = l.x; lo[1] = l.y; lo[2] = l.z;
+                hi[0] = h.x; hi[1] = h.y; hi[2] = h.z;
+                c[0] = m.x; c[1] = m.y; c[2] = m.z;
+            }
+            sah_bin_warp(sb, on, lo, hi, c, T.clo, T.chi);
         }
         __syncthreads();
-    }
-    for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-        const int t = task_of[i];
-        if (t < 0) continue;
-        const SahTask& T = tasks[t];
-        if (T.count <= SAH_SMALL) continue;
-        const uint32_t p = perm[i];
-        const float4 lo = tbox[2ull * p], hi = tbox[2ull * p + 1], c = cen[p];
-        const float cv[3] = {c.x, c.y, c.z};
-        uint32_t* base = priv ? sb : bins + (size_t)t * SAH_TASK_WORDS;
-        for (int a = 0; a < 3; ++a) sah_add(base + (a * SAH_BINS + sah_bin(cv[a], T.clo[a], T.chi[a])) * SAH_W, lo, hi, c);
-    }
-    if (priv) {
-        __syncthreads();
-        uint32_t* g = bins + (size_t)t0 * SAH_TASK_WORDS;
+        uint32_t* g = bins + (size_t)t * SAH_TASK_WORDS;
         for (int w = threadIdx.x; w < SAH_TASK_WORDS; w += blockDim.x) {
             const int k = w % SAH_W;
             const uint32_t v = sb[w];
-            if (k == 0) {
-                if (v) atomicAdd(&g[w], v);
-            } else if (((k - 1) % 6) < 3) {
-                if (v != 0xFFFFFFFFu) atomicMin(&g[w], v);
-            } else if (v) {
-                atomicMax(&g[w], v);
-            }
+            if (v == sah_empty(w)) continue;
+            if (k == 0) atomicAdd(&g[w], v);
+            else if (((k - 1) % 6) < 3) atomicMin(&g[w], v);
+            else atomicMax(&g[w], v);
         }
+        __syncthreads();
+        p = e;
     }
 }
 
@@ -1199,190 +1259,445 @@ __device__ __forceinline__ float sah_area(const float lo[3], const float hi[3]) 
     return dx * dy + dy * dz + dz * dx;
 }
 
-// One thread per task: the cheapest of the 3 x 15 bin boundaries by surface area x count.
-__global__ void k_sah_split(const SahTask* __restrict__ tasks, int n_tasks, const uint32_t* __restrict__ bins,
-                            SahSplit* __restrict__ splits) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tasks) return;
-    const SahTask T = tasks[t];
-    const uint32_t* B = bins + (size_t)t * SAH_TASK_WORDS;
+// The cheapest of the 3 x 15 bin boundaries by surface area x count (of equal ones the first axis, then the
+// first boundary), by one warp: a lane per bin, two axes at a time; prefix and suffix boxes by shuffles.
+__device__ __forceinline__ SahSplit sah_best_split(const uint32_t* B, const SahTask& T) {
+    const int lane = threadIdx.x & 31, bin = lane & 15;
     float best = 3.0e38f;
-    int ba = -1, bb = 0;
-    for (int a = 0; a < 3; ++a) {
-        if (!(T.chi[a] - T.clo[a] > 0.f)) continue;
-        // right sweep: area x count of bins [s, SAH_BINS)
-        float rcost[SAH_BINS];
-        float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    int where = 1 << 20;
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int a = 2 * pass + (lane >> 4);
         uint32_t cnt = 0;
-        for (int s = SAH_BINS - 1; s >= 1; --s) {
-            const uint32_t* w = B + (a * SAH_BINS + s) * SAH_W;
-            if (w[0]) {
-                cnt += w[0];
+        float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+        if (a < 3) {
+            const uint32_t* w = B + (a * SAH_BINS + bin) * SAH_W;
+            cnt = w[0];
+            if (cnt)
                 for (int k = 0; k < 3; ++k) {
-                    lo[k] = fminf(lo[k], fkey_inv(w[1 + k]));
-                    hi[k] = fmaxf(hi[k], fkey_inv(w[4 + k]));
+                    lo[k] = fkey_inv(w[1 + k]);
+                    hi[k] = fkey_inv(w[4 + k]);
                 }
-            }
-            rcost[s] = cnt ? sah_area(lo, hi) * (float)cnt : -1.f;
         }
-        for (int k = 0; k < 3; ++k) { lo[k] = 3.0e38f; hi[k] = -3.0e38f; }
-        cnt = 0;
-        for (int s = 1; s < SAH_BINS; ++s) {
-            const uint32_t* w = B + (a * SAH_BINS + s - 1) * SAH_W;
-            if (w[0]) {
-                cnt += w[0];
-                for (int k = 0; k < 3; ++k) {
-                    lo[k] = fminf(lo[k], fkey_inv(w[1 + k]));
-                    hi[k] = fmaxf(hi[k], fkey_inv(w[4 + k]));
-                }
+        uint32_t lc = cnt, rc = cnt;   // bins [0, bin], bins [bin, 16)
+        float llo[3], lhi[3], rlo[3], rhi[3];
+        for (int k = 0; k < 3; ++k) {
+            llo[k] = rlo[k] = lo[k];
+            lhi[k] = rhi[k] = hi[k];
+        }
+        for (int o = 1; o < 16; o <<= 1) {
+            const uint32_t uc = __shfl_up_sync(WARP, lc, o, 16), dc = __shfl_down_sync(WARP, rc, o, 16);
+            if (bin >= o) lc += uc;
+            if (bin + o < 16) rc += dc;
+            for (int k = 0; k < 3; ++k) {   // a lane without a source gets its own value back
+                llo[k] = fminf(llo[k], __shfl_up_sync(WARP, llo[k], o, 16));
+                lhi[k] = fmaxf(lhi[k], __shfl_up_sync(WARP, lhi[k], o, 16));
+                rlo[k] = fminf(rlo[k], __shfl_down_sync(WARP, rlo[k], o, 16));
+                rhi[k] = fmaxf(rhi[k], __shfl_down_sync(WARP, rhi[k], o, 16));
             }
-            if (cnt == 0 || rcost[s] < 0.f) continue;
-            const float c = sah_area(lo, hi) * (float)cnt + rcost[s];
+        }
+        // boundary `bin`: bins below it left, the others right
+        lc = __shfl_up_sync(WARP, lc, 1, 16);
+        for (int k = 0; k < 3; ++k) {
+            llo[k] = __shfl_up_sync(WARP, llo[k], 1, 16);
+            lhi[k] = __shfl_up_sync(WARP, lhi[k], 1, 16);
+        }
+        const float ext = a == 0 ? T.chi[0] - T.clo[0] : a == 1 ? T.chi[1] - T.clo[1] : T.chi[2] - T.clo[2];
+        if (a < 3 && bin >= 1 && ext > 0.f && lc && rc) {
+            const float c = __fmaf_rn(sah_area(llo, lhi), (float)lc, __fmul_rn(sah_area(rlo, rhi), (float)rc));
             if (c < best) {
                 best = c;
-                ba = a;
-                bb = s;
+                where = a * SAH_BINS + bin;
             }
         }
     }
+    for (int o = 1; o < 32; o <<= 1) {
+        const float c = __shfl_xor_sync(WARP, best, o);
+        const int v = __shfl_xor_sync(WARP, where, o);
+        if (c < best || (c == best && v < where)) {
+            best = c;
+            where = v;
+        }
+    }
     SahSplit S;
-    if (ba < 0) {
+    if (where == 1 << 20) {
         S.nl = T.count / 2;
         S.axis = -1;
         S.bin = 0;
         for (int k = 0; k < 3; ++k) {
-            S.lclo[k] = S.rclo[k] = T.clo[k];
-            S.lchi[k] = S.rchi[k] = T.chi[k];
+            S.clo[0][k] = S.clo[1][k] = T.clo[k];
+            S.chi[0][k] = S.chi[1][k] = T.chi[k];
         }
-    } else {
-        int nl = 0;
-        float llo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, lhi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-        float rlo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, rhi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-        for (int s = 0; s < SAH_BINS; ++s) {
-            const uint32_t* w = B + (ba * SAH_BINS + s) * SAH_W;
-            if (!w[0]) continue;
-            float* clo = s < bb ? llo : rlo;
-            float* chi = s < bb ? lhi : rhi;
-            if (s < bb) nl += (int)w[0];
-            for (int k = 0; k < 3; ++k) {
-                clo[k] = fminf(clo[k], fkey_inv(w[7 + k]));
-                chi[k] = fmaxf(chi[k], fkey_inv(w[10 + k]));
-            }
-        }
-        S.nl = nl;
-        S.axis = ba;
-        S.bin = bb;
-        for (int k = 0; k < 3; ++k) {
-            S.lclo[k] = llo[k];
-            S.lchi[k] = lhi[k];
-            S.rclo[k] = rlo[k];
-            S.rchi[k] = rhi[k];
-        }
+        return S;
     }
-    splits[t] = S;
-}
-
-__device__ __forceinline__ bool sah_left(const SahTask& T, const SahSplit& S, int i, const float4& c) {
-    if (S.axis < 0) return i - T.first < S.nl;
-    const float cv[3] = {c.x, c.y, c.z};
-    return sah_bin(cv[S.axis], T.clo[S.axis], T.chi[S.axis]) < S.bin;
-}
-
-__global__ void k_sah_flags(const uint32_t* __restrict__ perm, const int* __restrict__ task_of,
-                            const SahTask* __restrict__ tasks, const SahSplit* __restrict__ splits,
-                            const float4* __restrict__ cen, int n, uint32_t* __restrict__ flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int t = task_of[i];
-    flags[i] = t >= 0 && sah_left(tasks[t], splits[t], i, cen[perm[i]]) ? 1u : 0u;
-}
-
-// child-task and segment flags: [2t] left, [2t + 1] right
-__global__ void k_sah_child_flags(const SahTask* __restrict__ tasks, const SahSplit* __restrict__ splits, int n_tasks,
-                                  uint32_t* __restrict__ tflag, uint32_t* __restrict__ sflag) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tasks) return;
-    const int cl = splits[t].nl, cr = tasks[t].count - cl;
-    tflag[2 * t] = cl > SAH_T;
-    tflag[2 * t + 1] = cr > SAH_T;
-    sflag[2 * t] = cl <= SAH_T;
-    sflag[2 * t + 1] = cr <= SAH_T;
-}
-
-// Split nodes and the next level's tasks / final segments.  tscan / sscan: exclusive scans of the
-// child flags; seg_base: segments found by earlier levels.
-__global__ void k_sah_emit(const SahTask* __restrict__ tasks, const SahSplit* __restrict__ splits, int n_tasks,
-                           const uint32_t* __restrict__ tflag, const uint32_t* __restrict__ tscan,
-                           const uint32_t* __restrict__ sflag, const uint32_t* __restrict__ sscan, uint32_t seg_base,
-                           SahTask* __restrict__ next, SahSeg* __restrict__ segs, int2* __restrict__ child,
-                           int2* __restrict__ range, int* __restrict__ parent) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tasks) return;
-    const SahTask T = tasks[t];
-    const SahSplit S = splits[t];
-    const int X = T.first + S.nl - 1;
-    range[X] = make_int2(T.first, T.first + T.count - 1);
-    parent[X] = T.parent;
-    if (T.parent >= 0) {
-        if (T.side == 0) child[T.parent].x = X;
-        else child[T.parent].y = X;
+    S.axis = where / SAH_BINS;
+    S.bin = where % SAH_BINS;
+    const uint32_t* w = B + (S.axis * SAH_BINS + bin) * SAH_W;
+    const bool left = bin < S.bin;
+    S.nl = (int)__reduce_add_sync(WARP, lane < 16 && left ? w[0] : 0u);
+    for (int k = 0; k < 3; ++k) {   // empty bins hold the neutral keys
+        S.clo[0][k] = fkey_inv(__reduce_min_sync(WARP, left ? w[7 + k] : 0xFFFFFFFFu));
+        S.clo[1][k] = fkey_inv(__reduce_min_sync(WARP, left ? 0xFFFFFFFFu : w[7 + k]));
+        S.chi[0][k] = fkey_inv(__reduce_max_sync(WARP, left ? w[10 + k] : 0u));
+        S.chi[1][k] = fkey_inv(__reduce_max_sync(WARP, left ? 0u : w[10 + k]));
     }
-    for (int side = 0; side < 2; ++side) {
-        const int f = side ? T.first + S.nl : T.first;
-        const int c = side ? T.count - S.nl : S.nl;
-        if (tflag[2 * t + side]) {
+    return S;
+}
+
+// Split node of a task, by one lane: its range and links
+__device__ __forceinline__ int sah_node(const SahTree& tree, int first, int count, int nl, int parent, int side) {
+    const int X = first + nl - 1;
+    tree.range[X] = make_int2(first, first + count - 1);
+    tree.parent[X] = parent;
+    if (parent >= 0) {
+        if (side == 0) tree.child[parent].x = X;
+        else tree.child[parent].y = X;
+    }
+    return X;
+}
+
+// Final segment [first, first + count) under split node `parent`, by one lane
+__device__ __forceinline__ void sah_segment(const SahTree& tree, int first, int count, int parent, int side) {
+    for (int p = first; p < first + count; ++p) {
+        tree.seg_lo[p] = first;
+        tree.seg_hi[p] = first + count - 1;
+    }
+    const int root = count >= 2 ? first : ~first;
+    if (side == 0) tree.child[parent].x = root;
+    else tree.child[parent].y = root;
+    tree.parent[root >= 0 ? root : (tree.n - 1) + ~root] = parent;
+}
+
+// where a task of a level sends its triangles
+struct SahMove {
+    int nl, axis, bin;
+    int next[2];             // task of the next level of each child, -1: none
+    uint32_t before;         // left triangles before the task's first position in its tile (k_sah_flags)
+};
+
+// One warp per task of a level: its split, the node, and its children: tasks of the next level (bins
+// cleared), tasks of k_sah_subtree, or segments.
+__global__ void __launch_bounds__(128) k_sah_split(SahTree tree, const SahTask* __restrict__ tasks, int level,
+                                                   SahState* __restrict__ state, const uint32_t* __restrict__ bins,
+                                                   SahMove* __restrict__ moves, SahTask* __restrict__ next,
+                                                   uint32_t* __restrict__ next_bins, SahTask* __restrict__ sub) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t todo = state->n_tasks[level], warps = gridDim.x * 4;
+    for (uint32_t t = blockIdx.x * 4 + (threadIdx.x >> 5); t < todo; t += warps) {
+        const SahTask T = tasks[t];
+        const SahSplit S = sah_best_split(bins + (size_t)t * SAH_TASK_WORDS, T);
+        int X = 0, slot[2] = {-1, -1};
+        if (lane == 0) {
+            X = sah_node(tree, T.first, T.count, S.nl, T.parent, T.side);
+            if (T.parent < 0) state->root = X;
+        }
+        for (int side = 0; side < 2; ++side) {
             SahTask C;
-            C.first = f;
-            C.count = c;
+            C.first = side ? T.first + S.nl : T.first;
+            C.count = side ? T.count - S.nl : S.nl;
             for (int k = 0; k < 3; ++k) {
-                C.clo[k] = side ? S.rclo[k] : S.lclo[k];
-                C.chi[k] = side ? S.rchi[k] : S.lchi[k];
+                C.clo[k] = S.clo[side][k];
+                C.chi[k] = S.chi[side][k];
             }
             C.parent = X;
             C.side = side;
-            next[tscan[2 * t + side]] = C;
-        } else if (sflag[2 * t + side]) {
-            segs[seg_base + sscan[2 * t + side]] = SahSeg{f, c, X, side};
+            if (C.count > SAH_SUB) {
+                if (lane == 0) {
+                    slot[side] = (int)atomicAdd(&state->n_tasks[level + 1], 1u);
+                    next[slot[side]] = C;
+                }
+                slot[side] = __shfl_sync(WARP, slot[side], 0);
+                for (int w = lane; w < SAH_TASK_WORDS; w += 32) next_bins[(size_t)slot[side] * SAH_TASK_WORDS + w] = sah_empty(w);
+            } else if (lane == 0) {
+                if (C.count > SAH_T) sub[atomicAdd(&state->n_sub, 1u)] = C;
+                else sah_segment(tree, C.first, C.count, X, side);
+            }
+        }
+        if (lane == 0) moves[t] = SahMove{S.nl, S.axis, S.bin, {slot[0], slot[1]}, 0u};
+    }
+}
+
+__device__ __forceinline__ bool sah_left(const SahTask& T, const SahMove& S, int i, const float4& c) {
+    if (S.axis < 0) return i - T.first < S.nl;
+    const float v = S.axis == 0 ? c.x : S.axis == 1 ? c.y : c.z;
+    return sah_bin(v, T.clo[S.axis], T.chi[S.axis]) < S.bin;
+}
+
+// Exclusive prefix over the words of left flags of a block (at most 32, in shared memory), by one warp;
+// returns their number of left flags.
+constexpr int SAH_WORDS = SAH_TILE / 32;
+static_assert(SAH_WORDS == 32 && SAH_SUB <= SAH_TILE, "one word per lane");
+__device__ __forceinline__ uint32_t sah_word_scan(const uint32_t* words, int n_words, uint32_t* prefix) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t v = lane < n_words ? (uint32_t)__popc(words[lane]) : 0u;
+    uint32_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(WARP, x, o);
+        if (lane >= o) x += y;
+    }
+    prefix[lane] = x - v;
+    return __shfl_sync(WARP, x, 31);
+}
+
+__global__ void __launch_bounds__(256) k_sah_flags(const uint32_t* __restrict__ perm, const int* __restrict__ task_of,
+                                                   const SahTask* __restrict__ tasks,
+                                                   const uint32_t* __restrict__ n_tasks, SahMove* __restrict__ moves,
+                                                   const float4* __restrict__ cen, int n, uint32_t* __restrict__ flags,
+                                                   uint32_t* __restrict__ tile_total) {
+    __shared__ uint32_t words[SAH_WORDS], prefix[SAH_WORDS];
+    if (!*n_tasks) return;
+    const int b0 = blockIdx.x * SAH_TILE, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t firsts = 0;   // of this thread's positions, those that begin a task
+#pragma unroll
+    for (int j = 0; j < SAH_TILE / 256; ++j) {
+        const int i = b0 + j * 256 + threadIdx.x;
+        bool left = false;
+        if (i < n) {
+            const int t = task_of[i];
+            if (t >= 0) {
+                const SahTask& T = tasks[t];
+                left = sah_left(T, moves[t], i, cen[perm[i]]);
+                if (i == T.first) firsts |= 1u << j;
+            }
+        }
+        const uint32_t m = __ballot_sync(WARP, left);
+        if (lane == 0) words[j * 8 + warp] = flags[(size_t)blockIdx.x * SAH_WORDS + j * 8 + warp] = m;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t total = sah_word_scan(words, SAH_WORDS, prefix);
+        if (lane == 0) tile_total[blockIdx.x] = total;
+    }
+    __syncthreads();
+    for (int j = 0; j < SAH_TILE / 256; ++j)
+        if ((firsts >> j) & 1u)
+            moves[task_of[b0 + j * 256 + threadIdx.x]].before = prefix[j * 8 + warp] +
+                                                               (uint32_t)__popc(words[j * 8 + warp] & ((1u << lane) - 1u));
+}
+
+// Stable partition of every task's range; finished positions move along.
+__global__ void __launch_bounds__(256) k_sah_scatter(const uint32_t* __restrict__ perm_in, uint32_t* __restrict__ perm_out,
+                                                     const int* __restrict__ task_in, int* __restrict__ task_out,
+                                                     const SahTask* __restrict__ tasks,
+                                                     const uint32_t* __restrict__ n_tasks,
+                                                     const SahMove* __restrict__ moves, int n,
+                                                     const uint32_t* __restrict__ flags,
+                                                     const uint32_t* __restrict__ tile_first) {
+    __shared__ uint32_t words[SAH_WORDS], prefix[SAH_WORDS];
+    if (!*n_tasks) return;
+    const int b0 = blockIdx.x * SAH_TILE, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        words[lane] = flags[(size_t)blockIdx.x * SAH_WORDS + lane];
+        __syncwarp();
+        sah_word_scan(words, SAH_WORDS, prefix);
+    }
+    __syncthreads();
+    const uint32_t here = tile_first[blockIdx.x];
+#pragma unroll
+    for (int j = 0; j < SAH_TILE / 256; ++j) {
+        const int i = b0 + j * 256 + threadIdx.x;
+        if (i >= n) break;
+        const int t = task_in[i];
+        int pos = i, to = -1;
+        if (t >= 0) {
+            const SahMove& S = moves[t];
+            const int f = tasks[t].first;
+            const uint32_t m = words[j * 8 + warp];
+            const uint32_t scan = here + prefix[j * 8 + warp] + (uint32_t)__popc(m & ((1u << lane) - 1u));
+            const int lr = (int)(scan - (tile_first[f / SAH_TILE] + S.before));   // left triangles before i in the task
+            const bool left = (m >> lane) & 1u;
+            pos = left ? f + lr : f + S.nl + (i - f - lr);
+            to = S.next[left ? 0 : 1];
+        }
+        perm_out[pos] = perm_in[i];
+        task_out[pos] = to;
+    }
+}
+
+// One block takes a task of at most SAH_SUB triangles to its segments: boxes, centroids and the order in
+// shared memory.  Per level, tasks of more than SUB_WIDE triangles are taken by all warps, one after the
+// other, the rest by a warp each.  The task's part of `sorted` is read first and rewritten segment by
+// segment.
+struct SubTask {
+    float clo[3], chi[3];
+    int parent;
+    uint16_t first, count;   // within the block's task
+    uint16_t side, pad;
+};
+constexpr int SUB_TASKS = SAH_SUB / (SAH_T + 1) + 1, SUB_WARPS = 8, SUB_WIDE = 96;
+struct SubShared {
+    float lo[3][SAH_SUB], hi[3][SAH_SUB], c[3][SAH_SUB];
+    uint32_t prim[SAH_SUB];
+    uint32_t bins[SUB_WARPS][SAH_TASK_WORDS];
+    SubTask tasks[2][SUB_TASKS];
+    SahSplit split;
+    uint32_t words[32], prefix[32];
+    uint16_t order[2][SAH_SUB];
+    uint32_t n_tasks[2];
+};
+
+// The split node of a block-local task and its children, by one warp, after the task's part of order[cur ^ 1]
+// has been written
+__device__ __forceinline__ void sub_children(SubShared& M, const SahTree& tree, SahState* state, uint32_t* sorted,
+                                             int block_first, int cur, const SahTask& T, const SahSplit& S) {
+    const int lane = threadIdx.x & 31;
+    int X = 0;
+    if (lane == 0) {
+        X = sah_node(tree, block_first + T.first, T.count, S.nl, T.parent, T.side);
+        if (T.parent < 0) state->root = X;
+    }
+    for (int sd = 0; sd < 2; ++sd) {
+        const int f = sd ? T.first + S.nl : T.first, cnt = sd ? T.count - S.nl : S.nl;
+        if (cnt > SAH_T) {
+            if (lane == 0) {
+                SubTask& C = M.tasks[cur ^ 1][atomicAdd(&M.n_tasks[cur ^ 1], 1u)];
+                for (int k = 0; k < 3; ++k) {
+                    C.clo[k] = S.clo[sd][k];
+                    C.chi[k] = S.chi[sd][k];
+                }
+                C.parent = X;
+                C.first = (uint16_t)f;
+                C.count = (uint16_t)cnt;
+                C.side = (uint16_t)sd;
+            }
+        } else {
+            if (lane < cnt) sorted[block_first + f + lane] = M.prim[M.order[cur ^ 1][f + lane]];
+            if (lane == 0) sah_segment(tree, block_first + f, cnt, X, sd);
         }
     }
+    __syncwarp();
 }
 
-__global__ void k_sah_scatter(const uint32_t* __restrict__ perm_in, uint32_t* __restrict__ perm_out,
-                              const int* __restrict__ task_in, int* __restrict__ task_out,
-                              const SahTask* __restrict__ tasks, const SahSplit* __restrict__ splits,
-                              const uint32_t* __restrict__ flags, const uint32_t* __restrict__ scan,
-                              const uint32_t* __restrict__ tflag, const uint32_t* __restrict__ tscan, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int t = task_in[i];
-    if (t < 0) {
-        perm_out[i] = perm_in[i];
-        task_out[i] = -1;
-        return;
-    }
-    const int f = tasks[t].first, nl = splits[t].nl;
-    const int lr = (int)(scan[i] - scan[f]);   // left items before i in this task
-    const bool left = flags[i] != 0;
-    const int pos = left ? f + lr : f + nl + (i - f - lr);
-    const int side = left ? 0 : 1;
-    perm_out[pos] = perm_in[i];
-    task_out[pos] = tflag[2 * t + side] ? (int)tscan[2 * t + side] : -1;
-}
-
-__global__ void k_sah_segments(const SahSeg* __restrict__ segs, int n_segs, int n, int* __restrict__ seg_lo,
-                               int* __restrict__ seg_hi, int2* __restrict__ child, int* __restrict__ parent) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_segs) return;
-    const SahSeg S = segs[s];
-    for (int p = S.first; p < S.first + S.count; ++p) {
-        seg_lo[p] = S.first;
-        seg_hi[p] = S.first + S.count - 1;
-    }
-    const int root = S.count >= 2 ? S.first : ~S.first;
-    if (S.parent >= 0) {
-        if (S.side == 0) child[S.parent].x = root;
-        else child[S.parent].y = root;
-        parent[root >= 0 ? root : (n - 1) + ~root] = S.parent;
+__global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree(SahTree tree, const SahTask* __restrict__ sub,
+                                                                SahState* __restrict__ state,
+                                                                const float4* __restrict__ tbox,
+                                                                const float4* __restrict__ cen, uint32_t* sorted) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    SubShared& M = *reinterpret_cast<SubShared*>(sub_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    auto task = [&](int cur, uint32_t t) {
+        const SubTask& U = M.tasks[cur][t];
+        SahTask T;
+        for (int k = 0; k < 3; ++k) {
+            T.clo[k] = U.clo[k];
+            T.chi[k] = U.chi[k];
+        }
+        T.first = U.first;
+        T.count = U.count;
+        T.parent = U.parent;
+        T.side = U.side;
+        return T;
+    };
+    // bins the 32 positions from i0 of task T (order[cur]) with one warp
+    auto bin_chunk = [&](uint32_t* bins, int cur, const SahTask& T, int i0) {
+        const bool on = i0 + lane < T.count;
+        float lo[3], hi[3], c[3];
+        if (on) {
+            const int q = M.order[cur][T.first + i0 + lane];
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = M.lo[k][q];
+                hi[k] = M.hi[k][q];
+                c[k] = M.c[k][q];
+            }
+        }
+        sah_bin_warp(bins, on, lo, hi, c, T.clo, T.chi);
+    };
+    // item and left flag of position i0 + lane
+    auto side_of = [&](int cur, const SahTask& T, const SahSplit& S, int i0, int& q) {
+        q = 0;
+        if (i0 + lane >= T.count) return false;
+        q = M.order[cur][T.first + i0 + lane];
+        if (S.axis < 0) return i0 + lane < S.nl;
+        const float lo = S.axis == 0 ? T.clo[0] : S.axis == 1 ? T.clo[1] : T.clo[2];
+        const float hi = S.axis == 0 ? T.chi[0] : S.axis == 1 ? T.chi[1] : T.chi[2];
+        return sah_bin(M.c[S.axis][q], lo, hi) < S.bin;
+    };
+    const uint32_t todo = state->n_sub;
+    for (uint32_t item = blockIdx.x; item < todo; item += gridDim.x) {
+        const SahTask R = sub[item];
+        for (int i = threadIdx.x; i < R.count; i += blockDim.x) {
+            const uint32_t p = sorted[R.first + i];
+            const float4 l = tbox[2ull * p], h = tbox[2ull * p + 1], m = cen[p];
+            M.prim[i] = p;
+            M.lo[0][i] = l.x; M.lo[1][i] = l.y; M.lo[2][i] = l.z;
+            M.hi[0][i] = h.x; M.hi[1][i] = h.y; M.hi[2][i] = h.z;
+            M.c[0][i] = m.x; M.c[1][i] = m.y; M.c[2][i] = m.z;
+            M.order[0][i] = (uint16_t)i;
+        }
+        if (threadIdx.x == 0) {
+            SubTask& T = M.tasks[0][0];
+            for (int k = 0; k < 3; ++k) {
+                T.clo[k] = R.clo[k];
+                T.chi[k] = R.chi[k];
+            }
+            T.parent = R.parent;
+            T.first = 0;
+            T.count = (uint16_t)R.count;
+            T.side = (uint16_t)R.side;
+            M.n_tasks[0] = 1;
+            M.n_tasks[1] = 0;
+        }
+        __syncthreads();
+        for (int cur = 0; M.n_tasks[cur]; cur ^= 1) {
+            const uint32_t nt = M.n_tasks[cur];
+            for (uint32_t t = 0; t < nt; ++t) {   // wide tasks: the whole block
+                if (M.tasks[cur][t].count <= SUB_WIDE) continue;
+                const SahTask T = task(cur, t);
+                for (int w = threadIdx.x; w < SAH_TASK_WORDS; w += blockDim.x) M.bins[0][w] = sah_empty(w);
+                __syncthreads();
+                for (int i0 = 32 * warp; i0 < T.count; i0 += 32 * SUB_WARPS) bin_chunk(M.bins[0], cur, T, i0);
+                __syncthreads();
+                if (warp == 0) {
+                    const SahSplit S = sah_best_split(M.bins[0], T);
+                    if (lane == 0) M.split = S;
+                }
+                __syncthreads();
+                const SahSplit S = M.split;
+                for (int i0 = 32 * warp; i0 < T.count; i0 += 32 * SUB_WARPS) {
+                    int q;
+                    const uint32_t m = __ballot_sync(WARP, side_of(cur, T, S, i0, q));
+                    if (lane == 0) M.words[i0 / 32] = m;
+                }
+                __syncthreads();
+                if (warp == 0) sah_word_scan(M.words, (T.count + 31) / 32, M.prefix);
+                __syncthreads();
+                for (int i0 = 32 * warp; i0 < T.count; i0 += 32 * SUB_WARPS) {
+                    const int i = i0 + lane;
+                    if (i >= T.count) continue;
+                    const uint32_t m = M.words[i0 / 32];
+                    const int lr = (int)(M.prefix[i0 / 32] + (uint32_t)__popc(m & lt));
+                    M.order[cur ^ 1][T.first + ((m >> lane) & 1u ? lr : S.nl + (i - lr))] = M.order[cur][T.first + i];
+                }
+                __syncthreads();
+                if (warp == 0) sub_children(M, tree, state, sorted, R.first, cur, T, S);
+            }
+            __syncthreads();
+            for (uint32_t t = warp; t < nt; t += SUB_WARPS) {
+                if (M.tasks[cur][t].count > SUB_WIDE) continue;
+                const SahTask T = task(cur, t);
+                uint32_t* bins = M.bins[warp];
+                for (int w = lane; w < SAH_TASK_WORDS; w += 32) bins[w] = sah_empty(w);
+                __syncwarp();
+                for (int i0 = 0; i0 < T.count; i0 += 32) bin_chunk(bins, cur, T, i0);
+                const SahSplit S = sah_best_split(bins, T);
+                int nleft = 0;   // stable partition into the other order
+                for (int i0 = 0; i0 < T.count; i0 += 32) {
+                    int q;
+                    const uint32_t m = __ballot_sync(WARP, side_of(cur, T, S, i0, q));
+                    const int lr = nleft + __popc(m & lt);
+                    if (i0 + lane < T.count)
+                        M.order[cur ^ 1][T.first + ((m >> lane) & 1u ? lr : S.nl + (i0 + lane - lr))] = (uint16_t)q;
+                    nleft += __popc(m);
+                }
+                __syncwarp();
+                sub_children(M, tree, state, sorted, R.first, cur, T, S);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) M.n_tasks[cur] = 0;
+            __syncthreads();
+        }
+        __syncthreads();   // every thread has left the loop before the next task is set up
     }
 }
 
@@ -1432,149 +1747,90 @@ __global__ void k_karras_seg(const uint32_t* __restrict__ code, int n, const int
     parent[right >= 0 ? right : (n - 1) + ~right] = i;
 }
 
-// exclusive scan, multi-block: per-block totals, one-block scan of the totals, per-block scan
-constexpr int SCAN_ITEMS = 2048;
-__global__ void __launch_bounds__(256) k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                     uint32_t m, uint32_t* __restrict__ totals) {
-    __shared__ uint32_t part[256];
-    const uint32_t b0 = blockIdx.x * SCAN_ITEMS + threadIdx.x * 8;
-    uint32_t v[8], s = 0;
-    for (int k = 0; k < 8; ++k) {
-        v[k] = b0 + k < m ? in[b0 + k] : 0u;
-        s += v[k];
-    }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {
-        const uint32_t x = threadIdx.x >= (uint32_t)off ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += x;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - s;
-    for (int k = 0; k < 8; ++k) {
-        if (b0 + k < m) out[b0 + k] = run;
-        run += v[k];
-    }
-    if (threadIdx.x == 255) totals[blockIdx.x] = part[255];
-}
-
-__global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t m, const uint32_t* __restrict__ totals) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) out[i] += totals[i / SCAN_ITEMS];
-}
-
-void scan_exclusive(crt_context* ctx, const uint32_t* in, uint32_t* out, uint32_t m, uint32_t* totals) {
-    if (!m) return;
-    cudaStream_t st = ctx->stream;
-    const uint32_t nb = (m + SCAN_ITEMS - 1) / SCAN_ITEMS;
-    k_scan_blocks<<<nb, 256, 0, st>>>(in, out, m, totals);
-    check_launch(ctx, "k_scan_blocks");
-    k_scan<<<1, 1024, 0, st>>>(totals, nb);
-    check_launch(ctx, "k_scan");
-    k_scan_add<<<(m + 255) / 256, 256, 0, st>>>(out, m, totals);
-    check_launch(ctx, "k_scan_add");
-}
-
 // Binned-SAH binary tree over the Morton-sorted triangles (n > SAH_T): fills child / range / parent
-// like k_karras and writes the triangle order of the tree's leaves to `sorted` (in place of the
-// Morton order).  Returns the root's internal index, or -1 (with nothing modified) when its
-// temporaries (about 0.6 GB per million triangles) cannot be allocated.
-int sah_topology(crt_context* ctx, int n, const float4* tbox, const float4* cen, const uint32_t* keys,
-                 uint32_t* sorted, const uint32_t* code_by_prim, int2* child, int2* range, int* parent) {
+// like k_karras, writes the triangle order of the tree's leaves to `sorted` (in place of the Morton order)
+// and the root's internal index to *root (device memory).  Returns false, with nothing modified, when its
+// temporaries (about 60 bytes per triangle) cannot be allocated.
+bool sah_topology(crt_context* ctx, int n, const float4* tbox, const float4* cen, const uint32_t* keys,
+                  uint32_t* sorted, const uint32_t* code_by_prim, int2* child, int2* range, int* parent, int2* root) {
     cudaStream_t st = ctx->stream;
-    const size_t max_tasks = (size_t)n / (SAH_T + 1) + 2;
-    const size_t max_segs = (size_t)n;
-    char* mem = nullptr;
+    const size_t max_tasks = (size_t)n / SAH_SUB + 2;   // of one level: disjoint ranges of more than SAH_SUB
+    const uint32_t tiles = (uint32_t)(((size_t)n + SAH_TILE - 1) / SAH_TILE);
+    const uint32_t bin_tiles = (uint32_t)(((size_t)n + SAH_BIN_TILE - 1) / SAH_BIN_TILE);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t o_perm = take(4ull * n), o_task0 = take(4ull * n), o_task1 = take(4ull * n), o_flags = take(4ull * n),
-                 o_scan = take(4ull * n), o_tot = take(4ull * ((2 * max_tasks + n) / SCAN_ITEMS + 2)),
+    const size_t o_perm = take(4ull * n), o_task0 = take(4ull * n), o_task1 = take(4ull * n),
+                 o_flags = take(4ull * SAH_WORDS * tiles), o_tiles = take(4ull * tiles), o_state = take(sizeof(SahState)),
                  o_tasks0 = take(sizeof(SahTask) * max_tasks), o_tasks1 = take(sizeof(SahTask) * max_tasks),
-                 o_split = take(sizeof(SahSplit) * max_tasks), o_bins = take(4ull * SAH_TASK_WORDS * max_tasks),
-                 o_tf = take(8ull * max_tasks), o_ts = take(8ull * max_tasks), o_sf = take(8ull * max_tasks),
-                 o_ss = take(8ull * max_tasks), o_segs = take(sizeof(SahSeg) * max_segs), o_lo = take(4ull * n),
-                 o_hi = take(4ull * n), o_code = take(4ull * n);
-    if (cudaMalloc(&mem, off) != cudaSuccess) {   // nothing modified yet: the caller builds a radix tree
+                 o_moves = take(sizeof(SahMove) * max_tasks), o_bins0 = take(4ull * SAH_TASK_WORDS * max_tasks),
+                 o_bins1 = take(4ull * SAH_TASK_WORDS * max_tasks), o_sub = take(sizeof(SahTask) * ((size_t)n / (SAH_T + 1) + 2)),
+                 o_lo = take(4ull * n), o_hi = take(4ull * n), o_code = take(4ull * n);
+    char* mem = nullptr;
+    try {
+        mem = (char*)ctx_scratch(ctx, SCR_BUILD3, off);
+    } catch (const CrtError& e) {   // nothing modified yet: the caller builds a radix tree
+        if (e.status != CRT_ERR_OOM) throw;
         cudaGetLastError();
-        return -1;
+        return false;
     }
-    struct Free {
-        char* p;
-        ~Free() { cudaFree(p); }
-    } guard{mem};
     uint32_t* perm[2] = {sorted, (uint32_t*)(mem + o_perm)};
     int* task_of[2] = {(int*)(mem + o_task0), (int*)(mem + o_task1)};
-    uint32_t* flags = (uint32_t*)(mem + o_flags);
-    uint32_t* scan = (uint32_t*)(mem + o_scan);
-    uint32_t* totals = (uint32_t*)(mem + o_tot);
+    uint32_t *flags = (uint32_t*)(mem + o_flags), *tile = (uint32_t*)(mem + o_tiles);
+    SahState* state = (SahState*)(mem + o_state);
     SahTask* tasks[2] = {(SahTask*)(mem + o_tasks0), (SahTask*)(mem + o_tasks1)};
-    SahSplit* splits = (SahSplit*)(mem + o_split);
-    uint32_t* bins = (uint32_t*)(mem + o_bins);
-    uint32_t *tflag = (uint32_t*)(mem + o_tf), *tscan = (uint32_t*)(mem + o_ts);
-    uint32_t *sflag = (uint32_t*)(mem + o_sf), *sscan = (uint32_t*)(mem + o_ss);
-    SahSeg* segs = (SahSeg*)(mem + o_segs);
-    int *seg_lo = (int*)(mem + o_lo), *seg_hi = (int*)(mem + o_hi);
+    SahMove* moves = (SahMove*)(mem + o_moves);
+    uint32_t* bins[2] = {(uint32_t*)(mem + o_bins0), (uint32_t*)(mem + o_bins1)};
+    SahTask* sub = (SahTask*)(mem + o_sub);
     uint32_t* code = (uint32_t*)(mem + o_code);
+    const SahTree tree{n, child, range, parent, (int*)(mem + o_lo), (int*)(mem + o_hi)};
 
     CRT_CUDA(cudaMemsetAsync(task_of[0], 0, 4ull * n, st));   // every position in task 0 (the root)
-    k_sah_root<<<1, 1, 0, st>>>(keys, n, tasks[0]);
+    k_sah_root<<<1, 256, 0, st>>>(keys, n, tasks[0], sub, bins[0], state);
     check_launch(ctx, "k_sah_root");
-    int cur = 0, n_tasks = 1, root = -1;
-    uint32_t n_segs = 0;
-    for (int level = 0; n_tasks > 0; ++level) {
-        CRT_CHECK(level < 256 && (size_t)n_tasks <= max_tasks, CRT_ERR_DEVICE, "SAH build did not converge");
-        const size_t words = (size_t)n_tasks * SAH_TASK_WORDS;
-        k_sah_clear<<<(uint32_t)std::min<size_t>((words + 255) / 256, 4096), 256, 0, st>>>(bins, words);
-        check_launch(ctx, "k_sah_clear");
-        k_sah_bin<<<(n + SAH_BLOCK_ITEMS - 1) / SAH_BLOCK_ITEMS, 256, 0, st>>>(perm[cur], task_of[cur], tasks[cur],
-                                                                              tbox, cen, n, bins);
-        check_launch(ctx, "k_sah_bin");
-        k_sah_bin_small<<<(n_tasks + 7) / 8, 256, 0, st>>>(perm[cur], tasks[cur], n_tasks, tbox, cen, bins);
-        check_launch(ctx, "k_sah_bin_small");
-        k_sah_split<<<(n_tasks + 127) / 128, 128, 0, st>>>(tasks[cur], n_tasks, bins, splits);
-        check_launch(ctx, "k_sah_split");
-        k_sah_flags<<<(n + 255) / 256, 256, 0, st>>>(perm[cur], task_of[cur], tasks[cur], splits, cen, n, flags);
-        check_launch(ctx, "k_sah_flags");
-        scan_exclusive(ctx, flags, scan, (uint32_t)n, totals);
-        k_sah_child_flags<<<(n_tasks + 255) / 256, 256, 0, st>>>(tasks[cur], splits, n_tasks, tflag, sflag);
-        check_launch(ctx, "k_sah_child_flags");
-        scan_exclusive(ctx, tflag, tscan, 2u * n_tasks, totals);
-        scan_exclusive(ctx, sflag, sscan, 2u * n_tasks, totals);
-        k_sah_emit<<<(n_tasks + 255) / 256, 256, 0, st>>>(tasks[cur], splits, n_tasks, tflag, tscan, sflag, sscan, n_segs,
-                                                          tasks[cur ^ 1], segs, child, range, parent);
-        check_launch(ctx, "k_sah_emit");
-        k_sah_scatter<<<(n + 255) / 256, 256, 0, st>>>(perm[cur], perm[cur ^ 1], task_of[cur], task_of[cur ^ 1],
-                                                       tasks[cur], splits, flags, scan, tflag, tscan, n);
-        check_launch(ctx, "k_sah_scatter");
-        if (level == 0) {
-            int nl = 0;
-            CRT_CUDA(cudaMemcpyAsync(&nl, &splits[0].nl, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // levels of tasks larger than SAH_SUB: as many as a balanced tree has and three more, then a look
+    // at the task counts, then four at a time
+    int levels = 0;
+    if (n > SAH_SUB) {
+        uint32_t h[SAH_MAX_LEVELS + 1];
+        int batch = 3;
+        for (int m = n; m > SAH_SUB; m = (m + 1) / 2) ++batch;
+        for (int launched = 0;;) {
+            CRT_CHECK(launched + batch <= SAH_MAX_LEVELS, CRT_ERR_DEVICE, "SAH build did not converge");
+            for (int b = 0; b < batch; ++b, ++launched) {
+                const int cur = launched & 1, nxt = cur ^ 1;
+                const uint32_t* nt = &state->n_tasks[launched];
+                k_sah_bin<<<bin_tiles, SAH_BIN_TILE / 2, 0, st>>>(perm[cur], task_of[cur], tasks[cur], nt, tbox, cen, n, bins[cur]);
+                check_launch(ctx, "k_sah_bin");
+                const size_t bound = std::min<size_t>(launched < 30 ? size_t(1) << launched : max_tasks, max_tasks);
+                k_sah_split<<<(uint32_t)std::min<size_t>((bound + 3) / 4, (size_t)ctx->sm_count * 8), 128, 0, st>>>(
+                    tree, tasks[cur], launched, state, bins[cur], moves, tasks[nxt], bins[nxt], sub);
+                check_launch(ctx, "k_sah_split");
+                k_sah_flags<<<tiles, 256, 0, st>>>(perm[cur], task_of[cur], tasks[cur], nt, moves, cen, n, flags, tile);
+                check_launch(ctx, "k_sah_flags");
+                k_scan<<<1, 1024, 0, st>>>(tile, tiles);
+                check_launch(ctx, "k_scan");
+                k_sah_scatter<<<tiles, 256, 0, st>>>(perm[cur], perm[nxt], task_of[cur], task_of[nxt], tasks[cur], nt,
+                                                     moves, n, flags, tile);
+                check_launch(ctx, "k_sah_scatter");
+            }
+            CRT_CUDA(cudaMemcpyAsync(h, state->n_tasks, sizeof(uint32_t) * (launched + 1), cudaMemcpyDeviceToHost, st));
             CRT_CUDA(cudaStreamSynchronize(st));
-            root = nl - 1;
+            while (levels < launched && h[levels]) ++levels;
+            if (!h[launched]) break;
+            batch = 4;
         }
-        // next level's task count and the segment count: last exclusive-scan value + last flag
-        uint32_t h[4];
-        CRT_CUDA(cudaMemcpyAsync(&h[0], tscan + 2 * n_tasks - 1, 4, cudaMemcpyDeviceToHost, st));
-        CRT_CUDA(cudaMemcpyAsync(&h[1], tflag + 2 * n_tasks - 1, 4, cudaMemcpyDeviceToHost, st));
-        CRT_CUDA(cudaMemcpyAsync(&h[2], sscan + 2 * n_tasks - 1, 4, cudaMemcpyDeviceToHost, st));
-        CRT_CUDA(cudaMemcpyAsync(&h[3], sflag + 2 * n_tasks - 1, 4, cudaMemcpyDeviceToHost, st));
-        CRT_CUDA(cudaStreamSynchronize(st));
-        n_tasks = (int)(h[0] + h[1]);
-        n_segs += h[2] + h[3];
-        CRT_CHECK(n_segs <= max_segs, CRT_ERR_DEVICE, "SAH build: too many segments");
-        cur ^= 1;
     }
-    if (perm[cur] != sorted)
-        CRT_CUDA(cudaMemcpyAsync(sorted, perm[cur], 4ull * n, cudaMemcpyDeviceToDevice, st));
-    k_sah_segments<<<(n_segs + 255) / 256, 256, 0, st>>>(segs, (int)n_segs, n, seg_lo, seg_hi, child, parent);
-    check_launch(ctx, "k_sah_segments");
+    if (levels & 1) CRT_CUDA(cudaMemcpyAsync(sorted, perm[1], 4ull * n, cudaMemcpyDeviceToDevice, st));
+    CRT_CUDA(cudaFuncSetAttribute(k_sah_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SubShared)));
+    const uint32_t blocks = (uint32_t)std::min<size_t>((size_t)n / 64 + 1, (size_t)ctx->sm_count * 8);
+    k_sah_subtree<<<blocks, 32 * SUB_WARPS, sizeof(SubShared), st>>>(tree, sub, state, tbox, cen, sorted);
+    check_launch(ctx, "k_sah_subtree");
+    CRT_CUDA(cudaMemcpyAsync(&root->x, &state->root, sizeof(int), cudaMemcpyDeviceToDevice, st));
     k_gather_codes<<<(n + 255) / 256, 256, 0, st>>>(sorted, code_by_prim, n, code);
     check_launch(ctx, "k_gather_codes");
-    k_karras_seg<<<(n + 254) / 256, 256, 0, st>>>(code, n, seg_lo, seg_hi, child, range, parent);
+    k_karras_seg<<<(n + 254) / 256, 256, 0, st>>>(code, n, tree.seg_lo, tree.seg_hi, child, range, parent);
     check_launch(ctx, "k_karras_seg");
-    CRT_CUDA(cudaStreamSynchronize(st));   // the temporaries are released on return
-    return root;
+    return true;
 }
 
 inline uint32_t cdiv(size_t a, uint32_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -1631,7 +1887,7 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     // binned-SAH topology for scenes larger than one segment (the context's build setting), else
     // Karras' radix tree over the Morton order
     const bool sah = ctx->build_sah && n > (uint32_t)SAH_T;
-    int root_index = 0;
+    bool sah_built = false;   // its root is in front[0] on the device, else it is internal node 0
     // scratch layout
     float* d_xyz = (float*)ctx_scratch(ctx, SCR_BUILD0, nn * 9 * sizeof(float));
     float* d_vnin = any_vn ? (float*)ctx_scratch(ctx, SCR_BUILD1, nn * 9 * sizeof(float)) : nullptr;
@@ -1720,9 +1976,8 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
             std::swap(va, vb);
         }
         // after 4 passes the sorted data is back in (code_a, idx_a)
-        if (sah) root_index = sah_topology(ctx, (int)n, tbox, cen, keys, va, code_prim, child, range, parent);
-        if ((!sah || root_index < 0) && n > 1) {   // radix tree (also when the SAH temporaries do not fit)
-            root_index = 0;
+        sah_built = sah && sah_topology(ctx, (int)n, tbox, cen, keys, va, code_prim, child, range, parent, front);
+        if (!sah_built && n > 1) {   // radix tree (also when the SAH temporaries do not fit)
             k_karras<<<cdiv(n - 1, BLOCK), BLOCK, 0, st>>>(ka, (int)n, child, range, parent);
             check_launch(ctx, "k_karras");
         }
@@ -1773,8 +2028,9 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     CRT_CUDA(cudaMemcpyAsync(counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
     CRT_CUDA(cudaMemsetAsync(level_count, 0, sizeof(uint32_t) * (COLLAPSE_MAX_LEVELS + 1), st));
     CRT_CUDA(cudaMemcpyAsync(level_count, c0, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    int2 root = make_int2(n > 3 ? root_index : ALL_TRIS, 0);
-    CRT_CUDA(cudaMemcpyAsync(front, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+    const int2 root = make_int2(n > 3 ? 0 : ALL_TRIS, 0);
+    if (sah_built) CRT_CUDA(cudaMemsetAsync(&front->y, 0, sizeof(int), st));
+    else CRT_CUDA(cudaMemcpyAsync(front, &root, sizeof(root), cudaMemcpyHostToDevice, st));
 
     CollapseArgs A;
     A.n = (int)n;
