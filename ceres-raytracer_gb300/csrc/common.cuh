@@ -351,7 +351,8 @@ __host__ __device__ __forceinline__ float unif24(uint32_t x) { return (float)(x 
 struct CamBasis {
     float o[3];
     float a[3], b[3], c[3];
-    double o64[3], a64[3], b64[3], c64[3];   // the same basis in FP64 (reported distances)
+    double o64[3], a64[3], b64[3], c64[3];   // the same basis in FP64 (reported hit points), scaled so that
+                                             // the central direction has length 1
     uint32_t width, height;
 };
 
@@ -381,23 +382,27 @@ __device__ __forceinline__ double plane_t64(const float4* __restrict__ tris, uin
     return num * rcp64(den);
 }
 
-// Barycentric u, v of the FP64 ray (o, d) on the FP32 triangle at leaf `slot`, with the reference's
-// formula (triangle.hpp:140-160) in FP64; false if the determinant vanishes.
-__device__ __forceinline__ bool bary64(const float4* __restrict__ tris, uint32_t slot, const double o[3],
-                                       const double d[3], double& u, double& v) {
-    const float4 a = __ldg(tris + 3ull * slot), b = __ldg(tris + 3ull * slot + 1), c4 = __ldg(tris + 3ull * slot + 2);
+// Distance t (in lengths of d, which need not be a unit vector) and, when UV is set, barycentric u, v of
+// the FP64 ray (o, d) on the FP32 triangle at leaf `slot`, with the reference's formula
+// (triangle.hpp:140-160) in FP64: one determinant and one reciprocal for all three.  Non-finite where
+// the determinant vanishes.
+template <bool UV>
+__device__ __forceinline__ void hit64(const float4* __restrict__ tris, uint32_t slot, const double o[3],
+                                      const double d[3], double& t, double& u, double& v) {
+    const float4 a = __ldg(tris + 3ull * slot), c4 = __ldg(tris + 3ull * slot + 2);
     const double p0[3] = {a.x, a.y, a.z}, n[3] = {c4.y, c4.z, c4.w};
-    // e1 = p0 - p1, e2 = p2 - p0 (triangle.hpp:31-33), exact in FP64 from the FP32 vertices
-    const double e1[3] = {p0[0] - (double)a.w, p0[1] - (double)b.x, p0[2] - (double)b.y};
-    const double e2[3] = {(double)b.z - p0[0], (double)b.w - p0[1], (double)c4.x - p0[2]};
     const double c[3] = {p0[0] - o[0], p0[1] - o[1], p0[2] - o[2]};
-    const double r[3] = {d[1] * c[2] - d[2] * c[1], d[2] * c[0] - d[0] * c[2], d[0] * c[1] - d[1] * c[0]};
-    const double det = n[0] * d[0] + n[1] * d[1] + n[2] * d[2];
-    if (det == 0.0) return false;
-    const double inv = rcp64(det);
-    u = (r[0] * e2[0] + r[1] * e2[1] + r[2] * e2[2]) * inv;
-    v = (r[0] * e1[0] + r[1] * e1[1] + r[2] * e1[2]) * inv;
-    return isfinite(u) && isfinite(v);
+    const double inv = rcp64(n[0] * d[0] + n[1] * d[1] + n[2] * d[2]);
+    t = (n[0] * c[0] + n[1] * c[1] + n[2] * c[2]) * inv;
+    if (UV) {
+        const float4 b = __ldg(tris + 3ull * slot + 1);
+        // e1 = p0 - p1, e2 = p2 - p0 (triangle.hpp:31-33), exact in FP64 from the FP32 vertices
+        const double e1[3] = {p0[0] - (double)a.w, p0[1] - (double)b.x, p0[2] - (double)b.y};
+        const double e2[3] = {(double)b.z - p0[0], (double)b.w - p0[1], (double)c4.x - p0[2]};
+        const double r[3] = {d[1] * c[2] - d[2] * c[1], d[2] * c[0] - d[0] * c[2], d[0] * c[1] - d[1] * c[0]};
+        u = (r[0] * e2[0] + r[1] * e2[1] + r[2] * e2[2]) * inv;
+        v = (r[0] * e1[0] + r[1] * e1[1] + r[2] * e1[2]) * inv;
+    }
 }
 CamBasis make_camera_basis(const crt_camera_desc* cam);
 

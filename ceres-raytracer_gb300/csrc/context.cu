@@ -149,6 +149,19 @@ CamBasis make_camera_basis(const crt_camera_desc* cam) {
         cb.c[k] = (float)cb.c64[k];
         cb.o[k] = (float)cb.o64[k];
     }
+    const double u0 = cam->resolution[0] / 2.0, v0 = cam->resolution[1] / 2.0;
+    double len = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        const double d = cb.a64[k] + u0 * cb.b64[k] + v0 * cb.c64[k];
+        len += d * d;
+    }
+    len = std::sqrt(len);
+    if (len > 0 && std::isfinite(len))
+        for (int k = 0; k < 3; ++k) {
+            cb.a64[k] /= len;
+            cb.b64[k] /= len;
+            cb.c64[k] /= len;
+        }
     cb.width = (uint32_t)std::floor(cam->resolution[0]);
     cb.height = (uint32_t)std::floor(cam->resolution[1]);
     return cb;

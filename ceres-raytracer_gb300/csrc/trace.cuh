@@ -91,6 +91,28 @@ struct trace_min_blocks<J, std::void_t<decltype(J::kMinBlocks)>> {
     static constexpr int value = J::kMinBlocks;
 };
 
+// Jobs that keep the FP64 direction of a beam from ray() to write() (kKeepsBeam) hold it in shared memory
+// while the ray is traversed: worked out again after it, it was half of a beam scan's FP64, which took 16
+// cycles per instruction and warp (1024^2 beams 197 -> 187 us).
+extern __shared__ __align__(16) unsigned char trace_smem[];
+constexpr uint32_t TRACE_BEAM = 24u * CRT_TRACE_BLOCK;   // bytes, after TRACE_SMEM
+__device__ __forceinline__ void beam_keep(const double d[3]) {
+    double* s = reinterpret_cast<double*>(trace_smem + TRACE_SMEM) + threadIdx.x;
+    for (int k = 0; k < 3; ++k) s[k * CRT_TRACE_BLOCK] = d[k];
+}
+__device__ __forceinline__ void beam_kept(double d[3]) {
+    const double* s = reinterpret_cast<const double*>(trace_smem + TRACE_SMEM) + threadIdx.x;
+    for (int k = 0; k < 3; ++k) d[k] = s[k * CRT_TRACE_BLOCK];
+}
+template <class J, class = void>
+struct trace_beam_bytes {
+    static constexpr uint32_t value = 0;
+};
+template <class J>
+struct trace_beam_bytes<J, std::void_t<decltype(J::kKeepsBeam)>> {
+    static constexpr uint32_t value = TRACE_BEAM;
+};
+
 // How a job's launches choose the items per warp (group_size): by the bound on the item count known to the
 // host, the default; by the count on the device (kGroups = GROUPS_DEVICE), for jobs whose bound is far
 // above the usual count (specular continuations of a sun-ray grid; waves of a mixed batch that hold
@@ -135,7 +157,6 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
                                                             const uint32_t* __restrict__ n_dev,
                                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ err,
                                                             unsigned long long* __restrict__ counters, uint32_t grab) {
-    extern __shared__ __align__(16) unsigned char trace_smem[];
     if (n_dev) n_items = *n_dev;   // item count produced by an earlier kernel on the stream
     const uint32_t lane = threadIdx.x & 31u;
     TravStats st{0u, 0u};
@@ -208,7 +229,7 @@ constexpr int RESET_BLOCKS = 128;
 template <bool ANY, class Job>
 void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items,
                   const uint32_t* n_dev = nullptr, uint32_t* queue = nullptr, bool full_groups = false) {
-    const size_t smem = TRACE_SMEM;
+    const size_t smem = TRACE_SMEM + trace_beam_bytes<Job>::value;
     static std::atomic<int> per_sm[2] = {{0}, {0}};   // resident blocks per SM, a property of the kernel
     int blocks = per_sm[ctx->counting].load(std::memory_order_relaxed);
     if (!blocks) {
