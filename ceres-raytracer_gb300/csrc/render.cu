@@ -206,9 +206,7 @@ __device__ __forceinline__ bool tile_px(uint32_t i, uint32_t W, uint32_t H, uint
 // of the wave's SRP request.  Batches without SRP requests use the SRP = false instantiation.
 template <bool SRP>
 struct PrimaryJobT {
-    static constexpr int kGroups = SRP ? GROUPS_DEVICE : GROUPS_HOST;   // SRP: a wave may hold one small query only
     Batch B;
-    __device__ __forceinline__ bool full_groups() const { return B.cur->n_lidar_items != 0; }
     struct Item {
         uint32_t req;
         uint32_t lidar;   // 0 camera path, 1 LiDAR beam, 2 SRP sun ray
@@ -799,14 +797,14 @@ inline uint32_t tiles_items(uint32_t W, uint32_t H) { return ((W + 7) / 8) * ((H
 // srp_items: bound on the wave's SRP items (crt_batch_mixed, serving); when non-zero the primary
 // trace also traces the wave's SRP sun rays and srp_stages (launches of the SRP shade and specular
 // segments) runs right after it.  srp_mask (when given): the SRP hit mask, zeroed before the primary
-// trace.  small_scenes: every scene of the wave has fewer than SMALL_SCENE triangles (group_size).
+// trace.  min_tris: triangles of the smallest scene of the wave, 0 unknown (launch_trace).
 // direct: B.cur already is the wave's descriptor and the counters are zero (a call of a single wave):
 // no k_wave_begin and k_wave_end (8 us).  With srp_stages reading the wave's range from the device descriptor (srp_wave_stages_dev)
 // the sequence is the same for every wave and can be captured and replayed.
 void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, uint32_t lidar_items,
                          int max_bounces, uint32_t* qa, uint32_t* qb, uint32_t srp_items = 0,
                          const std::function<void()>* srp_stages = nullptr, uint32_t* srp_mask = nullptr,
-                         size_t srp_mask_len = 0, bool small_scenes = false, bool direct = false) {
+                         size_t srp_mask_len = 0, size_t min_tris = 0, bool direct = false) {
     cudaStream_t st = ctx->stream;
     const uint32_t g_shade = grid_for(ctx, k_shade, P), g_accum = grid_for(ctx, k_accum, P);
     const uint32_t g_update = max_bounces <= 1 ? grid_for(ctx, k_update<true>, P) : grid_for(ctx, k_update<false>, P);
@@ -818,12 +816,12 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
     if (srp_items) {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<true>{B},
                             (uint32_t)std::min<size_t>(P + lidar_items + srp_items, 0xFFFFFF00u), &B.cur->n_primary,
-                            B.counts + 6, small_scenes);
+                            B.counts + 6, lidar_items ? 0 : min_tris);   // beams have FP64 work
         if (srp_stages) (*srp_stages)();
     } else {
         launch_trace<false>(ctx, SceneView{}, PrimaryJobT<false>{B},
                             (uint32_t)std::min<size_t>(P + lidar_items, 0xFFFFFF00u), &B.cur->n_primary,
-                            B.counts + 6, small_scenes || lidar_items > 0);
+                            B.counts + 6, lidar_items ? 0 : min_tris);
     }
     const uint32_t* q_in = nullptr;
     uint32_t* q_out = qa;
@@ -833,14 +831,14 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
                                          ctx->counting ? ctx->d_counters : nullptr);
         check_launch(ctx, "k_shade");
         launch_trace<true>(ctx, SceneView{}, ShadowJob{B}, (uint32_t)std::min<size_t>(P * NL, 0xFFFFFF00u),
-                           &B.counts[2 * (b % 3) + 1], B.counts + 7, small_scenes);
+                           &B.counts[2 * (b % 3) + 1], B.counts + 7, min_tris);
         if (!fuse) {
             k_accum<<<g_accum, 256, 0, st>>>(B, b, q_in);
             check_launch(ctx, "k_accum");
         }
         if (b < max_bounces - 1) {
             launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[2 * (b % 3)],
-                                B.counts + 8, small_scenes);
+                                B.counts + 8, min_tris);
             q_in = q_out;
             q_out = (q_out == qa) ? qb : qa;
         }
@@ -1208,10 +1206,11 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
     B.L = (uint32_t)NL;
 
     // ---- one wave: every launch reads the wave from B.cur (graph-capturable)
-    bool small_scenes = n_srp == 0;
-    for (size_t i = 0; i < n; ++i) small_scenes = small_scenes && reqs[i].scene->n_tris < SMALL_SCENE;
+    size_t min_tris = SIZE_MAX;
+    for (size_t i = 0; i < n; ++i) min_tris = std::min(min_tris, reqs[i].scene->n_tris);
+    for (size_t j = 0; j < n_srp; ++j) min_tris = std::min(min_tris, srps[j]->base.scene->n_tris);
     auto launch_wave = [&]() {
-        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, 0, nullptr, nullptr, 0, small_scenes, direct);
+        launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, 0, nullptr, nullptr, 0, min_tris, direct);
     };
 
     size_t waves_run = 0;
@@ -1229,7 +1228,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         if (with_srp) {
             const SrpStage* d_stage = &B.cur->srp;
             srp_stages = [&, d_stage]() {
-                srp_wave_stages_dev(ctx, d_stage, (uint32_t)srp_max, srp_nb, s_bq, s_bcount);
+                srp_wave_stages_dev(ctx, d_stage, (uint32_t)srp_max, srp_nb, s_bq, s_bcount, min_tris);
             };
             srp_mask = (uint32_t*)(s_state + srp_mask_offset(srp_max, srp_nb));
         }
@@ -1248,7 +1247,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         try {
             if (with_srp)
                 launch_wave_kernels(ctx, B, P, NL, lidar_items, max_bounces, qa, qb, (uint32_t)srp_max,
-                                    &srp_stages, srp_mask, srp_zero_bytes(srp_max));
+                                    &srp_stages, srp_mask, srp_zero_bytes(srp_max), min_tris);
             else
                 launch_wave();
         } catch (...) {
@@ -1265,7 +1264,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
                 ctx->launches += per_wave;
             } else {
                 launch_wave_kernels(ctx, B, 1, NL, 0, 0, qa, qb, plan[w].n_srp_items, &srp_stages, srp_mask,
-                                    srp_zero_bytes(srp_max));
+                                    srp_zero_bytes(srp_max), min_tris);
             }
         }
         waves_run = plan.size();
@@ -1285,7 +1284,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
             }
             const WaveDesc& wd = plan[w];
             launch_wave_kernels(ctx, B, std::max<uint32_t>(wd.n_paths, 1), NL, wd.n_lidar_items, wd.n_paths ? max_bounces : 0, qa,
-                                qb, std::max<uint32_t>(wd.n_srp_items, 1), stages ? &stages : nullptr, nullptr, 0, false, direct);
+                                qb, std::max<uint32_t>(wd.n_srp_items, 1), stages ? &stages : nullptr, nullptr, 0, min_tris, direct);
         }
         waves_run = plan.size();
     } else {
@@ -2147,7 +2146,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
                 const SrpStage* d_stage = &e->d_cur->srp;
                 stages = [&, d_stage]() {
                     srp_wave_stages_dev(ctx, d_stage, (uint32_t)e->srp_cap, (uint32_t)srp_nb, e->srp_bq,
-                                        e->srp_bcount);
+                                        e->srp_bcount, SMALL_SCENE);
                 };
                 mask = (uint32_t*)(e->srp_state + srp_mask_offset(e->srp_cap, 1));
             }

@@ -104,8 +104,7 @@ struct SrpPrimaryJob : JobBase {
 
 // continuing rays: a compacted queue of item indices (hits still land at the item's own slot)
 struct SrpBounceJob {
-    static constexpr int kGroups = GROUPS_DEVICE;   // trace_groups
-    __device__ __forceinline__ bool full_groups() const { return false; }
+    static constexpr int kOct = OCT_COUNT;   // trace_oct
     SrpWave W;
     const uint32_t* q;
     struct Item {
@@ -323,8 +322,7 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
 // continuing rays of a device stage descriptor's range
 struct SrpBounceJobDev {
     static constexpr int kMinBlocks = 7;   // trace_min_blocks
-    static constexpr int kGroups = GROUPS_DEVICE;
-    __device__ __forceinline__ bool full_groups() const { return false; }
+    static constexpr int kOct = OCT_COUNT;
     const SrpStage* S;
     const uint32_t* q;
     struct Item {
@@ -501,7 +499,7 @@ void srp_wave_stages(crt_context* ctx, const SceneView& sv, const SrpWave& W, ui
             SrpBounceJob J;
             J.W = W;
             J.q = bq;
-            launch_trace<false>(ctx, sv, J, n, bcount + (seg - 1) % 3, bcount + 4);
+            launch_trace<false>(ctx, sv, J, n, bcount + (seg - 1) % 3, bcount + 4, n_tris);
             k_srp_shade<false><<<nblk, SRP_SHADE_THREADS, 0, st>>>(sv, W, A);
         }
         check_launch(ctx, "k_srp_shade");
@@ -524,7 +522,7 @@ SrpStage srp_stage(const SceneView& sv, const SrpWave& W, uint32_t n, const SrpP
 }
 
 void srp_wave_stages_dev(crt_context* ctx, const SrpStage* d_stage, uint32_t n_max, uint32_t nb_max, uint32_t* bq,
-                         uint32_t* bcount) {
+                         uint32_t* bcount, size_t min_tris) {
     cudaStream_t st = ctx->stream;
     const uint32_t nblk = std::max<uint32_t>(1, (n_max + SRP_BLOCK_ITEMS - 1) / SRP_BLOCK_ITEMS);
     for (uint32_t seg = 0; seg <= nb_max; ++seg) {
@@ -535,7 +533,7 @@ void srp_wave_stages_dev(crt_context* ctx, const SrpStage* d_stage, uint32_t n_m
             SrpBounceJobDev J;
             J.S = d_stage;
             J.q = bq;
-            launch_trace<false>(ctx, SceneView{}, J, n_max, bcount + (seg - 1) % 3, bcount + 4);
+            launch_trace<false>(ctx, SceneView{}, J, n_max, bcount + (seg - 1) % 3, bcount + 4, min_tris);
             k_srp_shade_dev<false><<<nblk, SRP_SHADE_THREADS, 0, st>>>(d_stage, seg, bq, q_count, bcount);
         }
         check_launch(ctx, "k_srp_shade");
@@ -584,7 +582,7 @@ void srp_run(crt_context* ctx, crt_scene* s, const crt_srp_desc* desc, const dou
             SrpPrimaryJob J;
             J.W = W;
             CRT_CUDA(cudaMemsetAsync(bcount, 0, srp_zero_bytes(n), st));   // counters and hit mask
-            launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5);
+            launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5, s->n_tris);
             srp_wave_stages(ctx, sv, W, n, P, d_partial, d_facet, (uint32_t)s->n_tris, bq, bcount);
         }
         srp_reduce(ctx, d_partial, P, d_force, d_torque);
@@ -711,7 +709,7 @@ extern "C" int crt_srp_static(crt_scene* s, const crt_srp_desc* desc, const doub
                 SrpPrimaryJob J;
                 J.W = W;
                 CRT_CUDA(cudaMemsetAsync(bcount, 0, srp_zero_bytes(n), st));   // counters and hit mask
-                launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5);
+                launch_trace<false>(ctx, sv, J, n, nullptr, bcount + 5, s->n_tris);
                 // block sums of this wave only: slot = (block of the attitude group) - (wave's first block)
                 const uint64_t block0 = i0 / SRP_BLOCK_ITEMS;
                 srp_wave_stages(ctx, sv, W, n, G, d_partial, nullptr, (uint32_t)s->n_tris, bq, bcount, block0);

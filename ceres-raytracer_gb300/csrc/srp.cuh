@@ -174,7 +174,8 @@ SrpStage srp_stage(const SceneView& sv, const SrpWave& W, uint32_t n, const SrpP
 // srp_wave_stages for the range in d_stage (device memory, filled before the launches run): launches
 // nb_max specular segments over n_max items; segments and blocks beyond the range's own do nothing.
 // No argument depends on the range, so the launches can be captured once and replayed per wave.
+// min_tris: triangles of the smallest scene of the ranges (launch_trace).
 void srp_wave_stages_dev(crt_context* ctx, const SrpStage* d_stage, uint32_t n_max, uint32_t nb_max, uint32_t* bq,
-                         uint32_t* bcount);
+                         uint32_t* bcount, size_t min_tris);
 // Per-attitude force and torque from the request's partial sums (device outputs)
 void srp_reduce(crt_context* ctx, const double* partial, const SrpPlan& P, double* force, double* torque);

@@ -15,6 +15,7 @@ namespace {
 
 // ---------------------------------------------------------------- jobs
 struct RayClosestJob : JobBase {
+    static constexpr int kOct = OCT_SMALL;   // trace_oct
     const float4* rays;   // crt_ray as 2 x float4
     crt_hit* hits;
     __device__ bool ray(uint32_t i, TRay& r, Item&) const {
@@ -66,7 +67,7 @@ __device__ __forceinline__ bool tile_pixel(uint32_t i, uint32_t W, uint32_t H, u
 // the point and the barycentrics share one determinant and reciprocal and the ray is not normalised:
 // 1021 x 767 pixels of a smooth-shaded body 175 -> 146 us in the kernel.
 struct PassJob : JobBase {
-    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
+    static constexpr int kOct = OCT_NEVER;   // trace_oct
     CamBasis cam;
     double* xyz;
     uint32_t* ids;
@@ -130,7 +131,7 @@ struct PassJob : JobBase {
 };
 
 struct LidarBatchJob : JobBase {
-    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
+    static constexpr int kOct = OCT_NEVER;   // trace_oct
     const double* pos;
     const double* rot;
     float zsign;
@@ -161,7 +162,7 @@ struct LidarBatchJob : JobBase {
 };
 
 struct LidarGridJob : JobBase {
-    static constexpr int kGroups = GROUPS_FULL;   // trace_groups
+    static constexpr int kOct = OCT_NEVER;   // trace_oct
     static constexpr bool kKeepsBeam = true;
     double o[3];
     double rt[9];         // R^T row-major (world = rt * sensor direction)

@@ -113,77 +113,75 @@ struct trace_beam_bytes<J, std::void_t<decltype(J::kKeepsBeam)>> {
     static constexpr uint32_t value = TRACE_BEAM;
 };
 
-// How a job's launches choose the items per warp (group_size): by the bound on the item count known to the
-// host, the default; by the count on the device (kGroups = GROUPS_DEVICE), for jobs whose bound is far
-// above the usual count (specular continuations of a sun-ray grid; waves of a mixed batch that hold
-// nothing but one small query; the job's full_groups() says where it has FP64 items); or always 32 (GROUPS_FULL), for jobs with FP64 work per item, which
-// takes the same time for a warp with one active lane (a 229 x 128 beam scan: 34 us, in small groups 53).
-// A group size from the device is a register of every thread, which cost 1.7 % of a 2048^2 render's
-// traces, so it is not the default.
-enum { GROUPS_HOST, GROUPS_DEVICE, GROUPS_FULL };
+// Which kernel a launch takes.  k_trace, a lane per ray, has the higher throughput; but a small launch lasts
+// as long as its longest chain of node visits, and there k_trace_oct, eight lanes per ray, is faster.  Of
+// a scene's asteroid-like bodies (4 k .. 500 k triangles), 30 k rays or camera paths: 1.03 - 1.48 times;
+// 60 k random closest-hit rays 0.84 - 0.89, any-hit rays and camera paths 1.04 - 1.20 from 32 k triangles
+// on, 0.88 - 1.0 below; 100 k and more 0.5 - 1.1.  Jobs with FP64 work per ray stay with k_trace (OCT_NEVER):
+// a warp's FP64 instruction takes the same 16 cycles for four rays as for 32.  So do scenes of fewer than
+// SMALL_SCENE triangles, whose rays are done in a few nodes.
+constexpr uint32_t OCT_ITEMS = 40000, OCT_ITEMS_DEEP = 80000, OCT_DEEP_TRIS = 32768, SMALL_SCENE = 1024;
+// A job's kOct: OCT_NEVER, OCT_SMALL (up to OCT_ITEMS), OCT_DEEP (the default: up to OCT_ITEMS_DEEP in scenes of
+// OCT_DEEP_TRIS triangles), or OCT_COUNT: the host knows only a bound far above the usual count, so both
+// kernels are launched and the one that the count on the device does not call for returns at once.
+enum { OCT_NEVER, OCT_SMALL, OCT_DEEP, OCT_COUNT };
 template <class J, class = void>
-struct trace_groups {
-    static constexpr int value = GROUPS_HOST;
+struct trace_oct {
+    static constexpr int value = OCT_DEEP;
 };
 template <class J>
-struct trace_groups<J, std::void_t<decltype(J::kGroups)>> {
-    static constexpr int value = J::kGroups;
+struct trace_oct<J, std::void_t<decltype(J::kOct)>> {
+    static constexpr int value = J::kOct;
 };
 
-// Items a warp takes at a time in a launch of n items on `warps` warps: 32, one per lane, unless that
-// would leave more than half of the warps without work; then fewer, the other lanes idle.  A small
-// launch lasts as long as its slowest warp, and a warp of 32 rays is slower than its slowest ray by
-// every node and triangle that only other lanes visit.  256 rays on 20 k triangles 37 -> 21.5 us,
-// a 128^2 render 167 -> 142 us, one 250^2 sun-ray grid with two bounces 181 -> 137 us.  (Groups that also
-// shrink at the end of a large launch cost it 1 - 3 %: its last rays then take more issue slots.)
-// Scenes of fewer than SMALL_SCENE triangles always get 32: their rays are done in a few nodes, and the
-// work per ray outside the traversal, repeated per warp, is what they wait for (27 k camera paths in a
-// box of 36 triangles: 64 us, in groups of 8 67 us).
-constexpr size_t SMALL_SCENE = 1024;
-__host__ __device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t warps) {
-    const uint32_t per = n / warps;
-    return per >= 16u ? 32u : per >= 8u ? 16u : per >= 4u ? 8u : per >= 2u ? 4u : per >= 1u ? 2u : 1u;
-}
-
-// Persistent ray-queue kernel.  Each warp takes one group of consecutive items per atomic grab, or,
-// with chunk > 1 and full groups, a guided number of up to `chunk` groups, shrinking with the work left
-// so that the last grabs stay small (few atomics on the queue counter while much work is left, balance
-// at the end).  queue: the next item, zero at the start.  grab: group size (0: from the count, GROUPS_DEVICE) | chunk << 8
+// Persistent ray-queue kernel.  Each warp takes 32 consecutive items per atomic grab, or, with chunk > 1, a
+// guided number of up to `chunk` times 32, shrinking with the work left so that the last grabs stay
+// small (few atomics on the queue counter while much work is left, balance at the end).  queue: the next
+// item, zero at the start.  A count of at most `over` items is left to the other kernel.  grab: chunk
 // | GRAB_RESET: leave the queue at zero (queue[1] counts the blocks that have finished).
 constexpr uint32_t GRAB_RESET = 1u << 31;
+
+__device__ __forceinline__ void queue_reset(uint32_t* queue, uint32_t grab) {
+    if (grab & GRAB_RESET) {   // the last block to finish leaves both counters zero for the next launch
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(queue + 1, 1u) == gridDim.x - 1u) queue[0] = queue[1] = 0u;
+        }
+    }
+}
 
 template <bool ANY, bool COUNT, class Job>
 __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value) k_trace(SceneView sv, Job job, uint32_t n_items,
                                                             const uint32_t* __restrict__ n_dev,
                                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ err,
-                                                            unsigned long long* __restrict__ counters, uint32_t grab) {
+                                                            unsigned long long* __restrict__ counters, uint32_t grab,
+                                                            uint32_t over) {
     if (n_dev) n_items = *n_dev;   // item count produced by an earlier kernel on the stream
-    const uint32_t lane = threadIdx.x & 31u;
+    if (n_items <= over) return;
+    const int lane = threadIdx.x & 31;
     TravStats st{0u, 0u};
     uint32_t nrays = 0, nres = 0;
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
-    const uint32_t chunk = (grab >> 8) & 0xFFu;
-    uint32_t group = grab & 0xFFu;
-    if constexpr (trace_groups<Job>::value == GROUPS_DEVICE)
-        if (!group) group = job.full_groups() ? 32u : group_size(n_items, warps_total);
+    const uint32_t chunk = grab & 0xFFu;
     while (true) {
-        uint32_t base = 0, take = group;
+        uint32_t base = 0, take = 1;
         if (lane == 0) {
-            if (chunk > 1 && group == 32u) {
+            if (chunk > 1) {
                 const uint32_t cur = *reinterpret_cast<volatile uint32_t*>(queue);
                 const uint32_t left = cur < n_items ? (n_items - cur) >> 5 : 0u;
-                take = 32u * min(chunk, max(1u, left / (4u * warps_total)));
+                take = min(chunk, max(1u, left / (4u * warps_total)));
             }
-            base = atomicAdd(queue, take);
+            base = atomicAdd(queue, 32u * take);
         }
         base = __shfl_sync(0xffffffffu, base, 0);
         take = __shfl_sync(0xffffffffu, take, 0);
         if (base >= n_items) break;
-        for (const uint32_t end = base + ((take + 31u) & ~31u); base != end; base += 32u) {
+        for (const uint32_t end = base + 32u * take; base != end; base += 32u) {
             const uint32_t i = base + lane;
             TRay r;
             typename Job::Item it;
-            const int kind = lane < group && i < n_items ? (int)job.ray(i, r, it) : 0;
+            const int kind = i < n_items ? (int)job.ray(i, r, it) : 0;
             if (kind == 1) {
                 const THit h = traverse<ANY, COUNT>(job.view(sv, it), r, trace_smem, st, err);
                 job.write(sv, i, r, h, it);
@@ -209,63 +207,122 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
             if (d) atomicAdd(counters + 3, d);
         }
     }
-    if (grab & GRAB_RESET) {   // the last block to finish leaves both counters zero for the next launch
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            if (atomicAdd(queue + 1, 1u) == gridDim.x - 1u) queue[0] = queue[1] = 0u;
-        }
-    }
+    queue_reset(queue, grab);
 }
 
-// Launches the persistent trace kernel over n_items work items (or over *n_dev items when n_dev is
-// given: n_items is then the upper bound used to size the grid).  full_groups: 32 items per warp whatever
-// the count (launches with FP64 items among others).
+// The ray queue with eight lanes per ray (traverse_oct): 1, 2 or 4 rays per warp and grab, the most that
+// leave no warp without work.  A job's ray() runs on all of a ray's lanes (what it stores is the same
+// from each), its write() on one.  A count above `upto` is left to k_trace.  6 blocks per SM (80
+// registers): at 8 the kernels spill (a 128^2 render 92 -> 103 us).
+template <bool ANY, bool COUNT, class Job>
+__global__ void __launch_bounds__(CRT_TRACE_BLOCK, 6) k_trace_oct(SceneView sv, Job job, uint32_t n_items,
+                                                                  const uint32_t* __restrict__ n_dev,
+                                                                  uint32_t* __restrict__ queue,
+                                                                  uint32_t* __restrict__ err,
+                                                                  unsigned long long* __restrict__ counters,
+                                                                  uint32_t grab, uint32_t upto) {
+    if (n_dev) n_items = *n_dev;
+    if (n_items > upto) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warps = gridDim.x * (CRT_TRACE_BLOCK / 32), per = n_items / warps;
+    const uint32_t take = per >= 4u ? 4u : per >= 2u ? 2u : 1u;
+    TravStats st{0u, 0u};
+    uint32_t nrays = 0, nres = 0;
+    while (true) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(queue, take);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= n_items) break;
+        const uint32_t i = base + (lane >> 3);
+        TRay r;
+        r.o = r.d = f3(0.f, 0.f, 1.f);
+        r.tmin = r.tmax = 0.f;
+        typename Job::Item it;
+        const int kind = (lane >> 3) < take && i < n_items ? (int)job.ray(i, r, it) : 0;
+        SceneView v{};
+        if (kind == 1) v = job.view(sv, it);
+        const THit h = traverse_oct<ANY, COUNT>(v, r, kind == 1, trace_smem, st, err);
+        if (kind == 1 && (lane & 7u) == 0) job.write(sv, i, r, h, it);
+        if (COUNT && (lane & 7u) == 0) {
+            nrays += kind == 1;
+            nres += kind == 2;
+        }
+    }
+    if (COUNT) {
+        atomicAdd(counters + 0, (unsigned long long)nrays);
+        atomicAdd(counters + 1, (unsigned long long)st.nodes);
+        atomicAdd(counters + 2, (unsigned long long)st.tris);
+        atomicAdd(counters + 3, (unsigned long long)nres);
+    }
+    queue_reset(queue, grab);
+}
+
+// Resident blocks per SM of a kernel (a property of the kernel and its shared memory), asked for once.
+template <class Kernel>
+int resident_blocks(crt_context* ctx, Kernel* kernel, size_t smem, std::atomic<int>& known) {
+    int blocks = known.load(std::memory_order_relaxed);
+    if (!blocks) {
+        blocks = occupancy_grid(ctx, (const void*)kernel, CRT_TRACE_BLOCK, smem) / ctx->sm_count;
+        known.store(blocks, std::memory_order_relaxed);
+    }
+    return blocks;
+}
+
+// Launches a trace over n_items work items (or over *n_dev items when n_dev is given: n_items is then an
+// upper bound).  tris: triangles of the smallest scene the rays meet, 0: keep to k_trace.
 // queue: a work counter that an earlier operation on the stream has zeroed; null: the context's own.
 // There a small launch finds its counter at zero and leaves it so; past RESET_BLOCKS blocks the atomics of
 // the finishing blocks take longer (2.4 us with 1216) than a memset before the launch, which overlaps
 // the end of the work before it (256 rays: 23.0 us with the memset, 22.0 without).
 constexpr int RESET_BLOCKS = 128;
 template <bool ANY, class Job>
-void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items,
-                  const uint32_t* n_dev = nullptr, uint32_t* queue = nullptr, bool full_groups = false) {
-    const size_t smem = TRACE_SMEM + trace_beam_bytes<Job>::value;
-    static std::atomic<int> per_sm[2] = {{0}, {0}};   // resident blocks per SM, a property of the kernel
-    int blocks = per_sm[ctx->counting].load(std::memory_order_relaxed);
-    if (!blocks) {
-        const void* kfn = ctx->counting ? (const void*)k_trace<ANY, true, Job> : (const void*)k_trace<ANY, false, Job>;
-        blocks = occupancy_grid(ctx, kfn, CRT_TRACE_BLOCK, smem) / ctx->sm_count;
-        per_sm[ctx->counting].store(blocks, std::memory_order_relaxed);
-    }
-    int grid = blocks * ctx->sm_count;
-    constexpr int groups = trace_groups<Job>::value;
-    full_groups = full_groups || groups == GROUPS_FULL || (sv.nodes && sv.n_tris < SMALL_SCENE);
-    // at most one warp per group (per item where groups may be smaller than 32)
-    const uint32_t per_block = full_groups ? CRT_TRACE_BLOCK : CRT_TRACE_BLOCK / 32;
-    const uint32_t need = std::max<uint32_t>((n_items + per_block - 1) / per_block, 1u);
-    if ((uint32_t)grid > need) grid = (int)need;
-    const uint32_t group = full_groups ? 32u : groups == GROUPS_DEVICE ? 0u : group_size(n_items, (uint32_t)grid * (CRT_TRACE_BLOCK / 32));
-    uint32_t grab = group | (ctx->queue_chunk ? ctx->queue_chunk : 1u) << 8;
-    if (!queue) {
-        queue = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
+void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items, const uint32_t* n_dev,
+                  uint32_t* queue, size_t tris) {
+    constexpr int oct = trace_oct<Job>::value;
+    const uint32_t chunk = ctx->queue_chunk ? ctx->queue_chunk : 1u;
+    const bool counting = ctx->counting;
+    auto own_queue = [&](uint32_t* q, int grid, uint32_t& grab) {
+        if (q) return q;
+        q = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
         if (grid <= RESET_BLOCKS) {
             grab |= GRAB_RESET;
-        } else {
-            queue += 8;   // words 0 and 1 stay zero for the small launches
-            CRT_CUDA(cudaMemsetAsync(queue, 0, sizeof(uint32_t), ctx->stream));
+            return q;
+        }
+        q += 8;   // words 0 and 1 stay zero for the small launches
+        CRT_CUDA(cudaMemsetAsync(q, 0, sizeof(uint32_t), ctx->stream));
+        return q;
+    };
+    uint32_t over = 0;
+    if constexpr (oct != OCT_NEVER) {
+        const uint32_t limit = tris < SMALL_SCENE ? 0u : oct != OCT_SMALL && tris >= OCT_DEEP_TRIS ? OCT_ITEMS_DEEP : OCT_ITEMS;
+        const bool fits = n_items <= limit, both = oct == OCT_COUNT && limit && !fits;
+        if (fits || both) {
+            static std::atomic<int> known[2] = {{0}, {0}};
+            auto kernel = counting ? k_trace_oct<ANY, true, Job> : k_trace_oct<ANY, false, Job>;
+            const uint32_t want = std::max<uint32_t>((std::min(n_items, limit) + CRT_TRACE_BLOCK / 32 - 1) / (CRT_TRACE_BLOCK / 32), 1u);
+            const int grid = (int)std::min<uint32_t>((uint32_t)(resident_blocks(ctx, kernel, OCT_SMEM, known[counting]) * ctx->sm_count), want);
+            uint32_t grab = 0;
+            uint32_t* q = own_queue(queue, grid, grab);
+            kernel<<<grid, CRT_TRACE_BLOCK, OCT_SMEM, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters,
+                                                                   grab, both ? limit : 0xFFFFFFFFu);
+            check_launch(ctx, "k_trace_oct");
+            if (fits) return;
+            over = limit;
         }
     }
-    if (ctx->counting)
-        k_trace<ANY, true, Job><<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, queue,
-                                                                             ctx->d_error, ctx->d_counters, grab);
-    else
-        k_trace<ANY, false, Job><<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, queue,
-                                                                              ctx->d_error, ctx->d_counters, grab);
+    static std::atomic<int> known[2] = {{0}, {0}};
+    auto kernel = counting ? k_trace<ANY, true, Job> : k_trace<ANY, false, Job>;
+    constexpr size_t smem = TRACE_SMEM + trace_beam_bytes<Job>::value;
+    int grid = resident_blocks(ctx, kernel, smem, known[counting]) * ctx->sm_count;
+    const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
+    if ((uint32_t)grid > need) grid = (int)std::max<uint32_t>(need, 1u);
+    uint32_t grab = chunk;
+    uint32_t* q = own_queue(queue, grid, grab);
+    kernel<<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters, grab, over);
     check_launch(ctx, "k_trace");
 }
 
 template <bool ANY, class Job>
-void launch_trace(crt_scene* s, const Job& job, uint32_t n_items, const uint32_t* n_dev = nullptr,
-                  uint32_t* queue = nullptr) {
-    launch_trace<ANY>(s->ctx, scene_view(s), job, n_items, n_dev, queue);
+void launch_trace(crt_scene* s, const Job& job, uint32_t n_items) {
+    launch_trace<ANY>(s->ctx, scene_view(s), job, n_items, nullptr, nullptr, s->n_tris);
 }

@@ -256,3 +256,158 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
     hit.v = h.y * inv;
     return hit;
 }
+
+// ---------------------------------------------------------------- eight lanes per ray
+// The same traversal for launches of few rays, which last as long as their longest chain of dependent
+// node visits: lane c of a ray's eight lanes tests child c, and up to eight triangles are tested at once.
+// The four rays of a warp step together.  Visits, hits and their order are those of traverse: of the
+// triangles of one step the nearest wins, of equal ones the last, as when they are tested in turn.
+// What bounds it is the length of one step: the loads of a node (a word per plane and lane), a child's slab
+// test, the choice of the next child, the loads and test of its triangles.  Against a lane per ray, in
+// groups small enough to fill the GPU: 256 rays on 20 k triangles 22.4 -> 16.8 us, a 128^2 render 125 ->
+// 93 us, a 250^2 sun-ray grid with two bounces 130 -> 113 us.
+constexpr uint32_t OCT_RAYS = CRT_TRACE_BLOCK / 8;                        // rays of a block
+constexpr uint32_t OCT_SMEM = 8u * CRT_STACK_TOTAL * OCT_RAYS;   // their stacks, indexed by ray last
+
+// Called by the whole warp; `active`, the ray and the scene are the same for a ray's eight lanes.
+template <bool ANY, bool COUNT>
+__device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool active, unsigned char* smem,
+                                             TravStats& st, uint32_t* __restrict__ err) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, oct0 = lane & 24u;
+    THit hit;
+    hit.slot = CRT_MISS;
+    hit.t = hit.u = hit.v = 0.f;
+    float det = 1.0f;
+    uint2* const stack = reinterpret_cast<uint2*>(smem) + (threadIdx.x >> 3);
+    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
+                         ((__float_as_uint(ray.d.z) >> 31) << 2);
+    const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
+    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
+    // row of the near planes per axis, and the lane's word in it
+    const uint32_t word = (sub >> 1) * 4u;
+    const uint32_t rowx = ((oct & 1u) ? 0x50u : 0x20u) + word, rowy = ((oct & 2u) ? 0x60u : 0x30u) + word,
+                   rowz = ((oct & 4u) ? 0x70u : 0x40u) + word;
+    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
+                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
+    TShear shear = make_shear(ray.d);
+    shear.ox = shear_proj(ray.o, shear.bx);
+    shear.oy = shear_proj(ray.o, shear.by);
+    int sp = 0;
+    uint32_t node = 0;   // the root
+    while (__any_sync(ALL, active)) {
+        __syncwarp();   // stack entries written in the last step are visible
+        // ---- visit: the lane's child
+        bool in = false;
+        uint32_t vm = 0, tbase = 0, cbase = 0;
+        if (active) {
+            const uintptr_t np = reinterpret_cast<uintptr_t>(sv.nodes + node) ^ ((node & 7u) << 4);
+            auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
+            auto plane = [&](uint32_t off) {
+                const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(np ^ off));
+                return (sub & 1u) ? __half2float(__habs(__ushort_as_half((unsigned short)(w & 0xFFFFu)))) : __uint_as_float(w);
+            };
+            const float4 w0 = row(0x00u), w1 = row(0x10u);
+            const float xn = plane(rowx), xf = plane(rowx ^ 0x70u), yn = plane(rowy), yf = plane(rowy ^ 0x50u),
+                        zn = plane(rowz), zf = plane(rowz ^ 0x30u);
+            if (COUNT) st.nodes += sub == 0;
+            const uint32_t ew = __float_as_uint(w0.w);
+            const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
+            const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
+            const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
+            const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
+            const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
+            const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
+            const float gap = fminf(fminf(fmaf(xf, sx, ax), fmaf(yf, sy, ay)), fminf(fmaf(zf, sz, az), ray.tmax)) -
+                              fmaxf(fmaxf(fmaf(xn, sx, ax), fmaf(yn, sy, ay)), fmaxf(fmaf(zn, sz, az), ray.tmin));
+            in = !(__float_as_uint(gap) >> 31);
+            cbase = __float_as_uint(w1.x);
+            tbase = __float_as_uint(w1.y);
+            vm = __float_as_uint(w1.z);
+        }
+        const uint32_t hits = (__ballot_sync(ALL, in) >> oct0) & 0xFFu;
+        uint32_t leaf3 = hits;
+        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
+        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
+        leaf3 = (leaf3 * 0x5u) & 0x249249u;
+        const uint32_t tvalid = vm & 0x00FFFFFFu;
+        uint32_t tmask = (leaf3 * 7u) & tvalid;
+        // ---- next internal node (a nearer hit does not change which)
+        uint2 group = make_uint2(cbase, ((hits << 24) & vm) | (vm >> 24));
+        bool more = active;
+        if (active && group.y <= 0x00FFFFFFu) {
+            more = sp != 0;
+            if (more) group = stack[--sp * OCT_RAYS];
+        }
+        __syncwarp();   // the entry has been read by the ray's lanes before it may be overwritten
+        if (more) {
+            uint32_t cb = group.y & 0xFF000000u;
+            uint32_t pr = cb & pick2;
+            cb = pr ? pr : cb;
+            pr = cb & pick1;
+            cb = pr ? pr : cb;
+            pr = cb & pick0;
+            cb = pr ? pr : cb;
+            node = group.x + __popc(group.y & ((cb >> 24) - 1u));
+            group.y ^= cb;
+            if (group.y > 0x00FFFFFFu) {
+                if (sp < CRT_STACK_TOTAL) {
+                    if (sub == 0) stack[sp * OCT_RAYS] = group;
+                    ++sp;
+                } else {
+                    if (sub == 0) atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
+                    more = false;
+                }
+            }
+        }
+        // ---- leaf triangles of the visited node, eight at a time: lane k takes the k-th
+        while (__any_sync(ALL, tmask != 0u)) {
+            uint32_t m = tmask;
+            for (uint32_t k = 0; k < sub; ++k) m &= m - 1u;   // (0 stays 0)
+            const uint32_t low = m & (0u - m);
+            bool ok = false;
+            float t = 0.f, wv = 0.f, ww = 0.f, dt = 1.f;
+            uint32_t slot = 0;
+            if (m) {
+                slot = tbase + __popc(tvalid & (low - 1u));
+                if (slot != ray.skip) {
+                    const float4* tp = sv.tris + 3ull * slot;
+                    const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+                    if (COUNT) st.tris++;
+                    ok = tri_test(a, b, c, ray, shear, t, wv, ww, dt);
+                }
+            }
+            const uint32_t any = (__ballot_sync(ALL, ok) >> oct0) & 0xFFu;
+            if (ANY) {
+                if (any) {
+                    hit.slot = 0;
+                    more = false;
+                    tmask = 0;
+                }
+            } else if (__any_sync(ALL, ok)) {
+                float best = ok ? t : 3.402823466e38f;
+                for (int o = 1; o < 8; o <<= 1) best = fminf(best, __shfl_xor_sync(ALL, best, o));
+                const uint32_t win = (__ballot_sync(ALL, ok && t == best) >> oct0) & 0xFFu;
+                const int from = (int)oct0 + (win ? 31 - __clz(win) : 0);
+                const float u = __shfl_sync(ALL, wv, from), v = __shfl_sync(ALL, ww, from);
+                const float d = __shfl_sync(ALL, dt, from);
+                const uint32_t sl = __shfl_sync(ALL, slot, from);
+                if (win) {
+                    ray.tmax = best;
+                    hit.u = u;
+                    hit.v = v;
+                    det = d;
+                    hit.slot = sl;
+                }
+            }
+            for (int k = 0; k < 8; ++k) tmask &= tmask - 1u;
+        }
+        active = more;
+    }
+    if (ANY) return hit;
+    const float inv = 1.0f / det;
+    hit.t = hit.slot != CRT_MISS ? ray.tmax : 0.0f;
+    hit.u *= inv;
+    hit.v *= inv;
+    return hit;
+}
