@@ -69,6 +69,7 @@ struct RenderCtl {
     float noise_threshold;
     int num_bounces;
     uint32_t seed_lo, seed_hi, request;
+    FastDiv by4W, byW;
 };
 
 struct RReq {            // render request
@@ -88,6 +89,7 @@ struct LReq {            // LiDAR beam-grid request
     double rt[9];        // R^T row-major
     double zsign;
     uint32_t nx, ny;
+    FastDiv tiles;       // tiles of 8 beams per row
     uint32_t tan_base;   // nx + ny tangents in the batch table
     uint32_t item_base;  // first primary item (8 x 4 tile order)
     double* range;
@@ -96,6 +98,7 @@ struct LReq {            // LiDAR beam-grid request
 
 struct Slice {
     uint32_t req, s0, ns, npix;
+    FastDiv by_npix;
     uint32_t path_base, upd_base;
     const uint32_t* active;   // pixel set of the slice (nullptr: every pixel of the request)
 };
@@ -182,23 +185,22 @@ __device__ __forceinline__ uint32_t find_slice_by_path(const WaveDesc& w, uint32
 // camera rays cover one tile (which shares more BVH nodes than 32 pixels of one row: about 12 %
 // faster primary and shadow traversal).  A bijection of [0, W*H) for any W, H: rows are grouped in
 // bands of 4 (the last band may be lower) and a band's last tile is W mod 8 wide.
-__device__ __forceinline__ uint32_t tile_slot_pixel(uint32_t j, uint32_t W, uint32_t H) {
-    const uint32_t y0 = j / (4u * W) * 4u;
-    const uint32_t hb = min(4u, H - y0);
-    const uint32_t r = j - y0 * W;
-    const uint32_t full = W >> 3;
-    const uint32_t tx = min(r / (8u * hb), full);
+__device__ __forceinline__ void tile_slot_pixel(uint32_t j, const RenderCtl& c, uint32_t& px, uint32_t& py) {
+    const uint32_t band = div_by(j, c.by4W), y0 = band * 4u;
+    const uint32_t hb = min(4u, c.H - y0);
+    const uint32_t r = j - band * c.by4W.d;
+    const uint32_t full = c.W >> 3;
+    // a band of full height: tiles of 32 (r / 32), else general
+    const uint32_t tx = min(hb == 4u ? r >> 5 : r / (8u * hb), full);
     const uint32_t rr = r - tx * 8u * hb;
-    const uint32_t wt = tx < full ? 8u : W - 8u * full;   // r < hb * W keeps wt > 0 here
-    return (y0 + rr / wt) * W + tx * 8u + rr % wt;
-}
-
-__device__ __forceinline__ bool tile_px(uint32_t i, uint32_t W, uint32_t H, uint32_t& px, uint32_t& py) {
-    const uint32_t tiles_x = (W + 7) >> 3;
-    const uint32_t tile = i >> 5, w = i & 31u;
-    px = (tile % tiles_x) * 8u + (w & 7u);
-    py = (tile / tiles_x) * 4u + (w >> 3);
-    return px < W && py < H;
+    if (tx < full) {
+        px = tx * 8u + (rr & 7u);
+        py = y0 + (rr >> 3);
+    } else {   // r < hb W keeps the last tile's width > 0 here
+        const uint32_t wt = c.W - 8u * full, y = rr / wt;
+        px = tx * 8u + rr - y * wt;
+        py = y0 + y;
+    }
 }
 
 // ---------------------------------------------------------------- primary stage
@@ -231,7 +233,7 @@ struct PrimaryJobT {
             }
             const LReq& L = B.lr[lo];
             uint32_t px, py;
-            if (!tile_px(i - L.item_base, L.nx, L.ny, px, py)) return false;
+            if (!tile_px(i - L.item_base, L.tiles, L.nx, L.ny, px, py)) return false;
             double d[3];
             beam64(L, px, py, d);
             r.o = f3((float)L.o[0], (float)L.o[1], (float)L.o[2]);
@@ -251,11 +253,19 @@ struct PrimaryJobT {
         const uint32_t p = i - w.n_lidar_items;
         const Slice& S = w.slices[find_slice_by_path(w, p)];
         const uint32_t q = p - S.path_base;
-        const uint32_t a = q % S.npix;
-        const uint32_t sample = S.s0 + q / S.npix;
+        const uint32_t k = div_by(q, S.by_npix), a = q - k * S.npix;
+        const uint32_t sample = S.s0 + k;
         const RReq& R = B.rr[S.req];
-        const uint32_t pixel = S.active ? S.active[a] : tile_slot_pixel(a, R.c.W, R.c.H);
-        float u = (float)(pixel % R.c.W), v = (float)(pixel / R.c.W);
+        uint32_t px, py;
+        if (S.active) {
+            const uint32_t pix = S.active[a];
+            py = div_by(pix, R.c.byW);
+            px = pix - py * R.c.W;
+        } else {
+            tile_slot_pixel(a, R.c, px, py);
+        }
+        const uint32_t pixel = py * R.c.W + px;
+        float u = (float)px, v = (float)py;
         if (R.c.max_samples != 1) {   // do_render.hpp:76-82: pixel corner for a single sample
             float ja, jb;
             rng2(R.c, pixel, sample, 0, 0, ja, jb);
@@ -278,7 +288,7 @@ struct PrimaryJobT {
         if (it.lidar) {
             const LReq& L = B.lr[it.req];
             uint32_t px, py;
-            tile_px(i - L.item_base, L.nx, L.ny, px, py);
+            tile_px(i - L.item_base, L.tiles, L.nx, L.ny, px, py);
             const size_t k = (size_t)py * L.nx + px;
             double rng = 0.0;
             if (h.slot != CRT_MISS) {
@@ -680,7 +690,14 @@ __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
         const Slice& S = w.slices[lo];
         const uint32_t a = u - S.upd_base;
         const RReq& R = B.rr[S.req];
-        const uint32_t pixel = S.active ? S.active[a] : tile_slot_pixel(a, R.c.W, R.c.H);
+        uint32_t pixel;
+        if (S.active) {
+            pixel = S.active[a];
+        } else {
+            uint32_t px, py;
+            tile_slot_pixel(a, R.c, px, py);
+            pixel = py * R.c.W + px;
+        }
         const size_t g = (size_t)R.pix_base + pixel;
         // a slice that starts at sample 0 holds the pixel's first samples: its state (running mean, count
         // and done flag) is not set yet and not read
@@ -729,10 +746,16 @@ __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
 // still-active pixels of an adaptive request, in the order of its previous pixel set (tile order
 // at first), so that the camera rays of a warp stay close together
 __global__ void k_compact(const uint32_t* __restrict__ active, uint32_t n_active, const uint8_t* __restrict__ done,
-                          uint32_t pix_base, uint32_t W, uint32_t H, uint32_t* __restrict__ out,
-                          uint32_t* __restrict__ count) {
+                          uint32_t pix_base, RenderCtl c, uint32_t* __restrict__ out, uint32_t* __restrict__ count) {
     for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n_active; a += gridDim.x * blockDim.x) {
-        const uint32_t pixel = active ? active[a] : tile_slot_pixel(a, W, H);
+        uint32_t pixel;
+        if (active) {
+            pixel = active[a];
+        } else {
+            uint32_t px, py;
+            tile_slot_pixel(a, c, px, py);
+            pixel = py * c.W + px;
+        }
         if (!done[pix_base + pixel]) out[warp_append(count, 1u)] = pixel;
     }
 }
@@ -926,7 +949,8 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
             R.cam = make_camera_basis(q.camera);
             const crt_render_params& p = *q.params;
             R.c = RenderCtl{R.cam.width, R.cam.height, p.min_samples, p.max_samples, (float)p.noise_threshold,
-                            p.num_bounces, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), p.request};
+                            p.num_bounces, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), p.request,
+                            fast_div(4u * R.cam.width), fast_div(R.cam.width)};
             R.light_base = (uint32_t)lights.size();
             R.n_lights = q.n_lights;
             for (uint32_t l = 0; l < q.n_lights; ++l) {
@@ -971,6 +995,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
                 for (int b = 0; b < 3; ++b) Lq.rt[3 * a + b] = g.rotation[3 * b + a];
             Lq.zsign = g.z_positive ? 1.0 : -1.0;
             Lq.nx = g.nx;
+            Lq.tiles = fast_div((g.nx + 7) / 8);
             Lq.ny = g.ny;
             Lq.tan_base = tan_total;
             tan_total += g.nx + g.ny;
@@ -1001,6 +1026,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         S.s0 = s0;
         S.ns = ns;
         S.npix = npix;
+        S.by_npix = fast_div(npix);
         S.path_base = w.n_paths;
         S.upd_base = w.n_update;
         S.active = active;
@@ -1313,7 +1339,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
                 CRT_CUDA(cudaMemsetAsync(acount, 0, 4, st));
                 const RReq& R = rr[h->rr_index];
                 k_compact<<<grid_for(ctx, k_compact, h->n_active), 256, 0, st>>>(h->active, h->n_active, B.done, R.pix_base,
-                                                                       R.c.W, R.c.H, out, acount);
+                                                                       R.c, out, acount);
                 check_launch(ctx, "k_compact");
                 uint32_t cnt = 0;
                 CRT_CUDA(cudaMemcpyAsync(&cnt, acount, 4, cudaMemcpyDeviceToHost, st));
@@ -1790,7 +1816,8 @@ bool engine_admit(WaveEngine* e, const crt_request& q, uint64_t tag) {
         R.sv = scene_view(q.scene);
         R.cam = cam;
         R.c = RenderCtl{cam.width, cam.height, p.min_samples, p.max_samples, (float)p.noise_threshold, p.num_bounces,
-                        (uint32_t)p.seed, (uint32_t)(p.seed >> 32), p.request};
+                        (uint32_t)p.seed, (uint32_t)(p.seed >> 32), p.request, fast_div(4u * cam.width),
+                        fast_div(cam.width)};
         R.light_base = r.slot * MAX_LIGHTS;
         R.n_lights = q.n_lights;
         R.pix_base = (uint32_t)r.unit_off;
@@ -2001,7 +2028,8 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
         for (size_t k = 0; k < compacting.size(); ++k) {
             EReq& r = *compacting[k];
             k_compact<<<grid_for(ctx, k_compact, r.n_active), 256, 0, st>>>(r.active, r.n_active, B.done, (uint32_t)r.unit_off,
-                                                                 r.W, r.H, r.act_buf[r.act_sel], e->d_acount + k);
+                                                                 RenderCtl{.W = r.W, .H = r.H, .by4W = fast_div(4u * r.W), .byW = fast_div(r.W)},
+                                                                 r.act_buf[r.act_sel], e->d_acount + k);
             check_launch(ctx, "k_compact");
         }
         std::vector<uint32_t> cnt(compacting.size());
@@ -2033,6 +2061,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
             for (int b = 0; b < 3; ++b) L.rt[3 * a + b] = g.rotation[3 * b + a];
         L.zsign = g.z_positive ? 1.0 : -1.0;
         L.nx = g.nx;
+        L.tiles = fast_div((g.nx + 7) / 8);
         L.ny = g.ny;
         L.tan_base = (uint32_t)(r.byte_off / 8);   // byte arena < 32 GiB (checked at creation)
         L.item_base = lidar_items;
@@ -2073,6 +2102,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
             S.s0 = r.next_sample;
             S.ns = ns;
             S.npix = r.npix;
+            S.by_npix = fast_div(r.npix);
             S.active = nullptr;
         } else {
             if (r.n_active > room) {
@@ -2083,6 +2113,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
             S.s0 = r.next_sample;
             S.ns = 1;
             S.npix = r.n_active;
+            S.by_npix = fast_div(r.n_active);
             S.active = r.active;
         }
         S.path_base = w.n_paths;

@@ -454,9 +454,9 @@ SrpWave srp_wave(const SrpPlan& P, const SrpAtt* d_att, char* state, uint64_t ca
     SrpWave W;
     W.att = d_att;
     W.G = P.G;
-    W.tiles_x = P.tiles_x;
+    W.tiles_x = fast_div(P.tiles_x);
     W.tiles = P.tiles;
-    W.items_per_att = (uint32_t)P.ipa;
+    W.items_per_att = fast_div((uint32_t)P.ipa);
     W.i0 = i0;
     W.a0 = (uint32_t)(i0 / P.ipa);
     W.r0 = (uint32_t)(i0 % P.ipa);

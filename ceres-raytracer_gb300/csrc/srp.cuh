@@ -26,8 +26,8 @@ struct SrpAtt {
 
 struct SrpWave {
     const SrpAtt* att;
-    uint32_t G, tiles_x, tiles;
-    uint32_t items_per_att;   // multiple of SRP_BLOCK_ITEMS
+    uint32_t G, tiles;
+    FastDiv tiles_x, items_per_att;   // the latter a multiple of SRP_BLOCK_ITEMS
     uint64_t i0;              // first item of the wave
     uint32_t a0, r0;          // i0 = a0 * items_per_att + r0
     uint32_t multi;           // the wave holds whole attitudes (r0 == 0) rather than part of one
@@ -42,8 +42,8 @@ struct SrpWave {
 // attitude of wave item i (32-bit arithmetic: a wave is whole attitudes or a part of one)
 __device__ __forceinline__ uint32_t srp_att(const SrpWave& W, uint32_t i, uint32_t& local) {
     if (W.multi) {
-        const uint32_t q = i / W.items_per_att;
-        local = i - q * W.items_per_att;
+        const uint32_t q = div_by(i, W.items_per_att);
+        local = i - q * W.items_per_att.d;
         return W.a0 + q;
     }
     local = W.r0 + i;
@@ -53,11 +53,8 @@ __device__ __forceinline__ uint32_t srp_att(const SrpWave& W, uint32_t i, uint32
 __device__ __forceinline__ bool srp_item(const SrpWave& W, uint32_t i, uint32_t& a, uint32_t& px, uint32_t& py) {
     uint32_t local;
     a = srp_att(W, i, local);
-    const uint32_t tile = local >> 5, lane = local & 31u;
-    if (tile >= W.tiles) return false;
-    px = (tile % W.tiles_x) * 8u + (lane & 7u);
-    py = (tile / W.tiles_x) * 4u + (lane >> 3);
-    return px < W.G && py < W.G;
+    if ((local >> 5) >= W.tiles) return false;
+    return tile_px(local, W.tiles_x, W.G, W.G, px, py);
 }
 
 // sun ray of wave item i: 1 to trace, 0 for a padding item, 2 for a ray that misses the enlarged

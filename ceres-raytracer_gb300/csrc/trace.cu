@@ -55,32 +55,25 @@ struct RayAnyJob : JobBase {
     }
 };
 
-__device__ __forceinline__ bool tile_pixel(uint32_t i, uint32_t W, uint32_t H, uint32_t& px, uint32_t& py) {
-    const uint32_t tiles_x = (W + 7) >> 3;
-    const uint32_t tile = i >> 5, w = i & 31u;
-    px = (tile % tiles_x) * 8u + (w & 7u);
-    py = (tile / tiles_x) * 4u + (w >> 3);
-    return px < W && py < H;
-}
-
 // What bounds it: the FP64 of the smooth-shaded hits (GB300 runs a warp's FP64 instruction in 16 cycles), so
 // the point and the barycentrics share one determinant and reciprocal and the ray is not normalised:
 // 1021 x 767 pixels of a smooth-shaded body 175 -> 146 us in the kernel.
 struct PassJob : JobBase {
     static constexpr int kOct = OCT_NEVER;   // trace_oct
     CamBasis cam;
+    FastDiv tiles;
     double* xyz;
     uint32_t* ids;
     double* normals;
     __device__ bool ray(uint32_t i, TRay& r, Item&) const {
         uint32_t px, py;
-        if (!tile_pixel(i, cam.width, cam.height, px, py)) return false;
+        if (!tile_px(i, tiles, cam.width, cam.height, px, py)) return false;
         r = camera_ray(cam, (float)px, (float)py);
         return true;
     }
     __device__ void write(const SceneView& sv, uint32_t i, const TRay&, const THit& h, const Item&) const {
         uint32_t px, py;
-        tile_pixel(i, cam.width, cam.height, px, py);
+        tile_px(i, tiles, cam.width, cam.height, px, py);
         const size_t pix = (size_t)py * cam.width + px;
         double x[3] = {0.0, 0.0, 0.0};
         float3 nrm = f3(0.f, 0.f, 0.f);
@@ -168,6 +161,7 @@ struct LidarGridJob : JobBase {
     double rt[9];         // R^T row-major (world = rt * sensor direction)
     double zsign;
     uint32_t nx, ny;
+    FastDiv tiles;
     const double* tx;     // nx tangents
     const double* ty;     // ny tangents
     double* range;
@@ -179,7 +173,7 @@ struct LidarGridJob : JobBase {
     }
     __device__ bool ray(uint32_t i, TRay& r, Item&) const {
         uint32_t px, py;
-        if (!tile_pixel(i, nx, ny, px, py)) return false;
+        if (!tile_px(i, tiles, nx, ny, px, py)) return false;
         double d[3];
         beam64(px, py, d);
         beam_keep(d);
@@ -191,7 +185,7 @@ struct LidarGridJob : JobBase {
     }
     __device__ void write(const SceneView& sv, uint32_t i, const TRay&, const THit& h, const Item&) const {
         uint32_t px, py;
-        tile_pixel(i, nx, ny, px, py);
+        tile_px(i, tiles, nx, ny, px, py);
         const size_t k = (size_t)py * nx + px;
         double rng = 0.0;
         if (h.slot != CRT_MISS) {
@@ -270,7 +264,7 @@ int crt_passes(crt_scene* s, const crt_camera_desc* cam, double* xyz, uint32_t* 
         double* d_xyz = (double*)out_direct(ctx, xyz, np * 24, SCR_OUT0);
         uint32_t* d_ids = (uint32_t*)out_direct(ctx, ids, np * 4, SCR_OUT1);
         double* d_nrm = (double*)out_direct(ctx, normals, np * 24, SCR_OUT2);
-        launch_trace<false>(s, PassJob{{}, cb, d_xyz, d_ids, d_nrm}, tiles_items(cb.width, cb.height));
+        launch_trace<false>(s, PassJob{{}, cb, fast_div((cb.width + 7) / 8), d_xyz, d_ids, d_nrm}, tiles_items(cb.width, cb.height));
         out_finish(ctx, xyz, d_xyz, np * 24);
         out_finish(ctx, ids, d_ids, np * 4);
         out_finish(ctx, normals, d_nrm, np * 24);
@@ -314,6 +308,7 @@ int crt_lidar_grid(crt_scene* s, const crt_lidar_grid_desc* g, double* range, ui
         J.zsign = g->z_positive ? 1.0 : -1.0;
         J.nx = g->nx;
         J.ny = g->ny;
+        J.tiles = fast_div((g->nx + 7) / 8);
         const uint32_t nt = g->nx + g->ny;
         double* d_tan = (double*)ctx_scratch(ctx, SCR_IN0, (size_t)nt * sizeof(double));
         k_tan_table<<<(nt + 255) / 256, 256, 0, ctx->stream>>>(d_tan, g->nx, g->ny, g->half_angle_x, g->half_angle_y);
