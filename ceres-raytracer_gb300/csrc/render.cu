@@ -10,9 +10,10 @@
 //             segments follow: srp_wave_stages)
 //   shade     surface point, one shadow ray per light, bounce ray             (k_shade)
 //   shadow    any hit for the shadow queue                                     (persistent trace)
-//   accum     sum lights, clamp after the first bounce, times path weight      (k_accum; folded into
-//             k_update when the wave has at most one bounce: bounce 0's weight is the constant
-//             2 pi and its radiance starts at zero, so neither is stored)
+//             (the light of a vertex, summed, clamped after the first bounce, times the path weight, is
+//             added where the path is handled next: by the next bounce's shade, or after its last vertex
+//             by the update; bounce 0's weight is the constant 2 pi and its radiance starts at zero, so
+//             neither is stored)
 //   bounce    closest hit for the continuing-path queue                        (persistent trace)
 //   update    per-pixel running mean and adaptive stop, samples in order       (k_update; with a
 //             fixed sample count the request's last slice also stores the outputs)
@@ -127,13 +128,13 @@ struct Batch {
     float4* ray;
     uint32_t* skip;
     float4* hit;
-    float4* wgt[2];            // path weight at bounce b >= 1 in wgt[b & 1] (bounce 0: path_weight's constant)
+    float* wgt[2];             // path weight (of every channel) at bounce b >= 1 in wgt[b & 1] (bounce 0:
+                               // path_weight's constant)
     float4* rad;               // radiance gathered so far (written from bounce 0's accumulation on)
     uint32_t* preq;
     uint32_t* ppix;
     uint32_t* psample;
-    float4* contrib;
-    uint8_t* occ;
+    float4* contrib;           // contribution of light l at p * L + l; w: not zero when the light is hidden
     float4* sray;              // shadow ray of path p, light l at p * L + l: (origin, skip slot bits) (dir, tmax)
     uint2* sidx;               // shadow queue: (p * L + l, request) of each shadow ray to trace, in path order
     float4* pix;               // per-pixel running mean (all render requests)
@@ -327,7 +328,7 @@ struct ShadowJob {
         return true;
     }
     __device__ void write(const SceneView&, uint32_t, const TRay&, const THit& h, const Item& it) const {
-        if (h.slot != CRT_MISS) B.occ[it.k] = 1;
+        if (h.slot != CRT_MISS) B.contrib[it.k].w = 1.0f;
     }
 };
 
@@ -384,11 +385,10 @@ __global__ void k_wave_begin(Batch B) {
     if (threadIdx.x < 9) B.counts[threadIdx.x] = 0;
 }
 __global__ void k_wave_end(Batch B) { *B.wave_idx += 1; }
-// Path weight at bounce b: Color(2*M_PI) at the camera vertex (unidirectional.hpp:38), then
-// multiplied by (1 - r1) per bounce (k_shade)
-__device__ __forceinline__ float4 path_weight(const Batch& B, uint32_t p, int bounce) {
-    const float w0 = (float)(2.0 * 3.14159265358979323846);
-    return bounce == 0 ? make_float4(w0, w0, w0, 0.f) : B.wgt[bounce & 1][p];
+// Path weight at bounce b, the same for every channel: Color(2*M_PI) at the camera vertex
+// (unidirectional.hpp:38), then multiplied by (1 - r1) per bounce (k_shade)
+__device__ __forceinline__ float path_weight(const Batch& B, uint32_t p, int bounce) {
+    return bounce == 0 ? (float)(2.0 * 3.14159265358979323846) : B.wgt[bounce & 1][p];
 }
 
 // ---------------------------------------------------------------- shade
@@ -507,7 +507,7 @@ __device__ __noinline__ uint32_t mark_self_occluded(const Batch& B, uint32_t p, 
         const size_t k = (size_t)p * B.L + l;
         const float4 db = B.sray[2 * k + 1];   // direction and distance as written by shade_path
         if (shadow_self_occluded(f3(db.x, db.y, db.z), db.w, f3(nc.x, nc.y, nc.z), nc.w)) {
-            B.occ[k] = 1;
+            B.contrib[k].w = 1.0f;
             keep &= ~(1u << l);
         } else {
             B.sray[2 * k].w = __uint_as_float(CRT_MISS);
@@ -553,7 +553,6 @@ __device__ __forceinline__ uint32_t shade_path(const Batch& B, int bounce, uint3
         const float ldn = -dot3(dir, sp.shading_n);
         const float3 cb = col * ldn;
         B.contrib[(size_t)p * B.L + l] = make_float4(cb.x * inten, cb.y * inten, cb.z * inten, 0.f);
-        B.occ[(size_t)p * B.L + l] = 0;
         if (dot3(dir, sp.flat_n) > 0.0f) cross |= 1u << l;   // checked below
         const size_t k = (size_t)p * B.L + l;
         B.sray[2 * k] = make_float4(x.x, x.y, x.z, __uint_as_float(h.slot));   // tmin 0; skip the origin triangle
@@ -569,8 +568,7 @@ __device__ __forceinline__ uint32_t shade_path(const Batch& B, int bounce, uint3
         // sampled about a smooth-shading normal): the reference meets that triangle again there
         B.skip[p] = dot3(nd, sp.flat_n) > 0.0f ? CRT_MISS : h.slot;
         const float bc = 1.0f - r1;
-        const float4 wt = path_weight(B, p, bounce);
-        B.wgt[(bounce + 1) & 1][p] = make_float4(wt.x * bc, wt.y * bc, wt.z * bc, 0.f);
+        B.wgt[(bounce + 1) & 1][p] = path_weight(B, p, bounce) * bc;
         oct = (__float_as_uint(nd.x) >> 31) | ((__float_as_uint(nd.y) >> 31) << 1) | ((__float_as_uint(nd.z) >> 31) << 2);
     }
     // shadow rays that stop on their own triangle (at every bounce): occluded now, not traced
@@ -579,10 +577,31 @@ __device__ __forceinline__ uint32_t shade_path(const Batch& B, int bounce, uint3
     return keep | (oct << 16);
 }
 
+// Light reaching path p's vertex at `bounce` (unidirectional.hpp:62-80): the unoccluded contributions
+// in light order, clamped to [0, 1] after the first bounce, times the path weight, added to r.  Called by
+// the next bounce's shade and by the update, with explicit roundings, so both give the same bits.
+__device__ __forceinline__ float4 add_light(const Batch& B, uint32_t p, uint32_t n_lights, int bounce, float4 r) {
+    float3 lr = f3(0.f, 0.f, 0.f);
+    for (uint32_t l = 0; l < n_lights; ++l) {
+        const float4 cb = B.contrib[(size_t)p * B.L + l];
+        if (cb.w == 0.f) lr = f3(__fadd_rn(lr.x, cb.x), __fadd_rn(lr.y, cb.y), __fadd_rn(lr.z, cb.z));
+    }
+    if (bounce >= 1) {   // unidirectional.hpp:74-78
+        lr.x = fminf(fmaxf(lr.x, 0.f), 1.f);
+        lr.y = fminf(fmaxf(lr.y, 0.f), 1.f);
+        lr.z = fminf(fmaxf(lr.z, 0.f), 1.f);
+    }
+    const float w = path_weight(B, p, bounce);
+    return make_float4(__fmaf_rn(lr.x, w, r.x), __fmaf_rn(lr.y, w, r.y), __fmaf_rn(lr.z, w, r.z), 0.f);
+}
+
 // 256-thread blocks (block_append2); the loop's trip count is uniform over a block.  The shadow queue
 // receives the shadow rays still to trace after the shade, in path order within a block; rays that
 // their own triangle stops (mark_self_occluded) are not queued, and the counting build (counters
 // non-null) counts them among the rays resolved without a traversal (counters[3]).
+// From bounce 1 on, the light of the path's previous vertex is added first (its shadow rays have been
+// traced, and shade_path reuses their slots): a kernel of its own for that waited on one load after
+// another, 54 of the Cornell box's 477 us (444 so).
 __global__ void __launch_bounds__(256) k_shade(Batch B, int bounce, const uint32_t* __restrict__ q_in,
                                                uint32_t* __restrict__ q_out, bool any_cont,
                                                unsigned long long* __restrict__ counters) {
@@ -601,11 +620,17 @@ __global__ void __launch_bounds__(256) k_shade(Batch B, int bounce, const uint32
             const float4 hv = B.hit[p];
             h.t = hv.x; h.u = hv.y; h.v = hv.z;
             h.slot = __float_as_uint(hv.w);
-            if (h.slot != CRT_MISS) {
+            if (bounce > 0 || h.slot != CRT_MISS) {
                 req = B.preq[p];
-                const RenderCtl& c = B.rr[req].c;
-                live = bounce < c.num_bounces;
-                cont = bounce < c.num_bounces - 1;
+                const RReq& R = B.rr[req];
+                if (bounce > 0) {
+                    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                    B.rad[p] = add_light(B, p, R.n_lights, bounce - 1, bounce == 1 ? zero : B.rad[p]);
+                }
+                live = h.slot != CRT_MISS && bounce < R.c.num_bounces;
+                cont = live && bounce < R.c.num_bounces - 1;
+            } else if (any_cont) {   // no vertex: nothing adds to its radiance
+                B.rad[p] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         const uint32_t sp = live ? shade_path(B, bounce, p, req, h, cont) : 0u;
@@ -627,42 +652,6 @@ __global__ void __launch_bounds__(256) k_shade(Batch B, int bounce, const uint32
     }
 }
 
-// ---------------------------------------------------------------- accumulate
-// Light reaching path p's current vertex (unidirectional.hpp:62-80): the unoccluded contributions
-// in light order, clamped to [0, 1] after the first bounce, times the path weight.  Shared by
-// k_accum and the fused accumulate of k_update, with explicit roundings, so both give the same bits.
-__device__ __forceinline__ float4 add_light(const Batch& B, uint32_t p, uint32_t n_lights, int bounce, float4 r) {
-    float3 lr = f3(0.f, 0.f, 0.f);
-    for (uint32_t l = 0; l < n_lights; ++l) {
-        // both loads issued together (the contribution slot exists whether or not it was written)
-        const uint8_t oc = B.occ[(size_t)p * B.L + l];
-        const float4 cb = B.contrib[(size_t)p * B.L + l];
-        if (!oc) lr = f3(__fadd_rn(lr.x, cb.x), __fadd_rn(lr.y, cb.y), __fadd_rn(lr.z, cb.z));
-    }
-    if (bounce >= 1) {   // unidirectional.hpp:74-78
-        lr.x = fminf(fmaxf(lr.x, 0.f), 1.f);
-        lr.y = fminf(fmaxf(lr.y, 0.f), 1.f);
-        lr.z = fminf(fmaxf(lr.z, 0.f), 1.f);
-    }
-    const float4 wa = path_weight(B, p, bounce);
-    return make_float4(__fmaf_rn(lr.x, wa.x, r.x), __fmaf_rn(lr.y, wa.y, r.y), __fmaf_rn(lr.z, wa.z, r.z), 0.f);
-}
-
-__global__ void k_accum(Batch B, int bounce, const uint32_t* __restrict__ q_in) {
-    const uint32_t n = bounce == 0 ? B.cur->n_paths : B.counts[2 * ((bounce - 1) % 3)];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t p = bounce == 0 ? i : q_in[i];
-        const bool hit = __float_as_uint(B.hit[p].w) != CRT_MISS;
-        const RReq& R = B.rr[B.preq[p]];
-        if (bounce == 0) {   // every path of the wave: its radiance starts here
-            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-            B.rad[p] = hit && R.c.num_bounces > 0 ? add_light(B, p, R.n_lights, 0, zero) : zero;
-        } else if (hit && bounce < R.c.num_bounces) {
-            B.rad[p] = add_light(B, p, R.n_lights, bounce, B.rad[p]);
-        }
-    }
-}
-
 // ---------------------------------------------------------------- pixel update (do_render.hpp:84-114)
 // Final RGBA float and clamp(v * 256, 0, 255) bytes of a pixel (do_render.hpp:118-134)
 __device__ __forceinline__ void store_pixel(const RReq& R, uint32_t pixel, float4 m) {
@@ -675,7 +664,8 @@ __device__ __forceinline__ void store_pixel(const RReq& R, uint32_t pixel, float
     }
 }
 
-// ACC0: the wave's only bounce is bounce 0 and its light is added here instead of by k_accum.
+// Adds the light of each path's last vertex: a path whose last ray hit ends at bounce num_bounces - 1.
+// ACC0: every request of the wave has at most one bounce, so there is no radiance to add to.
 // A request with a fixed sample count (fin_update) gets its outputs from its last slice here.
 template <bool ACC0>
 __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
@@ -710,17 +700,14 @@ __global__ void __launch_bounds__(256, 5) k_update(Batch B) {
         for (uint32_t k = 0; k < S.ns; ++k) {
             const uint32_t sample = S.s0 + k + 1;   // 1-based as in the reference loop
             const size_t p = (size_t)S.path_base + (size_t)k * S.npix + a;
-            float4 L;
-            if (ACC0) {
-                // the lights' flags and contributions are read with the hit flag, not after it (a missed
-                // path's slots hold stale values, which are not used)
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                const bool hit = __float_as_uint(B.hit[p].w) != CRT_MISS;
-                const float4 Lh = add_light(B, (uint32_t)p, R.n_lights, 0, zero);
-                L = R.c.num_bounces > 0 && hit ? Lh : zero;
-            } else {
-                L = B.rad[p];
-            }
+            // the lights' contributions are read with the hit flag, not after it (a missed path's slots
+            // hold stale values, which are not used)
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const bool hit = __float_as_uint(B.hit[p].w) != CRT_MISS;
+            const int nb = R.c.num_bounces;
+            const float4 before = ACC0 || nb <= 1 ? zero : B.rad[p];
+            const float4 Lh = add_light(B, (uint32_t)p, R.n_lights, ACC0 ? 0 : max(nb - 1, 0), before);
+            const float4 L = nb > 0 && hit ? Lh : before;
             const float inv = 1.0f / (float)sample;
             const float dx = (L.x - m.x) * inv, dy = (L.y - m.y) * inv, dz = (L.z - m.z) * inv;
             m.x += dx; m.y += dy; m.z += dz;
@@ -829,7 +816,7 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
                          const std::function<void()>* srp_stages = nullptr, uint32_t* srp_mask = nullptr,
                          size_t srp_mask_len = 0, size_t min_tris = 0, bool direct = false) {
     cudaStream_t st = ctx->stream;
-    const uint32_t g_shade = grid_for(ctx, k_shade, P), g_accum = grid_for(ctx, k_accum, P);
+    const uint32_t g_shade = grid_for(ctx, k_shade, P);
     const uint32_t g_update = max_bounces <= 1 ? grid_for(ctx, k_update<true>, P) : grid_for(ctx, k_update<false>, P);
     if (!direct) {
         k_wave_begin<<<1, 512, 0, st>>>(B);
@@ -848,17 +835,12 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
     }
     const uint32_t* q_in = nullptr;
     uint32_t* q_out = qa;
-    const bool fuse = max_bounces <= 1;   // k_update adds the light of the only bounce (if any)
     for (int b = 0; b < max_bounces; ++b) {
         k_shade<<<g_shade, 256, 0, st>>>(B, b, q_in, q_out, b < max_bounces - 1,
                                          ctx->counting ? ctx->d_counters : nullptr);
         check_launch(ctx, "k_shade");
         launch_trace<true>(ctx, SceneView{}, ShadowJob{B}, (uint32_t)std::min<size_t>(P * NL, 0xFFFFFF00u),
                            &B.counts[2 * (b % 3) + 1], B.counts + 7, min_tris);
-        if (!fuse) {
-            k_accum<<<g_accum, 256, 0, st>>>(B, b, q_in);
-            check_launch(ctx, "k_accum");
-        }
         if (b < max_bounces - 1) {
             launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[2 * (b % 3)],
                                 B.counts + 8, min_tris);
@@ -866,7 +848,7 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
             q_out = (q_out == qa) ? qb : qa;
         }
     }
-    if (fuse) k_update<true><<<g_update, 256, 0, st>>>(B);
+    if (max_bounces <= 1) k_update<true><<<g_update, 256, 0, st>>>(B);
     else k_update<false><<<g_update, 256, 0, st>>>(B);
     check_launch(ctx, "k_update");
     if (direct) return;
@@ -1122,14 +1104,13 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
         B.ray = (float4*)take(P * 32);
         B.skip = (uint32_t*)take(P * 4);
         B.hit = (float4*)take(P * 16);
-        B.wgt[0] = (float4*)take(P * 16);
-        B.wgt[1] = (float4*)take(P * 16);
+        B.wgt[0] = (float*)take(P * 4);
+        B.wgt[1] = (float*)take(P * 4);
         B.rad = (float4*)take(P * 16);
         B.preq = (uint32_t*)take(P * 4);
         B.ppix = (uint32_t*)take(P * 4);
         B.psample = (uint32_t*)take(P * 4);
         B.contrib = (float4*)take(P * NL * 16);
-        B.occ = (uint8_t*)take(P * NL);
         B.sray = (float4*)take(P * NL * 32);
         B.sidx = (uint2*)take(P * NL * 8);
         B.pix = (float4*)take((size_t)std::max<uint32_t>(pix_total, 1) * 16);
@@ -1986,14 +1967,13 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
         B.ray = (float4*)take(P * 32);
         B.skip = (uint32_t*)take(P * 4);
         B.hit = (float4*)take(P * 16);
-        B.wgt[0] = (float4*)take(P * 16);
-        B.wgt[1] = (float4*)take(P * 16);
+        B.wgt[0] = (float*)take(P * 4);
+        B.wgt[1] = (float*)take(P * 4);
         B.rad = (float4*)take(P * 16);
         B.preq = (uint32_t*)take(P * 4);
         B.ppix = (uint32_t*)take(P * 4);
         B.psample = (uint32_t*)take(P * 4);
         B.contrib = (float4*)take(P * NL * 16);
-        B.occ = (uint8_t*)take(P * NL);
         B.sray = (float4*)take(P * NL * 32);
         B.sidx = (uint2*)take(P * NL * 8);
     }
