@@ -308,6 +308,7 @@ struct PrimaryJobT {
 };
 
 struct ShadowJob {
+    static constexpr bool kCoop = true;    // trace_coop
     static constexpr int kMinBlocks = 7;   // trace_min_blocks
     Batch B;
     struct Item {
@@ -333,6 +334,7 @@ struct ShadowJob {
 };
 
 struct BounceJob {
+    static constexpr bool kCoop = true;
     static constexpr int kMinBlocks = 7;
     Batch B;
     const uint32_t* q;
@@ -840,7 +842,7 @@ void launch_wave_kernels(crt_context* ctx, const Batch& B, size_t P, size_t NL, 
                                          ctx->counting ? ctx->d_counters : nullptr);
         check_launch(ctx, "k_shade");
         launch_trace<true>(ctx, SceneView{}, ShadowJob{B}, (uint32_t)std::min<size_t>(P * NL, 0xFFFFFF00u),
-                           &B.counts[2 * (b % 3) + 1], B.counts + 7, min_tris);
+                           &B.counts[2 * (b % 3) + 1], B.counts + 7, min_tris, b == 0);
         if (b < max_bounces - 1) {
             launch_trace<false>(ctx, SceneView{}, BounceJob{B, q_out}, (uint32_t)P, &B.counts[2 * (b % 3)],
                                 B.counts + 8, min_tris);

@@ -104,6 +104,7 @@ struct SrpPrimaryJob : JobBase {
 
 // continuing rays: a compacted queue of item indices (hits still land at the item's own slot)
 struct SrpBounceJob {
+    static constexpr bool kCoop = true;    // trace_coop
     static constexpr int kOct = OCT_COUNT;   // trace_oct
     SrpWave W;
     const uint32_t* q;
@@ -321,6 +322,7 @@ __global__ void __launch_bounds__(SRP_SHADE_THREADS) k_srp_shade_dev(const SrpSt
 
 // continuing rays of a device stage descriptor's range
 struct SrpBounceJobDev {
+    static constexpr bool kCoop = true;
     static constexpr int kMinBlocks = 7;   // trace_min_blocks
     static constexpr int kOct = OCT_COUNT;
     const SrpStage* S;

@@ -15,7 +15,8 @@ namespace {
 
 // ---------------------------------------------------------------- jobs
 struct RayClosestJob : JobBase {
-    static constexpr int kOct = OCT_SMALL;   // trace_oct
+    static constexpr bool kCoop = true;     // trace_coop
+    static constexpr int kOct = OCT_MID;   // trace_oct
     const float4* rays;   // crt_ray as 2 x float4
     crt_hit* hits;
     __device__ bool ray(uint32_t i, TRay& r, Item&) const {
@@ -40,6 +41,8 @@ struct RayClosestJob : JobBase {
 };
 
 struct RayAnyJob : JobBase {
+    static constexpr bool kCoop = true;     // trace_coop
+    static constexpr int kOct = OCT_MID;   // trace_oct
     const float4* rays;
     uint8_t* occluded;
     __device__ bool ray(uint32_t i, TRay& r, Item&) const {

@@ -115,16 +115,19 @@ struct trace_beam_bytes<J, std::void_t<decltype(J::kKeepsBeam)>> {
 
 // Which kernel a launch takes.  k_trace, a lane per ray, has the higher throughput; but a small launch lasts
 // as long as its longest chain of node visits, and there k_trace_oct, eight lanes per ray, is faster.  Of
-// a scene's asteroid-like bodies (4 k .. 500 k triangles), 30 k rays or camera paths: 1.03 - 1.48 times;
-// 60 k random closest-hit rays 0.84 - 0.89, any-hit rays and camera paths 1.04 - 1.20 from 32 k triangles
-// on, 0.88 - 1.0 below; 100 k and more 0.5 - 1.1.  Jobs with FP64 work per ray stay with k_trace (OCT_NEVER):
-// a warp's FP64 instruction takes the same 16 cycles for four rays as for 32.  So do scenes of fewer than
-// SMALL_SCENE triangles, whose rays are done in a few nodes.
-constexpr uint32_t OCT_ITEMS = 40000, OCT_ITEMS_DEEP = 80000, OCT_DEEP_TRIS = 32768, SMALL_SCENE = 1024;
-// A job's kOct: OCT_NEVER, OCT_SMALL (up to OCT_ITEMS), OCT_DEEP (the default: up to OCT_ITEMS_DEEP in scenes of
-// OCT_DEEP_TRIS triangles), or OCT_COUNT: the host knows only a bound far above the usual count, so both
-// kernels are launched and the one that the count on the device does not call for returns at once.
-enum { OCT_NEVER, OCT_SMALL, OCT_DEEP, OCT_COUNT };
+// asteroid-like bodies of 4 k / 40 k / 500 k triangles, times of k_trace to k_trace_oct, over the number of rays:
+//   random closest-hit rays  2 k 1.44 / 1.53 / 1.46, 21 k 1.03 / 1.10 / 1.18, 31 k 0.89 / 0.95 / 1.08, 40 k 0.79 / 0.82 / 0.95
+//   random any-hit rays      2 k 1.45 / 1.40 / 1.50, 21 k 1.15 / 1.19 / 1.20, 31 k 0.99 / 1.07 / 1.18, 40 k 0.85 / 0.95 / 1.02
+//   path-traced images       21 k 1.08 / 1.28 / 1.39, 31 k 0.99 / 1.15 / 1.29, 58 k 0.89 / 1.04 / 1.20, 78 k 0.86 / 0.98 / 1.12
+// (a buffer's coherent rays cross earlier: 21 k 0.94 / 0.86 / 0.93).  Jobs with FP64 work per ray stay with
+// k_trace (OCT_NEVER): a warp's FP64 instruction takes the same 16 cycles for four rays as for 32.  So do
+// scenes of fewer than SMALL_SCENE triangles, whose rays are done in a few nodes.
+constexpr uint32_t OCT_ITEMS = 28000, OCT_ITEMS_MID = 40000, OCT_ITEMS_DEEP = 80000, OCT_DEEP_TRIS = 32768, SMALL_SCENE = 1024;
+// A job's kOct: OCT_NEVER; OCT_DEEP (the default): up to OCT_ITEMS, in scenes of OCT_DEEP_TRIS triangles
+// OCT_ITEMS_DEEP; OCT_MID: there up to OCT_ITEMS_MID; or OCT_COUNT: as OCT_DEEP, but the host knows only
+// a bound far above the usual count, so both kernels are launched and the one that the count on the device
+// does not call for returns at once.
+enum { OCT_NEVER, OCT_MID, OCT_DEEP, OCT_COUNT };
 template <class J, class = void>
 struct trace_oct {
     static constexpr int value = OCT_DEEP;
@@ -132,6 +135,19 @@ struct trace_oct {
 template <class J>
 struct trace_oct<J, std::void_t<decltype(J::kOct)>> {
     static constexpr int value = J::kOct;
+};
+
+// Jobs whose rays may be incoherent (kCoop) are traced with traverse_coop, unless the launch says that they
+// are not (first shadow rays: 2048^2 of them 3 % slower with it) or the scene is of fewer than SMALL_SCENE
+// triangles (a Cornell box's path-traced image: 563 us with it, 446 without).  A job over a buffer of rays
+// (JobBase) asks per warp (rays_apart).  Camera, beam and sun rays are coherent.
+template <class J, class = void>
+struct trace_coop {
+    static constexpr bool value = false;
+};
+template <class J>
+struct trace_coop<J, std::void_t<decltype(J::kCoop)>> {
+    static constexpr bool value = J::kCoop;
 };
 
 // Persistent ray-queue kernel.  Each warp takes 32 consecutive items per atomic grab, or, with chunk > 1, a
@@ -151,7 +167,7 @@ __device__ __forceinline__ void queue_reset(uint32_t* queue, uint32_t grab) {
     }
 }
 
-template <bool ANY, bool COUNT, class Job>
+template <bool ANY, bool COUNT, bool COOP, class Job>
 __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value) k_trace(SceneView sv, Job job, uint32_t n_items,
                                                             const uint32_t* __restrict__ n_dev,
                                                             uint32_t* __restrict__ queue, uint32_t* __restrict__ err,
@@ -182,7 +198,22 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
             TRay r;
             typename Job::Item it;
             const int kind = i < n_items ? (int)job.ray(i, r, it) : 0;
-            if (kind == 1) {
+            if constexpr (COOP) {
+                if (kind != 1) {
+                    r.o = r.d = f3(0.f, 0.f, 1.f);
+                    r.tmin = r.tmax = 0.f;
+                }
+                THit h;
+                if constexpr (std::is_base_of_v<JobBase, Job>) {
+                    if (rays_apart(sv, r, kind == 1)) h = traverse_coop<ANY, COUNT>(sv, r, kind == 1, trace_smem, st, err);
+                    else if (kind == 1) h = traverse<ANY, COUNT>(sv, r, trace_smem, st, err);
+                } else {
+                    SceneView v{};
+                    if (kind == 1) v = job.view(sv, it);
+                    h = traverse_coop<ANY, COUNT>(v, r, kind == 1, trace_smem, st, err);
+                }
+                if (kind == 1) job.write(sv, i, r, h, it);
+            } else if (kind == 1) {
                 const THit h = traverse<ANY, COUNT>(job.view(sv, it), r, trace_smem, st, err);
                 job.write(sv, i, r, h, it);
             }
@@ -268,33 +299,50 @@ int resident_blocks(crt_context* ctx, Kernel* kernel, size_t smem, std::atomic<i
     return blocks;
 }
 
-// Launches a trace over n_items work items (or over *n_dev items when n_dev is given: n_items is then an
-// upper bound).  tris: triangles of the smallest scene the rays meet, 0: keep to k_trace.
 // queue: a work counter that an earlier operation on the stream has zeroed; null: the context's own.
 // There a small launch finds its counter at zero and leaves it so; past RESET_BLOCKS blocks the atomics of
 // the finishing blocks take longer (2.4 us with 1216) than a memset before the launch, which overlaps
 // the end of the work before it (256 rays: 23.0 us with the memset, 22.0 without).
 constexpr int RESET_BLOCKS = 128;
+inline uint32_t* own_queue(crt_context* ctx, uint32_t* q, int grid, uint32_t& grab) {
+    if (q) return q;
+    q = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
+    if (grid <= RESET_BLOCKS) {
+        grab |= GRAB_RESET;
+        return q;
+    }
+    q += 8;   // words 0 and 1 stay zero for the small launches
+    CRT_CUDA(cudaMemsetAsync(q, 0, sizeof(uint32_t), ctx->stream));
+    return q;
+}
+
+template <bool ANY, bool COOP, class Job>
+void launch_queue(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items, const uint32_t* n_dev,
+                  uint32_t* q, uint32_t over) {
+    static std::atomic<int> known[2] = {{0}, {0}};
+    auto kernel = ctx->counting ? k_trace<ANY, true, COOP, Job> : k_trace<ANY, false, COOP, Job>;
+    constexpr size_t smem = (COOP ? COOP_SMEM : TRACE_SMEM) + trace_beam_bytes<Job>::value;
+    int grid = resident_blocks(ctx, kernel, smem, known[ctx->counting]) * ctx->sm_count;
+    const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
+    if ((uint32_t)grid > need) grid = (int)std::max<uint32_t>(need, 1u);
+    uint32_t grab = ctx->queue_chunk ? ctx->queue_chunk : 1u;
+    q = own_queue(ctx, q, grid, grab);
+    kernel<<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters, grab, over);
+    check_launch(ctx, "k_trace");
+}
+
+// Launches a trace over n_items work items (or over *n_dev items when n_dev is given: n_items is then an
+// upper bound).  tris: triangles of the smallest scene the rays meet, 0: keep to k_trace and traverse.
+// coherent: neighbouring items' rays are alike (of a job that is otherwise taken not to be).
 template <bool ANY, class Job>
 void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_t n_items, const uint32_t* n_dev,
-                  uint32_t* queue, size_t tris) {
+                  uint32_t* queue, size_t tris, bool coherent = false) {
     constexpr int oct = trace_oct<Job>::value;
-    const uint32_t chunk = ctx->queue_chunk ? ctx->queue_chunk : 1u;
     const bool counting = ctx->counting;
-    auto own_queue = [&](uint32_t* q, int grid, uint32_t& grab) {
-        if (q) return q;
-        q = (uint32_t*)ctx_scratch(ctx, SCR_QUEUE, 256);
-        if (grid <= RESET_BLOCKS) {
-            grab |= GRAB_RESET;
-            return q;
-        }
-        q += 8;   // words 0 and 1 stay zero for the small launches
-        CRT_CUDA(cudaMemsetAsync(q, 0, sizeof(uint32_t), ctx->stream));
-        return q;
-    };
     uint32_t over = 0;
     if constexpr (oct != OCT_NEVER) {
-        const uint32_t limit = tris < SMALL_SCENE ? 0u : oct != OCT_SMALL && tris >= OCT_DEEP_TRIS ? OCT_ITEMS_DEEP : OCT_ITEMS;
+        constexpr uint32_t deep = oct == OCT_MID ? OCT_ITEMS_MID : OCT_ITEMS_DEEP;
+        const uint32_t limit = tris < SMALL_SCENE ? 0u : tris >= OCT_DEEP_TRIS ? deep : OCT_ITEMS;
         const bool fits = n_items <= limit, both = oct == OCT_COUNT && limit && !fits;
         if (fits || both) {
             static std::atomic<int> known[2] = {{0}, {0}};
@@ -302,7 +350,7 @@ void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
             const uint32_t want = std::max<uint32_t>((std::min(n_items, limit) + CRT_TRACE_BLOCK / 32 - 1) / (CRT_TRACE_BLOCK / 32), 1u);
             const int grid = (int)std::min<uint32_t>((uint32_t)(resident_blocks(ctx, kernel, OCT_SMEM, known[counting]) * ctx->sm_count), want);
             uint32_t grab = 0;
-            uint32_t* q = own_queue(queue, grid, grab);
+            uint32_t* q = own_queue(ctx, queue, grid, grab);
             kernel<<<grid, CRT_TRACE_BLOCK, OCT_SMEM, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters,
                                                                    grab, both ? limit : 0xFFFFFFFFu);
             check_launch(ctx, "k_trace_oct");
@@ -310,16 +358,13 @@ void launch_trace(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
             over = limit;
         }
     }
-    static std::atomic<int> known[2] = {{0}, {0}};
-    auto kernel = counting ? k_trace<ANY, true, Job> : k_trace<ANY, false, Job>;
-    constexpr size_t smem = TRACE_SMEM + trace_beam_bytes<Job>::value;
-    int grid = resident_blocks(ctx, kernel, smem, known[counting]) * ctx->sm_count;
-    const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
-    if ((uint32_t)grid > need) grid = (int)std::max<uint32_t>(need, 1u);
-    uint32_t grab = chunk;
-    uint32_t* q = own_queue(queue, grid, grab);
-    kernel<<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters, grab, over);
-    check_launch(ctx, "k_trace");
+    if constexpr (trace_coop<Job>::value) {
+        if (!coherent && tris >= SMALL_SCENE) {
+            launch_queue<ANY, true>(ctx, sv, job, n_items, n_dev, queue, over);
+            return;
+        }
+    }
+    launch_queue<ANY, false>(ctx, sv, job, n_items, n_dev, queue, over);
 }
 
 template <bool ANY, class Job>

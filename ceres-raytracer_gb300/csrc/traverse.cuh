@@ -257,6 +257,316 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
     return hit;
 }
 
+// ---------------------------------------------------------------- triangles dealt to the warp
+// The same traversal for incoherent rays.  After a node a few lanes of such a warp have several triangles
+// each and the others none; tested by their own lanes they take as many rounds of the triangle test as
+// the lane with the most has.  Here the warp steps together, and when few triangles are spread unevenly
+// they are dealt to the lanes, 32 a round, which read the owner's ray from shared memory and report a hit
+// there.  The nodes visited and the hits are those of traverse (of equal distances the last triangle wins).
+// Lanes that step together wait for each other, and on coherent rays that costs more than dealing gives:
+// 2048^2 camera rays in tiles take 10 - 15 % longer this way, so it is for rays that are likely to be
+// incoherent (trace_coop).  Per kernel and without it: 3 M random closest-hit rays on 2 M triangles 1500 /
+// 1350 us, 333 k any-hit rays on 100 k 101 / 93 us; with the bounce, later shadow and specular rays of a
+// 24-image batch 3530 / 3466 us, of 12 x 2048^2 sun rays 2645 / 2592 us (whole calls).
+// rays_apart: whether the rays of a warp are such: their directions are of several octants, or their
+// origins lie further apart than an eighth of the scene.  For buffers of rays, of which nothing is known:
+// with it 2048^2 camera rays in tiles take 3 - 6 % longer than in a kernel with traverse alone, against the 10
+// - 15 % (closest hits on 20 k / 500 k / 2 M triangles: 303 / 387 / 436 us alone, 314 / 399 / 449 with
+// both; any hits 213 / 272 / 329 and 228 / 288 / 347).
+__device__ __forceinline__ bool rays_apart(const SceneView& sv, const TRay& ray, bool active) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    const uint32_t live = __ballot_sync(ALL, active);
+    if (!live) return false;
+    const int first = __ffs(live) - 1;
+    const uint32_t ew = __float_as_uint(__ldg(reinterpret_cast<const float4*>(sv.nodes)).w);
+    const float step = fmaxf(fmaxf(__uint_as_float(ew & 0x7F800000u), __uint_as_float((ew << 8) & 0x7F800000u)),
+                             __uint_as_float((ew << 16) & 0x7F800000u));   // the scene is at most 256 of these wide
+    const float dx = fabsf(ray.o.x - __shfl_sync(ALL, ray.o.x, first)), dy = fabsf(ray.o.y - __shfl_sync(ALL, ray.o.y, first)),
+                dz = fabsf(ray.o.z - __shfl_sync(ALL, ray.o.z, first));
+    const uint32_t turn = (__float_as_uint(ray.d.x) ^ __float_as_uint(__shfl_sync(ALL, ray.d.x, first))) |
+                          (__float_as_uint(ray.d.y) ^ __float_as_uint(__shfl_sync(ALL, ray.d.y, first))) |
+                          (__float_as_uint(ray.d.z) ^ __float_as_uint(__shfl_sync(ALL, ray.d.z, first)));
+    const bool apart = (turn >> 31) || fmaxf(fmaxf(dx, dy), dz) > 32.0f * step;
+    return __any_sync(ALL, active && apart);
+}
+
+// smem: the block's COOP_SMEM bytes.  An any-hit traversal returns a slot of 0 for a hit.  Called by the
+// whole warp; `active`: the lane has a ray.
+constexpr uint32_t COOP_OWNER = TRACE_SMEM;   // a lane number per thread
+constexpr uint32_t COOP_SMEM = COOP_OWNER + CRT_TRACE_BLOCK;
+template <bool ANY, bool COUNT>
+__device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, bool active, unsigned char* smem,
+                                              TravStats& st, uint32_t* __restrict__ err) {
+    constexpr uint32_t ALL = 0xFFFFFFFFu;
+    THit hit;
+    hit.slot = CRT_MISS;
+    hit.t = hit.u = hit.v = 0.f;
+    uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
+    // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
+    // -0.0 counts as negative, consistent with safe_rcp(-0.0) < 0
+    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
+                         ((__float_as_uint(ray.d.z) >> 31) << 2);
+    const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
+    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
+    // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative direction enters at hi)
+    // (byte offsets; the exit row is the entry row's partner, an exclusive or away)
+    const uint32_t rowx = (oct & 1u) ? 0x50u : 0x20u, rowy = (oct & 2u) ? 0x60u : 0x30u, rowz = (oct & 4u) ? 0x70u : 0x40u;
+    // the internal child to visit next is the pending one whose slot differs most from the octant: per
+    // slot bit, the slots that differ from the octant in it (in the group's top byte)
+    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
+                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
+    {
+        const TShear sh = make_shear(ray.d);
+        st_shared4(own + TRACE_RAY, sh.bx.x, sh.bx.y, sh.bx.z, shear_proj(ray.o, sh.bx));
+        st_shared4(own + TRACE_RAY + TRACE_ROW, sh.by.x, sh.by.y, sh.by.z, shear_proj(ray.o, sh.by));
+        st_shared4(own + TRACE_RAY + 2 * TRACE_ROW, ray.o.x, ray.o.y, ray.o.z, __uint_as_float(ray.skip));
+        st_shared4(own + TRACE_RAY + 3 * TRACE_ROW, ray.d.x, ray.d.y, ray.d.z, ray.tmin);
+        if (!ANY) st_shared4(own + TRACE_HIT, 0.f, 0.f, 1.f, __uint_as_float(CRT_MISS));
+    }
+    // the nearest hit of a round is found in the first half of the owner's hit row
+    auto best = [&](uint32_t thread) { return reinterpret_cast<unsigned long long*>(smem + TRACE_HIT + 16u * thread); };
+    uint8_t* const s_owner = smem + COOP_OWNER + (threadIdx.x & ~31u);
+    uint2 lstack[CRT_STACK_TOTAL - CRT_STACK_SMEM];
+    int sp = 0;
+    // root = slot 0 of a virtual parent whose children start at node 0
+    uint2 ngroup = make_uint2(0u, active ? 0x01000001u : 0u);
+    uint32_t tmask = 0, tvalid = 0, tbase = 0;
+    while (true) {
+        // ---- leaf triangles of the last visited node
+        const bool with = __any_sync(ALL, tmask != 0u);
+        bool deal = false;
+        if (with) {
+            // A round of dealt triangles takes about as long as 1.6 of the lanes' own, plus 0.6 to deal.
+            // (Dealing whenever a lane has three or more, 12 x 2048^2 sun rays take 6 % longer and
+            // small mirror-like scenes up to 1.6 times; only with at most 16 or 8 lanes that have
+            // triangles, 3 M random rays take 0.3 % and 2.4 % longer.)
+            const uint32_t own_rounds = __reduce_max_sync(ALL, (uint32_t)__popc(tmask));
+            const uint32_t sum = __reduce_add_sync(ALL, (uint32_t)__popc(tmask));
+            deal = 5u * own_rounds > 3u + 8u * ((sum + 31u) >> 5);
+        }
+        if (deal) {
+            // the warp's triangles dealt to its lanes, 32 at a time
+            const uint32_t lane = threadIdx.x & 31u;
+            const uint32_t cnt = __popc(tmask);
+            uint32_t incl = cnt;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(ALL, incl, o);
+                if ((int)lane >= o) incl += y;
+            }
+            const uint32_t total = __shfl_sync(ALL, incl, 31), first = incl - cnt;
+            bool found = false;
+            for (uint32_t r0 = 0; r0 < total; r0 += 32u) {
+                // owners with triangles among [r0, r0 + 32): one bit at each one's first place
+                const bool here = cnt && incl > r0 && first < r0 + 32u;
+                const uint32_t place = max(first, r0) - r0;
+                const uint32_t starts = __reduce_or_sync(ALL, here ? 1u << place : 0u);
+                const uint32_t owners = __ballot_sync(ALL, here);
+                const uint32_t upto = starts & (0xFFFFFFFFu >> (31u - lane));
+                if (here) s_owner[__popc(owners & ((1u << lane) - 1u))] = (uint8_t)lane;
+                __syncwarp();
+                const uint32_t o = s_owner[__popc(upto) - 1];   // the lane's owner
+                const uint32_t ofirst = __shfl_sync(ALL, first, o), ocnt = __shfl_sync(ALL, cnt, o);
+                uint32_t m = __shfl_sync(ALL, tmask, o);
+                const uint32_t ovalid = __shfl_sync(ALL, tvalid, o), obase = __shfl_sync(ALL, tbase, o);
+                const float otmax = __shfl_sync(ALL, ray.tmax, o);
+                const float4* const otris = reinterpret_cast<const float4*>(__shfl_sync(ALL, reinterpret_cast<unsigned long long>(sv.tris), o));
+                const uint32_t k = r0 + lane - ofirst;
+                bool ok = false;
+                float t = 0.f, wv = 0.f, ww = 0.f, det = 1.f;
+                uint32_t slot = 0;
+                const uint32_t ow = own + 16u * (o - lane);
+                if (r0 + lane < total && k < ocnt) {
+                    for (uint32_t q = 0; q < k; ++q) m &= m - 1u;
+                    slot = obase + __popc(ovalid & ((m & (0u - m)) - 1u));
+                    TRay r;
+                    TShear shear;
+                    const float4 q2 = ld_shared4(ow + TRACE_RAY + 2 * TRACE_ROW);
+                    r.o = f3(q2.x, q2.y, q2.z);
+                    r.skip = __float_as_uint(q2.w);
+                    if (slot != r.skip) {
+                        const float4* tp = otris + 3ull * slot;
+                        const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                        const float4 q0 = ld_shared4(ow + TRACE_RAY), q1 = ld_shared4(ow + TRACE_RAY + TRACE_ROW);
+                        const float4 q3 = ld_shared4(ow + TRACE_RAY + 3 * TRACE_ROW);
+                        shear.bx = f3(q0.x, q0.y, q0.z);
+                        shear.ox = q0.w;
+                        shear.by = f3(q1.x, q1.y, q1.z);
+                        shear.oy = q1.w;
+                        r.d = f3(q3.x, q3.y, q3.z);
+                        r.tmin = q3.w;
+                        r.tmax = otmax;
+                        if (COUNT) st.tris++;
+                        ok = tri_test(a, bb, c, r, shear, t, wv, ww, det);
+                    }
+                }
+                const uint32_t hits = __reduce_or_sync(ALL, ok ? 1u << o : 0u);
+                if (hits) {
+                    const bool mine = (hits >> lane) & 1u;
+                    if (ANY) {
+                        found = found || mine;
+                    } else {
+                        // per owner the nearest, of equal ones the last: as when they are tested in turn
+                        const uint32_t tu = __float_as_uint(t);
+                        const unsigned long long key = (unsigned long long)((tu & 0x80000000u) ? ~tu : (tu | 0x80000000u)) << 32 | (0xFFFFFFFFu - slot);
+                        unsigned long long* const sb = best(threadIdx.x - lane + o);
+                        if (mine) *best(threadIdx.x) = ~0ull;   // (the hit that was there is further away)
+                        __syncwarp();
+                        if (ok) atomicMin(sb, key);
+                        __syncwarp();
+                        const bool won = ok && *reinterpret_cast<volatile unsigned long long*>(sb) == key;
+                        if (mine) {
+                            const uint32_t u = (uint32_t)(*reinterpret_cast<volatile unsigned long long*>(best(threadIdx.x)) >> 32);
+                            ray.tmax = __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
+                        }
+                        __syncwarp();
+                        if (won) st_shared4(ow + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
+                        __syncwarp();
+                    }
+                }
+            }
+            if (ANY && found) {
+                hit.slot = 0;
+                ngroup.y = 0;
+                sp = 0;
+            }
+            tmask = 0;
+        } else if (with) {
+            bool stop = false;
+            if (tmask) {
+                TRay r;
+                TShear shear;
+                const float4 q0 = ld_shared4(own + TRACE_RAY), q1 = ld_shared4(own + TRACE_RAY + TRACE_ROW);
+                const float4 q2 = ld_shared4(own + TRACE_RAY + 2 * TRACE_ROW), q3 = ld_shared4(own + TRACE_RAY + 3 * TRACE_ROW);
+                shear.bx = f3(q0.x, q0.y, q0.z);
+                shear.ox = q0.w;
+                shear.by = f3(q1.x, q1.y, q1.z);
+                shear.oy = q1.w;
+                r.o = f3(q2.x, q2.y, q2.z);
+                r.skip = __float_as_uint(q2.w);
+                r.d = f3(q3.x, q3.y, q3.z);
+                r.tmin = q3.w;
+                do {
+                    const uint32_t low = tmask & (0u - tmask);
+                    tmask ^= low;
+                    const uint32_t slot = tbase + __popc(tvalid & (low - 1u));
+                    if (slot == r.skip) continue;
+                    const float4* tp = sv.tris + 3ull * slot;
+                    const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                    if (COUNT) st.tris++;
+                    r.tmax = ray.tmax;
+                    float t, wv, ww, det;
+                    if (tri_test(a, bb, c, r, shear, t, wv, ww, det)) {
+                        if (ANY) {
+                            stop = true;
+                            break;
+                        }
+                        ray.tmax = t;
+                        st_shared4(own + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
+                    }
+                } while (tmask);
+            }
+            if (ANY && stop) {
+                hit.slot = 0;
+                ngroup.y = 0;
+                tmask = 0;
+                sp = 0;
+            }
+        }
+        // ---- next internal node
+        bool go = ngroup.y > 0x00FFFFFFu;
+        if (!go && sp != 0) {
+            --sp;
+            ngroup = sp < CRT_STACK_SMEM ? sstack[sp * CRT_TRACE_BLOCK] : lstack[sp - CRT_STACK_SMEM];
+            go = true;
+        }
+        if (!__any_sync(ALL, go)) break;
+        tmask = 0;
+        if (go) {
+        uint32_t cb = ngroup.y & 0xFF000000u;   // pending children; ends as the one taken
+        uint32_t pr = cb & pick2;
+        cb = pr ? pr : cb;
+        pr = cb & pick1;
+        cb = pr ? pr : cb;
+        pr = cb & pick0;
+        cb = pr ? pr : cb;
+        const uint32_t node = ngroup.x + __popc(ngroup.y & ((cb >> 24) - 1u));
+        ngroup.y ^= cb;
+        if (ngroup.y > 0x00FFFFFFu) {
+            if (sp < CRT_STACK_SMEM) sstack[sp * CRT_TRACE_BLOCK] = ngroup;
+            else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
+            else {
+                atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
+                sp = -1;   // (taken up below: the ray ends)
+            }
+            ++sp;
+        }
+        // ---- visit: test the 8 quantised child boxes
+        const uintptr_t np = reinterpret_cast<uintptr_t>(sv.nodes + node) ^ ((node & 7u) << 4);   // rows permuted
+        auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
+        const float4 w0 = row(0x00u), w1 = row(0x10u);
+        if (COUNT) st.nodes++;
+        const uint32_t ew = __float_as_uint(w0.w);
+        const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
+        const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
+        const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
+        const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
+        const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
+        const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
+        const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+        const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+        // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
+        const float4 xn = row(rowx), xf = row(rowx ^ 0x70u), yn = row(rowy), yf = row(rowy ^ 0x50u), zn = row(rowz),
+                     zf = row(rowz ^ 0x30u);
+        // exit minus entry distance of each child: its sign bit is set where the ray misses the child
+        // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
+        // into `miss` in turn.
+        uint32_t miss = 0;
+#pragma unroll
+        for (int half = 1; half >= 0; --half) {   // children 4 half .. 4 half + 3: two words of each row
+            float2 gap[2];
+#pragma unroll
+            for (int odd = 1; odd >= 0; --odd) {
+                auto dist = [&](const float4& r, f32x2 s, f32x2 a) {
+                    return unpack2(fma2(half ? planes(r.z, r.w, odd) : planes(r.x, r.y, odd), s, a));
+                };
+                const float2 tx0 = dist(xn, sx2, ax2), tx1 = dist(xf, sx2, ax2);
+                const float2 ty0 = dist(yn, sy2, ay2), ty1 = dist(yf, sy2, ay2);
+                const float2 tz0 = dist(zn, sz2, az2), tz1 = dist(zf, sz2, az2);
+                gap[odd].x = fminf(fminf(tx1.x, ty1.x), fminf(tz1.x, ray.tmax)) -
+                             fmaxf(fmaxf(tx0.x, ty0.x), fmaxf(tz0.x, ray.tmin));
+                gap[odd].y = fminf(fminf(tx1.y, ty1.y), fminf(tz1.y, ray.tmax)) -
+                             fmaxf(fmaxf(tx0.y, ty0.y), fmaxf(tz0.y, ray.tmin));
+            }
+            miss = __funnelshift_l(__float_as_uint(gap[1].y), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[0].y), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[1].x), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(gap[0].x), miss, 1);
+        }
+        // internal children that were hit, and the triangles of the leaf children that were hit: each
+        // child's bit spread to three, one per triangle of a leaf (ascending bits are ascending slots)
+        const uint32_t vm = __float_as_uint(w1.z);   // 24 bits of triangles, 8 of internal children
+        const uint32_t hits = ~miss;
+        uint32_t leaf3 = hits & 0xFFu;
+        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
+        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
+        leaf3 = (leaf3 * 0x5u) & 0x249249u;
+        tvalid = vm & 0x00FFFFFFu;
+        tmask = (leaf3 * 7u) & tvalid;
+        tbase = __float_as_uint(w1.y);
+        ngroup = make_uint2(__float_as_uint(w1.x), ((hits << 24) & vm) | (vm >> 24));
+        }
+    }
+    if (ANY) return hit;
+    const float4 h = ld_shared4(own + TRACE_HIT);   // weights of p1 and p2, their sum with p0's, slot
+    hit.slot = __float_as_uint(h.w);
+    const float inv = 1.0f / h.z;
+    hit.t = hit.slot != CRT_MISS ? ray.tmax : 0.0f;
+    hit.u = h.x * inv;
+    hit.v = h.y * inv;
+    return hit;
+}
+
 // ---------------------------------------------------------------- eight lanes per ray
 // The same traversal for launches of few rays, which last as long as their longest chain of dependent
 // node visits: lane c of a ray's eight lanes tests child c, and up to eight triangles are tested at once.
