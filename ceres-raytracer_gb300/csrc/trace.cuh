@@ -150,11 +150,22 @@ struct trace_coop<J, std::void_t<decltype(J::kCoop)>> {
     static constexpr bool value = J::kCoop;
 };
 
+// Jobs with many items that need no traversal (kGroups) name the groups of 32 items that a grab of a large
+// launch takes: where most items end at once, the atomics on the one queue counter are the limit.
+template <class J, class = void>
+struct trace_groups {
+    static constexpr bool value = false;
+};
+template <class J>
+struct trace_groups<J, std::void_t<decltype(J::kGroups)>> {
+    static constexpr bool value = J::kGroups;
+};
+
 // Persistent ray-queue kernel.  Each warp takes 32 consecutive items per atomic grab, or, with chunk > 1, a
 // guided number of up to `chunk` times 32, shrinking with the work left so that the last grabs stay
 // small (few atomics on the queue counter while much work is left, balance at the end).  queue: the next
 // item, zero at the start.  A count of at most `over` items is left to the other kernel.  grab: chunk
-// | GRAB_RESET: leave the queue at zero (queue[1] counts the blocks that have finished).
+// | groups << 8 (trace_groups) | GRAB_RESET: leave the queue at zero (queue[1] counts the blocks that have finished).
 constexpr uint32_t GRAB_RESET = 1u << 31;
 
 __device__ __forceinline__ void queue_reset(uint32_t* queue, uint32_t grab) {
@@ -182,6 +193,7 @@ __global__ void __launch_bounds__(CRT_TRACE_BLOCK, trace_min_blocks<Job>::value)
     const uint32_t chunk = grab & 0xFFu;
     while (true) {
         uint32_t base = 0, take = 1;
+        if constexpr (trace_groups<Job>::value) take = grab >> 8 & 0xFFu;
         if (lane == 0) {
             if (chunk > 1) {
                 const uint32_t cur = *reinterpret_cast<volatile uint32_t*>(queue);
@@ -326,6 +338,8 @@ void launch_queue(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
     const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
     if ((uint32_t)grid > need) grid = (int)std::max<uint32_t>(need, 1u);
     uint32_t grab = ctx->queue_chunk ? ctx->queue_chunk : 1u;
+    if constexpr (trace_groups<Job>::value)   // at least 16 grabs a warp
+        grab |= std::max(1u, std::min(job.groups, (n_items >> 9) / (uint32_t)(grid * (CRT_TRACE_BLOCK / 32)))) << 8;
     q = own_queue(ctx, q, grid, grab);
     kernel<<<grid, CRT_TRACE_BLOCK, smem, ctx->stream>>>(sv, job, n_items, n_dev, q, ctx->d_error, ctx->d_counters, grab, over);
     check_launch(ctx, "k_trace");
