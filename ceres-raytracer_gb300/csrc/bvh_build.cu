@@ -818,7 +818,9 @@ __device__ __forceinline__ void node_grid(float lo, float hi, float& p, int& ex)
 }
 
 // One level of the collapse: eight lanes per wide node (fcount[0] nodes in `frontier`; the next level's are
-// appended to `next` and counted in fcount[1]).  What bounds it: the chain of dependent loads of the cost
+// appended to `next` and counted in fcount[1], once it is known that there is room for them: what is counted
+// has been written, and is at most node_cap entries).  A level of a build that has gone wrong (the error
+// word) does nothing; one that runs out of nodes shows in counters[0] (scene_build).  What bounds it: the chain of dependent loads of the cost
 // decisions and the copies of leaf triangles; the first levels are too small to fill the GPU, so a
 // node's own latency counts.  With one thread per node (736 bytes of local arrays) a level took 133 us
 // on 500 k triangles, 1061 us in all; with eight lanes 205 us in all.
@@ -837,6 +839,7 @@ __global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, con
     const int n = A.n;
     auto oct_ballot = [&](bool b) { return (__ballot_sync(ALL, b) >> oct0) & 0xFFu; };
     auto from = [&](auto v, int k) { return __shfl_sync(ALL, v, oct0 + k); };
+    if (__any_sync(ALL, *A.err != 0u)) return;
     // the warp's four nodes go through every step together (the trip count is uniform over the warp)
     const uint32_t t0 = (blockIdx.x * COLLAPSE_BLOCK + threadIdx.x) / 32u * 4u;
     for (uint32_t tw = t0; tw < todo; tw += octs) {
@@ -992,18 +995,16 @@ __global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, con
         tri_off -= leaf ? (uint32_t)cnt : 0u;
         uint32_t child_base = 0, tri_base = 0, next_base = 0;
         if (sub == 0) {
-            if (n_int) {
-                child_base = atomicAdd(&A.counters[0], n_int);
-                next_base = atomicAdd(&fcount[1], n_int);
-            }
+            if (n_int) child_base = atomicAdd(&A.counters[0], n_int);
             if (n_tri) tri_base = atomicAdd(&A.counters[1], n_tri);
         }
         child_base = from(child_base, 0);
-        next_base = from(next_base, 0);
         tri_base = from(tri_base, 0);
-        const bool fits = child_base + n_int <= A.node_cap && next_base + n_int <= A.node_cap && tri_base + n_tri <= (uint32_t)n;
-        if (!fits && sub == 0) atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
-        const bool write = live && fits && !node_bad;
+        const bool placed = tri_base + n_tri <= (uint32_t)n;
+        if (!placed && sub == 0) atomicOr(A.err, (uint32_t)DEVERR_BUILD_OVERFLOW);
+        const bool write = live && !node_bad && placed && child_base + n_int <= A.node_cap;
+        if (write && sub == 0 && n_int) next_base = atomicAdd(&fcount[1], n_int);
+        next_base = from(next_base, 0);
 
         // child planes in quanta; lane a finds the grid of axis a
         float p[3];
@@ -1887,7 +1888,7 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     // binned-SAH topology for scenes larger than one segment (the context's build setting), else
     // Karras' radix tree over the Morton order
     const bool sah = ctx->build_sah && n > (uint32_t)SAH_T;
-    bool sah_built = false;   // its root is in front[0] on the device, else it is internal node 0
+    bool sah_built = false;   // its root is in root->x on the device, else it is internal node 0
     // scratch layout
     float* d_xyz = (float*)ctx_scratch(ctx, SCR_BUILD0, nn * 9 * sizeof(float));
     float* d_vnin = any_vn ? (float*)ctx_scratch(ctx, SCR_BUILD1, nn * 9 * sizeof(float)) : nullptr;
@@ -1904,8 +1905,8 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     uint32_t *prim_ent = nullptr, *code_a = nullptr, *idx_a = nullptr, *code_b = nullptr, *idx_b = nullptr;
     uint32_t* code_prim = nullptr;
     float* dpc = nullptr;
-    uint32_t *hist = nullptr, *flags = nullptr, *keys = nullptr, *level_count = nullptr;
-    int2 *child = nullptr, *range = nullptr, *front = nullptr, *front_b = nullptr;
+    uint32_t *hist = nullptr, *flags = nullptr, *keys = nullptr, *counts = nullptr;
+    int2 *child = nullptr, *range = nullptr, *root = nullptr, *front = nullptr, *front_b = nullptr;
     int* parent = nullptr;
     int *tl_cnt = nullptr, *tl_pos = nullptr, *tl_par = nullptr;
     uint32_t* tl_sorted = nullptr;
@@ -1936,7 +1937,8 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
         nbox = (float4*)take(nn * 64);        // 2n - 1 nodes x (lo, hi)
         dpc = (float*)take(nn * 32);          // collapse costs: 8 per internal node
         keys = (uint32_t*)take(64 * 4);
-        level_count = (uint32_t*)take((COLLAPSE_MAX_LEVELS + 1) * 4);
+        counts = (uint32_t*)take((2 + COLLAPSE_MAX_LEVELS + 1) * 4);   // collapse: nodes, triangles, nodes per level
+        root = (int2*)take(8);                // the collapse's first level: binary root, wide node 0
         front = (int2*)take(nn * 8 + 8);
         front_b = (int2*)take(nn * 8 + 8);
         tl_cnt = (int*)take(nn * 4);
@@ -1976,7 +1978,7 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
             std::swap(va, vb);
         }
         // after 4 passes the sorted data is back in (code_a, idx_a)
-        sah_built = sah && sah_topology(ctx, (int)n, tbox, cen, keys, va, code_prim, child, range, parent, front);
+        sah_built = sah && sah_topology(ctx, (int)n, tbox, cen, keys, va, code_prim, child, range, parent, root);
         if (!sah_built && n > 1) {   // radix tree (also when the SAH temporaries do not fit)
             k_karras<<<cdiv(n - 1, BLOCK), BLOCK, 0, st>>>(ka, (int)n, child, range, parent);
             check_launch(ctx, "k_karras");
@@ -2016,21 +2018,13 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
         idx_a = va;
     }
 
-    // wide-node capacity: every wide node but the root is an internal child holding > 3 triangles
-    const uint32_t cap = std::max<uint32_t>(1, n / 3 + 2);
-    CRT_CUDA(cudaMalloc(&s->nodes, sizeof(WideNode) * cap));
     CRT_CUDA(cudaMalloc(&s->tris, sizeof(float4) * 3 * nn));
     CRT_CUDA(cudaMalloc(&s->leaf_prim, sizeof(uint32_t) * nn));
     CRT_CUDA(cudaMalloc(&s->leaf_entity, sizeof(uint32_t) * nn));
     if (any_vn) CRT_CUDA(cudaMalloc(&s->leaf_vn, sizeof(float4) * 3 * nn));
-    uint32_t* counters = keys + 16;
-    const uint32_t c0[2] = {1, 0};
-    CRT_CUDA(cudaMemcpyAsync(counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
-    CRT_CUDA(cudaMemsetAsync(level_count, 0, sizeof(uint32_t) * (COLLAPSE_MAX_LEVELS + 1), st));
-    CRT_CUDA(cudaMemcpyAsync(level_count, c0, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    const int2 root = make_int2(n > 3 ? 0 : ALL_TRIS, 0);
-    if (sah_built) CRT_CUDA(cudaMemsetAsync(&front->y, 0, sizeof(int), st));
-    else CRT_CUDA(cudaMemcpyAsync(front, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+    const int2 whole = make_int2(n > 3 ? 0 : ALL_TRIS, 0);
+    if (sah_built) CRT_CUDA(cudaMemsetAsync(&root->y, 0, sizeof(int), st));
+    else CRT_CUDA(cudaMemcpyAsync(root, &whole, sizeof(whole), cudaMemcpyHostToDevice, st));
 
     CollapseArgs A;
     A.n = (int)n;
@@ -2041,42 +2035,59 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     A.geo = geo;
     A.vn = any_vn ? vn : nullptr;
     A.prim_ent = prim_ent;
-    A.nodes = s->nodes;
     A.tris = s->tris;
     A.leaf_prim = s->leaf_prim;
     A.leaf_vn = s->leaf_vn;
     A.leaf_entity = s->leaf_entity;
-    A.counters = counters;
-    A.node_cap = cap;
+    A.counters = counts;
     A.err = ctx->d_error;
     A.dp = dpc;
     A.cost_tri = ctx->collapse_tri_cost;
 
-    // The levels are launched without waiting for their sizes, which stay on the device (level d of the
-    // tree has at most 8^d nodes): as many as a tree of this size usually has, then a look at the counts,
-    // then two at a time.
-    uint32_t depth = 0;
-    int2 *cur = front, *nxt = front_b;
-    uint32_t lc_h[COLLAPSE_MAX_LEVELS + 1];
-    uint32_t launched = 0, batch = 4;
-    for (uint32_t m = n / 3; m; m /= 8) ++batch;
-    for (uint64_t bound = 1;;) {
-        CRT_CHECK(launched + batch <= COLLAPSE_MAX_LEVELS, CRT_ERR_DEVICE, "BVH collapse did not terminate");
-        for (uint32_t b = 0; b < batch; ++b, ++launched) {
-            const uint32_t grid = std::min<uint32_t>(cdiv(bound, COLLAPSE_BLOCK / 8), (uint32_t)ctx->sm_count * 16);
-            k_collapse<<<grid, COLLAPSE_BLOCK, 0, st>>>(A, cur, level_count + launched, nxt);
-            check_launch(ctx, "k_collapse");
-            std::swap(cur, nxt);
-            bound = std::min<uint64_t>(bound * 8, cap);
+    // Wide-node capacity.  Every wide node but the root holds more than three triangles, and a tree that
+    // fills its nodes has fewer than n / 3.  That is no bound: where all costs are equal (a body whose FP32
+    // vertices coincide, far from the origin: every area zero) or lost beside a much larger one, nodes stay whole
+    // with two children each.  Such a collapse runs out of nodes, counts on (used[0]) and is done again
+    // with a node for every internal node of the binary tree, the most there can be.
+    uint32_t cap = std::max<uint32_t>(1, n / 3 + 2), depth = 0;
+    uint32_t used[2 + COLLAPSE_MAX_LEVELS + 1];   // nodes, triangles, nodes per level
+    const uint32_t* const per_level = used + 2;
+    for (;;) {
+        CRT_CUDA(cudaMalloc(&s->nodes, sizeof(WideNode) * cap));
+        A.nodes = s->nodes;
+        A.node_cap = cap;
+        const uint32_t c0[3] = {1, 0, 1};
+        CRT_CUDA(cudaMemsetAsync(counts, 0, sizeof(used), st));
+        CRT_CUDA(cudaMemcpyAsync(counts, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
+        // The levels are launched without waiting for their sizes, which stay on the device (level d of the
+        // tree has at most 8^d nodes): as many as a tree of this size usually has, then a look at the counts,
+        // then two at a time.
+        const int2* cur = root;
+        int2* nxt = front;
+        uint32_t launched = 0, batch = 4;
+        for (uint32_t m = n / 3; m; m /= 8) ++batch;
+        for (uint64_t bound = 1;;) {
+            CRT_CHECK(launched + batch <= COLLAPSE_MAX_LEVELS, CRT_ERR_DEVICE, "BVH collapse did not terminate");
+            for (uint32_t b = 0; b < batch; ++b, ++launched) {
+                const uint32_t grid = std::min<uint32_t>(cdiv(bound, COLLAPSE_BLOCK / 8), (uint32_t)ctx->sm_count * 16);
+                k_collapse<<<grid, COLLAPSE_BLOCK, 0, st>>>(A, cur, counts + 2 + launched, nxt);
+                check_launch(ctx, "k_collapse");
+                cur = nxt;
+                nxt = nxt == front ? front_b : front;
+                bound = std::min<uint64_t>(bound * 8, cap);
+            }
+            CRT_CUDA(cudaMemcpyAsync(used, counts, sizeof(uint32_t) * (2 + launched + 1), cudaMemcpyDeviceToHost, st));
+            CRT_CUDA(cudaStreamSynchronize(st));
+            if (!per_level[launched]) break;
+            batch = 2;
         }
-        CRT_CUDA(cudaMemcpyAsync(lc_h, level_count, sizeof(uint32_t) * (launched + 1), cudaMemcpyDeviceToHost, st));
-        CRT_CUDA(cudaStreamSynchronize(st));
-        if (!lc_h[launched]) break;
-        batch = 2;
+        for (depth = 0; depth < launched && per_level[depth];) ++depth;
+        if (used[0] <= cap) break;
+        CRT_CHECK(cap < n, CRT_ERR_DEVICE, "BVH collapse has more nodes than its binary tree");
+        CRT_CUDA(cudaFree(s->nodes));
+        s->nodes = nullptr;
+        cap = n;
     }
-    while (depth < launched && lc_h[depth]) ++depth;
-    uint32_t used[2];
-    CRT_CUDA(cudaMemcpyAsync(used, counters, sizeof(used), cudaMemcpyDeviceToHost, st));
     uint32_t kb_h[6] = {0, 0, 0, 0, 0, 0};
     if (n) CRT_CUDA(cudaMemcpyAsync(kb_h, keys, sizeof(kb_h), cudaMemcpyDeviceToHost, st));
     CRT_CUDA(cudaEventRecord(ev1, st));
