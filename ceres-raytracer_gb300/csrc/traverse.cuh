@@ -406,9 +406,11 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                     if (ANY) {
                         found = found || mine;
                     } else {
-                        // per owner the nearest, of equal ones the last: as when they are tested in turn
-                        const uint32_t tu = __float_as_uint(t);
-                        const unsigned long long key = (unsigned long long)((tu & 0x80000000u) ? ~tu : (tu | 0x80000000u)) << 32 | (0xFFFFFFFFu - slot);
+                        // per owner the nearest, of equal ones the last: as when they are tested in turn.
+                        // -0 equals +0: it takes +0's place, and its sign the lowest bit (slots have 31)
+                        const uint32_t tu = __float_as_uint(__fadd_rn(t, 0.0f)), neg0 = __float_as_uint(t) == 0x80000000u;
+                        const unsigned long long key = (unsigned long long)((tu & 0x80000000u) ? ~tu : (tu | 0x80000000u)) << 32 |
+                                                       ((0x7FFFFFFFu - slot) << 1 | neg0);
                         unsigned long long* const sb = best(threadIdx.x - lane + o);
                         if (mine) *best(threadIdx.x) = ~0ull;   // (the hit that was there is further away)
                         __syncwarp();
@@ -416,8 +418,9 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                         __syncwarp();
                         const bool won = ok && *reinterpret_cast<volatile unsigned long long*>(sb) == key;
                         if (mine) {
-                            const uint32_t u = (uint32_t)(*reinterpret_cast<volatile unsigned long long*>(best(threadIdx.x)) >> 32);
-                            ray.tmax = __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
+                            const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(best(threadIdx.x));
+                            const uint32_t u = (uint32_t)(k >> 32);
+                            ray.tmax = __uint_as_float(((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u) | (uint32_t)k << 31);
                         }
                         __syncwarp();
                         if (won) st_shared4(ow + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
@@ -700,10 +703,10 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
                 const uint32_t win = (__ballot_sync(ALL, ok && t == best) >> oct0) & 0xFFu;
                 const int from = (int)oct0 + (win ? 31 - __clz(win) : 0);
                 const float u = __shfl_sync(ALL, wv, from), v = __shfl_sync(ALL, ww, from);
-                const float d = __shfl_sync(ALL, dt, from);
+                const float d = __shfl_sync(ALL, dt, from), tw = __shfl_sync(ALL, t, from);   // (best may be the other zero)
                 const uint32_t sl = __shfl_sync(ALL, slot, from);
                 if (win) {
-                    ray.tmax = best;
+                    ray.tmax = tw;
                     hit.u = u;
                     hit.v = v;
                     det = d;

@@ -1,0 +1,56 @@
+"""Hits at equal distances, -0 beside +0: the triangle that is reported, and its distance
+to the last bit, do not depend on a ray's neighbours or on the size of the launch."""
+import numpy as np
+import pytest
+
+from crt_gb300 import lib, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def vertices():
+    """Rays that start at the vertices of a closed mesh, 32 of a kind at each.  Every triangle comes with each
+    of its vertices first, so that a ray is at distance 0 from six triangles, -0 from those it leaves by the back."""
+    m = scenes.asteroid(2_000, seed=0)
+    f = np.concatenate([np.roll(m.faces, k, axis=1) for k in range(3)])
+    rng = np.random.default_rng(2)
+    at = np.repeat(np.arange(len(m.vertices)), 96)
+    d = np.abs(rng.normal(size=(len(at), 3))) * np.repeat(rng.choice([-1.0, 1.0], (len(at) // 32, 3)), 32, axis=0)
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    return scenes.Mesh(m.vertices, f), lib.make_rays(m.vertices[at].astype(np.float32), d.astype(np.float32))
+
+
+@pytest.mark.parametrize("kind", [vertices])
+def test_hits_do_not_depend_on_the_company(kind):
+    mesh, rays = kind()
+    n = len(rays)
+    assert n > 80_000
+    rng = np.random.default_rng(4)
+    order = rng.permutation(n)
+    back = np.argsort(order)
+    strange = rays.copy()   # rays of all directions, one beside each
+    d = rng.normal(size=(n, 3))
+    strange["d"] = (d / np.linalg.norm(d, axis=1)[:, None]).astype(np.float32)
+    beside = np.stack([rays, strange], 1).ravel()
+    ctx = lib.Context(0)
+    try:
+        sc = ctx.scene([scenes.EntitySpec("m", mesh, smooth=False)])
+
+        def closest(r):
+            h = sc.trace_closest(r)
+            return np.stack([h["prim"], h["t"].view(np.uint32), h["u"].view(np.uint32), h["v"].view(np.uint32)], 1)
+
+        alike = closest(rays)
+        t = alike[:, 1].copy().view(np.float32)
+        hit = alike[:, 0] != lib.CRT_MISS
+        assert (hit & (t == 0) & np.signbit(t)).any() and (hit & (t == 0) & ~np.signbit(t)).any()
+        for what, got in (("shuffled", closest(rays[order])[back]), ("beside others", closest(beside)[::2]),
+                          ("few", np.concatenate([closest(rays[k:k + 20_000]) for k in range(0, n, 20_000)]))):
+            np.testing.assert_array_equal(got, alike, err_msg=what)
+        occluded = sc.trace_any(rays)
+        np.testing.assert_array_equal(occluded != 0, hit)
+        np.testing.assert_array_equal(sc.trace_any(rays[order])[back], occluded)
+        np.testing.assert_array_equal(sc.trace_any(beside)[::2], occluded)
+        np.testing.assert_array_equal(np.concatenate([sc.trace_any(rays[k:k + 20_000]) for k in range(0, n, 20_000)]), occluded)
+    finally:
+        ctx.close()
