@@ -698,7 +698,7 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
                     tmask = 0;
                 }
             } else if (__any_sync(ALL, ok)) {
-                float best = ok ? t : 3.402823466e38f;
+                float best = ok ? t : __uint_as_float(0x7F800000u);   // (+inf may be a hit's distance)
                 for (int o = 1; o < 8; o <<= 1) best = fminf(best, __shfl_xor_sync(ALL, best, o));
                 const uint32_t win = (__ballot_sync(ALL, ok && t == best) >> oct0) & 0xFFu;
                 const int from = (int)oct0 + (win ? 31 - __clz(win) : 0);
