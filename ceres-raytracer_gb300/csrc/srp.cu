@@ -99,13 +99,16 @@ constexpr uint32_t SRP_SHADE_THREADS = 256;
 // covered part is the box's mean silhouette over the grid's area.  With one / two groups: a spacecraft at
 // 0.19 and 4 x 4096^2 rays 2343 / 1797 us, turned to 0.29 and 0.41 and 12 x 2048^2 rays 2600 / 2460 us.
 // At one half (bodies near a cube) two groups gain or lose 3 % (4 x 4096^2 rays, 500 k triangles 7437 / 7530
-// us, 20 k 5405 / 5216), as neighbouring tiles that are traced wait for each other: one.  Four groups are
-// slower than two (spacecraft 12 x 2048^2 2630 us).
+// us, 20 k 5405 / 5216): one.  Bodies that fill their box gain less, and with more triangles nothing, as rays
+// that are traced take longer and the queue matters less: stretched asteroids of 0.25 - 0.45, 12 x 2048^2 and
+// 4 x 4096^2 rays, two groups against one, 20 k triangles -8 to -2 %, 48 k -3 to 0, 100 k -1.5 to +0.7, 200 k
+// +0.2 to +2, 500 k +0.5 to +4 (12 x 2048^2 at 0.25: 1683 / 1558 us at 20 k, 2438 / 2529 us at 500 k).
+// Hence the limit of 100 k.  Four groups are slower than two (spacecraft 12 x 2048^2 2630 us).
 uint32_t srp_groups(const crt_scene* s) {
     double e[3];
     for (int k = 0; k < 3; ++k) e[k] = (double)s->bounds[3 + k] - s->bounds[k];
     const double silhouette = 0.5 * (e[0] * e[1] + e[1] * e[2] + e[2] * e[0]);
-    return silhouette < 0.45 * (e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) ? 2u : 1u;
+    return s->n_tris < 100000 && silhouette < 0.45 * (e[0] * e[0] + e[1] * e[1] + e[2] * e[2]) ? 2u : 1u;
 }
 
 struct SrpPrimaryJob : JobBase {
