@@ -1047,7 +1047,7 @@ void run_batch(crt_context* ctx, const crt_request* reqs, size_t n, crt_batch_st
     std::vector<SrpRange> sranges;
     uint64_t srp_max = 0;
     uint32_t srp_nb = 0;
-    const uint64_t srp_cap = std::max<uint64_t>((uint64_t)cap / SRP_BLOCK_ITEMS * SRP_BLOCK_ITEMS, SRP_BLOCK_ITEMS);
+    const uint64_t srp_cap = srp_wave_cap(cap);
     for (size_t j = 0; j < n_srp; ++j) {
         const SrpPlan& SP = splans[j];
         for (uint64_t i0 = 0; i0 < SP.total;) {
@@ -1868,7 +1868,7 @@ bool engine_admit_srp(WaveEngine* e, crt_scene* scene, const crt_srp_desc& desc,
     auto plan = std::make_shared<SrpPlan>();
     srp_plan(scene, &desc, quats, n_att, *plan);
     if (!e->srp_state) {
-        const uint64_t cap = std::max<uint64_t>((uint64_t)e->want_P / SRP_BLOCK_ITEMS * SRP_BLOCK_ITEMS, SRP_BLOCK_ITEMS);
+        const uint64_t cap = srp_wave_cap(e->want_P);
         const size_t b_state = up256(srp_state_bytes(cap, 1)), b_q = up256(cap * 4);
         CRT_CUDA(cudaMalloc(&e->srp_state, b_state + b_q));
         e->srp_cap = cap;

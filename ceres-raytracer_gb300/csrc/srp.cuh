@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "trace.cuh"
 
+#include <algorithm>
 #include <vector>
 
 constexpr uint32_t SRP_BLOCK_ITEMS = 1024;
@@ -91,6 +92,11 @@ struct SrpPlan {
     size_t natt = 0;                  // attitudes (att holds their table unless the caller keeps it)
     size_t n_att() const { return natt; }
 };
+
+// Items of a wave of at most `paths`: whole blocks, and fewer than 2^31, the dividends of div_by (srp_att)
+inline uint64_t srp_wave_cap(uint32_t paths) {
+    return std::max<uint64_t>(std::min<uint32_t>(paths, 0x7FFFFFFFu) / SRP_BLOCK_ITEMS * SRP_BLOCK_ITEMS, SRP_BLOCK_ITEMS);
+}
 
 // The attitude-independent frame of a request: unit sun direction (inertial), grid centre and
 // half size, cell size and ray power.  srp_attitude turns one quaternion into its grid of rays.
