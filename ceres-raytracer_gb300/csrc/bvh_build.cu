@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace {
 
@@ -1748,42 +1749,59 @@ __global__ void k_karras_seg(const uint32_t* __restrict__ code, int n, const int
     parent[right >= 0 ? right : (n - 1) + ~right] = i;
 }
 
+// Temporaries of sah_topology: about 43 bytes per triangle, which lie where the node boxes and collapse costs
+// (96 bytes) come after it (scene_build), so that a context holds no memory for them.
+struct SahTemp {
+    uint32_t *perm, *flags, *tile, *bins[2], *code;
+    int *task_of[2], *seg_lo, *seg_hi;
+    SahState* state;
+    SahTask *tasks[2], *sub;
+    SahMove* moves;
+    static uint32_t tiles(size_t n) { return (uint32_t)((n + SAH_TILE - 1) / SAH_TILE); }
+    static size_t max_tasks(size_t n) { return n / SAH_SUB + 2; }   // of one level: disjoint ranges of more than SAH_SUB
+    // lays them out from mem (null: only the size) and returns the bytes taken
+    size_t carve(char* mem, size_t n) {
+        size_t off = 0;
+        auto take = [&](auto*& q, size_t count) {
+            q = mem ? reinterpret_cast<std::remove_reference_t<decltype(q)>>(mem + off) : nullptr;
+            off += (count * sizeof(*q) + 255) & ~size_t(255);
+        };
+        take(perm, n);
+        take(task_of[0], n);
+        take(task_of[1], n);
+        take(flags, (size_t)SAH_WORDS * tiles(n));
+        take(tile, tiles(n));
+        take(state, 1);
+        take(tasks[0], max_tasks(n));
+        take(tasks[1], max_tasks(n));
+        take(moves, max_tasks(n));
+        take(bins[0], SAH_TASK_WORDS * max_tasks(n));
+        take(bins[1], SAH_TASK_WORDS * max_tasks(n));
+        take(sub, n / (SAH_T + 1) + 2);
+        take(seg_lo, n);
+        take(seg_hi, n);
+        take(code, n);
+        return off;
+    }
+};
+
 // Binned-SAH binary tree over the Morton-sorted triangles (n > SAH_T): fills child / range / parent
 // like k_karras, writes the triangle order of the tree's leaves to `sorted` (in place of the Morton order)
-// and the root's internal index to *root (device memory).  Returns false, with nothing modified, when its
-// temporaries (about 60 bytes per triangle) cannot be allocated.
-bool sah_topology(crt_context* ctx, int n, const float4* tbox, const float4* cen, const uint32_t* keys,
+// and the root's internal index to *root (device memory).
+void sah_topology(crt_context* ctx, int n, const SahTemp& M, const float4* tbox, const float4* cen, const uint32_t* keys,
                   uint32_t* sorted, const uint32_t* code_by_prim, int2* child, int2* range, int* parent, int2* root) {
     cudaStream_t st = ctx->stream;
-    const size_t max_tasks = (size_t)n / SAH_SUB + 2;   // of one level: disjoint ranges of more than SAH_SUB
-    const uint32_t tiles = (uint32_t)(((size_t)n + SAH_TILE - 1) / SAH_TILE);
+    const size_t max_tasks = SahTemp::max_tasks(n);
+    const uint32_t tiles = SahTemp::tiles(n);
     const uint32_t bin_tiles = (uint32_t)(((size_t)n + SAH_BIN_TILE - 1) / SAH_BIN_TILE);
-    size_t off = 0;
-    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t o_perm = take(4ull * n), o_task0 = take(4ull * n), o_task1 = take(4ull * n),
-                 o_flags = take(4ull * SAH_WORDS * tiles), o_tiles = take(4ull * tiles), o_state = take(sizeof(SahState)),
-                 o_tasks0 = take(sizeof(SahTask) * max_tasks), o_tasks1 = take(sizeof(SahTask) * max_tasks),
-                 o_moves = take(sizeof(SahMove) * max_tasks), o_bins0 = take(4ull * SAH_TASK_WORDS * max_tasks),
-                 o_bins1 = take(4ull * SAH_TASK_WORDS * max_tasks), o_sub = take(sizeof(SahTask) * ((size_t)n / (SAH_T + 1) + 2)),
-                 o_lo = take(4ull * n), o_hi = take(4ull * n), o_code = take(4ull * n);
-    char* mem = nullptr;
-    try {
-        mem = (char*)ctx_scratch(ctx, SCR_BUILD3, off);
-    } catch (const CrtError& e) {   // nothing modified yet: the caller builds a radix tree
-        if (e.status != CRT_ERR_OOM) throw;
-        cudaGetLastError();
-        return false;
-    }
-    uint32_t* perm[2] = {sorted, (uint32_t*)(mem + o_perm)};
-    int* task_of[2] = {(int*)(mem + o_task0), (int*)(mem + o_task1)};
-    uint32_t *flags = (uint32_t*)(mem + o_flags), *tile = (uint32_t*)(mem + o_tiles);
-    SahState* state = (SahState*)(mem + o_state);
-    SahTask* tasks[2] = {(SahTask*)(mem + o_tasks0), (SahTask*)(mem + o_tasks1)};
-    SahMove* moves = (SahMove*)(mem + o_moves);
-    uint32_t* bins[2] = {(uint32_t*)(mem + o_bins0), (uint32_t*)(mem + o_bins1)};
-    SahTask* sub = (SahTask*)(mem + o_sub);
-    uint32_t* code = (uint32_t*)(mem + o_code);
-    const SahTree tree{n, child, range, parent, (int*)(mem + o_lo), (int*)(mem + o_hi)};
+    uint32_t* const perm[2] = {sorted, M.perm};
+    uint32_t *const flags = M.flags, *const tile = M.tile, *const code = M.code;
+    int* const* const task_of = M.task_of;
+    SahState* const state = M.state;
+    SahTask *const *const tasks = M.tasks, *const sub = M.sub;
+    SahMove* const moves = M.moves;
+    uint32_t* const* const bins = M.bins;
+    const SahTree tree{n, child, range, parent, M.seg_lo, M.seg_hi};
 
     CRT_CUDA(cudaMemsetAsync(task_of[0], 0, 4ull * n, st));   // every position in task 0 (the root)
     k_sah_root<<<1, 256, 0, st>>>(keys, n, tasks[0], sub, bins[0], state);
@@ -1831,7 +1849,6 @@ bool sah_topology(crt_context* ctx, int n, const float4* tbox, const float4* cen
     check_launch(ctx, "k_gather_codes");
     k_karras_seg<<<(n + 254) / 256, 256, 0, st>>>(code, n, tree.seg_lo, tree.seg_hi, child, range, parent);
     check_launch(ctx, "k_karras_seg");
-    return true;
 }
 
 inline uint32_t cdiv(size_t a, uint32_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -1888,7 +1905,7 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     // binned-SAH topology for scenes larger than one segment (the context's build setting), else
     // Karras' radix tree over the Morton order
     const bool sah = ctx->build_sah && n > (uint32_t)SAH_T;
-    bool sah_built = false;   // its root is in root->x on the device, else it is internal node 0
+    SahTemp sah_temp;
     // scratch layout
     float* d_xyz = (float*)ctx_scratch(ctx, SCR_BUILD0, nn * 9 * sizeof(float));
     float* d_vnin = any_vn ? (float*)ctx_scratch(ctx, SCR_BUILD1, nn * 9 * sizeof(float)) : nullptr;
@@ -1935,7 +1952,10 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
         parent = (int*)take(nn * 8);          // 2n - 1 entries: internal nodes then leaves
         flags = (uint32_t*)take(nn * 4);
         nbox = (float4*)take(nn * 64);        // 2n - 1 nodes x (lo, hi)
+        char* const over = base ? (char*)nbox : nullptr;   // sah_topology is done before these two are filled
+        const size_t first = off - nn * 64;
         dpc = (float*)take(nn * 32);          // collapse costs: 8 per internal node
+        if (sah) off = std::max(off, first + sah_temp.carve(over, nn));
         keys = (uint32_t*)take(64 * 4);
         counts = (uint32_t*)take((2 + COLLAPSE_MAX_LEVELS + 1) * 4);   // collapse: nodes, triangles, nodes per level
         root = (int2*)take(8);                // the collapse's first level: binary root, wide node 0
@@ -1978,8 +1998,9 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
             std::swap(va, vb);
         }
         // after 4 passes the sorted data is back in (code_a, idx_a)
-        sah_built = sah && sah_topology(ctx, (int)n, tbox, cen, keys, va, code_prim, child, range, parent, root);
-        if (!sah_built && n > 1) {   // radix tree (also when the SAH temporaries do not fit)
+        if (sah) {
+            sah_topology(ctx, (int)n, sah_temp, tbox, cen, keys, va, code_prim, child, range, parent, root);
+        } else if (n > 1) {
             k_karras<<<cdiv(n - 1, BLOCK), BLOCK, 0, st>>>(ka, (int)n, child, range, parent);
             check_launch(ctx, "k_karras");
         }
@@ -2023,7 +2044,7 @@ void scene_build(crt_scene* s, const crt_entity_desc* ents, uint32_t n_ents) {
     CRT_CUDA(cudaMalloc(&s->leaf_entity, sizeof(uint32_t) * nn));
     if (any_vn) CRT_CUDA(cudaMalloc(&s->leaf_vn, sizeof(float4) * 3 * nn));
     const int2 whole = make_int2(n > 3 ? 0 : ALL_TRIS, 0);
-    if (sah_built) CRT_CUDA(cudaMemsetAsync(&root->y, 0, sizeof(int), st));
+    if (sah) CRT_CUDA(cudaMemsetAsync(&root->y, 0, sizeof(int), st));
     else CRT_CUDA(cudaMemcpyAsync(root, &whole, sizeof(whole), cudaMemcpyHostToDevice, st));
 
     CollapseArgs A;
