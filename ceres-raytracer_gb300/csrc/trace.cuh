@@ -333,6 +333,7 @@ void launch_queue(crt_context* ctx, const SceneView& sv, const Job& job, uint32_
                   uint32_t* q, uint32_t over) {
     static std::atomic<int> known[2] = {{0}, {0}};
     auto kernel = ctx->counting ? k_trace<ANY, true, COOP, Job> : k_trace<ANY, false, COOP, Job>;
+    static_assert(!COOP || !trace_beam_bytes<Job>::value, "kept beams and the owners of dealt triangles share a place");
     constexpr size_t smem = (COOP ? COOP_SMEM : TRACE_SMEM) + trace_beam_bytes<Job>::value;
     int grid = resident_blocks(ctx, kernel, smem, known[ctx->counting]) * ctx->sm_count;
     const uint32_t need = (n_items + CRT_TRACE_BLOCK - 1) / CRT_TRACE_BLOCK;
