@@ -98,6 +98,10 @@ __device__ __forceinline__ f32x2 planes(float w0, float w1, bool odd) {
     return pack2(__half2float(__habs(h0)), __half2float(__habs(h1)));
 }
 
+// The end of a ray's range, and with it the distance of a hit, is never -0: a child whose exit is -0 and whose
+// entry +0 would count as missed (visits below), although the triangle test takes them for equal.
+__device__ __forceinline__ float not_neg0(float t) { return __fadd_rn(t, 0.0f); }
+
 // smem: the block's TRACE_SMEM bytes.  An any-hit traversal returns the slot only.
 template <bool ANY, bool COUNT>
 __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned char* smem, TravStats& st,
@@ -105,6 +109,7 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
     THit hit;
     hit.slot = CRT_MISS;
     hit.t = hit.u = hit.v = 0.f;
+    ray.tmax = not_neg0(ray.tmax);
     uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
     const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
     // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
@@ -163,7 +168,7 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
                         hit.slot = slot;
                         return hit;
                     }
-                    ray.tmax = t;
+                    ray.tmax = not_neg0(t);
                     st_shared4(own + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
                 }
             } while (tmask);
@@ -301,6 +306,7 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
     THit hit;
     hit.slot = CRT_MISS;
     hit.t = hit.u = hit.v = 0.f;
+    ray.tmax = not_neg0(ray.tmax);
     uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
     const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
     // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
@@ -406,11 +412,9 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                     if (ANY) {
                         found = found || mine;
                     } else {
-                        // per owner the nearest, of equal ones the last: as when they are tested in turn.
-                        // -0 equals +0: it takes +0's place, and its sign the lowest bit (slots have 31)
-                        const uint32_t tu = __float_as_uint(__fadd_rn(t, 0.0f)), neg0 = __float_as_uint(t) == 0x80000000u;
-                        const unsigned long long key = (unsigned long long)((tu & 0x80000000u) ? ~tu : (tu | 0x80000000u)) << 32 |
-                                                       ((0x7FFFFFFFu - slot) << 1 | neg0);
+                        // per owner the nearest, of equal ones the last: as when they are tested in turn
+                        const uint32_t tu = __float_as_uint(not_neg0(t));
+                        const unsigned long long key = (unsigned long long)((tu & 0x80000000u) ? ~tu : (tu | 0x80000000u)) << 32 | (0xFFFFFFFFu - slot);
                         unsigned long long* const sb = best(threadIdx.x - lane + o);
                         if (mine) *best(threadIdx.x) = ~0ull;   // (the hit that was there is further away)
                         __syncwarp();
@@ -418,9 +422,8 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                         __syncwarp();
                         const bool won = ok && *reinterpret_cast<volatile unsigned long long*>(sb) == key;
                         if (mine) {
-                            const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(best(threadIdx.x));
-                            const uint32_t u = (uint32_t)(k >> 32);
-                            ray.tmax = __uint_as_float(((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u) | (uint32_t)k << 31);
+                            const uint32_t u = (uint32_t)(*reinterpret_cast<volatile unsigned long long*>(best(threadIdx.x)) >> 32);
+                            ray.tmax = __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
                         }
                         __syncwarp();
                         if (won) st_shared4(ow + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
@@ -464,7 +467,7 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                             stop = true;
                             break;
                         }
-                        ray.tmax = t;
+                        ray.tmax = not_neg0(t);
                         st_shared4(own + TRACE_HIT, wv, ww, det, __uint_as_float(slot));
                     }
                 } while (tmask);
@@ -594,6 +597,7 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
     THit hit;
     hit.slot = CRT_MISS;
     hit.t = hit.u = hit.v = 0.f;
+    ray.tmax = not_neg0(ray.tmax);
     float det = 1.0f;
     uint2* const stack = reinterpret_cast<uint2*>(smem) + (threadIdx.x >> 3);
     const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
@@ -706,10 +710,10 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
                 const uint32_t win = (__ballot_sync(ALL, ok && t == best) >> oct0) & 0xFFu;
                 const int from = (int)oct0 + (win ? 31 - __clz(win) : 0);
                 const float u = __shfl_sync(ALL, wv, from), v = __shfl_sync(ALL, ww, from);
-                const float d = __shfl_sync(ALL, dt, from), tw = __shfl_sync(ALL, t, from);   // (best may be the other zero)
+                const float d = __shfl_sync(ALL, dt, from);
                 const uint32_t sl = __shfl_sync(ALL, slot, from);
                 if (win) {
-                    ray.tmax = tw;
+                    ray.tmax = not_neg0(best);
                     hit.u = u;
                     hit.v = v;
                     det = d;
