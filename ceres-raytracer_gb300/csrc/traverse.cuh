@@ -102,6 +102,118 @@ __device__ __forceinline__ f32x2 planes(float w0, float w1, bool odd) {
 // entry +0 would count as missed (visits below), although the triangle test takes them for equal.
 __device__ __forceinline__ float not_neg0(float t) { return __fadd_rn(t, 0.0f); }
 
+// What a node visit needs of the ray.
+struct NodeRay {
+    float3 idir, ood;
+    uint32_t rowx, rowy, rowz;      // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative
+                                    // direction enters at hi), as byte offsets; the exit row is the entry row's
+                                    // partner, an exclusive or away
+    uint32_t pick2, pick1, pick0;   // per slot bit, the slots that differ from the octant in it (in the group's top byte)
+};
+__device__ __forceinline__ NodeRay node_ray(const TRay& ray) {
+    // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
+    // -0.0 counts as negative, consistent with safe_rcp(-0.0) < 0
+    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
+                         ((__float_as_uint(ray.d.z) >> 31) << 2);
+    NodeRay c;
+    c.idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
+    c.ood = f3(-ray.o.x * c.idir.x, -ray.o.y * c.idir.y, -ray.o.z * c.idir.z);
+    c.rowx = (oct & 1u) ? 0x50u : 0x20u;
+    c.rowy = (oct & 2u) ? 0x60u : 0x30u;
+    c.rowz = (oct & 4u) ? 0x70u : 0x40u;
+    c.pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u;
+    c.pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u;
+    c.pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
+    return c;
+}
+
+// Takes the internal child to visit next out of a group and returns its node: the pending one whose slot
+// differs most from the octant.
+__device__ __forceinline__ uint32_t next_child(uint2& group, const NodeRay& c) {
+    uint32_t cb = group.y & 0xFF000000u;   // pending children; ends as the one taken
+    uint32_t pr = cb & c.pick2;
+    cb = pr ? pr : cb;
+    pr = cb & c.pick1;
+    cb = pr ? pr : cb;
+    pr = cb & c.pick0;
+    cb = pr ? pr : cb;
+    const uint32_t node = group.x + __popc(group.y & ((cb >> 24) - 1u));
+    group.y ^= cb;
+    return node;
+}
+
+// Each child's bit spread to three, one per triangle of a leaf (ascending bits are ascending slots).
+__device__ __forceinline__ uint32_t leaf_bits(uint32_t hits) {
+    uint32_t leaf3 = hits & 0xFFu;
+    leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
+    leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
+    leaf3 = (leaf3 * 0x5u) & 0x249249u;
+    return leaf3 * 7u;
+}
+
+// Tests the 8 quantised child boxes of a node: the group of internal children that the ray meets, and the
+// triangles of the leaf children that it meets (tmask, of the node's tvalid, from tbase on).
+__device__ __forceinline__ void visit_node(const WideNode* __restrict__ nodes, uint32_t node, const NodeRay& c, float tmin,
+                                           float tmax, uint2& group, uint32_t& tmask, uint32_t& tvalid, uint32_t& tbase) {
+    const uintptr_t np = reinterpret_cast<uintptr_t>(nodes + node) ^ ((node & 7u) << 4);   // rows permuted
+    auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
+    const float4 w0 = row(0x00u), w1 = row(0x10u);
+    const uint32_t ew = __float_as_uint(w0.w);
+    const float sx = __uint_as_float(ew & 0x7F800000u) * c.idir.x;
+    const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * c.idir.y;
+    const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * c.idir.z;
+    const float ax = fmaf(-256.0f, sx, fmaf(w0.x, c.idir.x, c.ood.x));
+    const float ay = fmaf(-256.0f, sy, fmaf(w0.y, c.idir.y, c.ood.y));
+    const float az = fmaf(-256.0f, sz, fmaf(w0.z, c.idir.z, c.ood.z));
+    const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+    const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+    // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
+    const float4 xn = row(c.rowx), xf = row(c.rowx ^ 0x70u), yn = row(c.rowy), yf = row(c.rowy ^ 0x50u), zn = row(c.rowz),
+                 zf = row(c.rowz ^ 0x30u);
+    // exit minus entry distance of each child: its sign bit is set where the ray misses the child
+    // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
+    // into `miss` in turn.
+    uint32_t miss = 0;
+#pragma unroll
+    for (int half = 1; half >= 0; --half) {   // children 4 half .. 4 half + 3: two words of each row
+        float2 gap[2];
+#pragma unroll
+        for (int odd = 1; odd >= 0; --odd) {
+            auto dist = [&](const float4& r, f32x2 s, f32x2 a) {
+                return unpack2(fma2(half ? planes(r.z, r.w, odd) : planes(r.x, r.y, odd), s, a));
+            };
+            const float2 tx0 = dist(xn, sx2, ax2), tx1 = dist(xf, sx2, ax2);
+            const float2 ty0 = dist(yn, sy2, ay2), ty1 = dist(yf, sy2, ay2);
+            const float2 tz0 = dist(zn, sz2, az2), tz1 = dist(zf, sz2, az2);
+            gap[odd].x = fminf(fminf(tx1.x, ty1.x), fminf(tz1.x, tmax)) -
+                         fmaxf(fmaxf(tx0.x, ty0.x), fmaxf(tz0.x, tmin));
+            gap[odd].y = fminf(fminf(tx1.y, ty1.y), fminf(tz1.y, tmax)) -
+                         fmaxf(fmaxf(tx0.y, ty0.y), fmaxf(tz0.y, tmin));
+        }
+        miss = __funnelshift_l(__float_as_uint(gap[1].y), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(gap[0].y), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(gap[1].x), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(gap[0].x), miss, 1);
+    }
+    const uint32_t vm = __float_as_uint(w1.z);   // 24 bits of triangles, 8 of internal children
+    const uint32_t hits = ~miss;
+    tvalid = vm & 0x00FFFFFFu;
+    tmask = leaf_bits(hits) & tvalid;
+    tbase = __float_as_uint(w1.y);
+    group = make_uint2(__float_as_uint(w1.x), ((hits << 24) & vm) | (vm >> 24));
+}
+
+// The ray constants of the triangle test, and no hit, into the lane's place.
+template <bool ANY>
+__device__ __forceinline__ void ray_to_shared(const TRay& ray, uint32_t own) {
+    const TShear sh = make_shear(ray.d);
+    st_shared4(own + TRACE_RAY, sh.bx.x, sh.bx.y, sh.bx.z, shear_proj(ray.o, sh.bx));
+    st_shared4(own + TRACE_RAY + TRACE_ROW, sh.by.x, sh.by.y, sh.by.z, shear_proj(ray.o, sh.by));
+    st_shared4(own + TRACE_RAY + 2 * TRACE_ROW, ray.o.x, ray.o.y, ray.o.z, __uint_as_float(ray.skip));
+    st_shared4(own + TRACE_RAY + 3 * TRACE_ROW, ray.d.x, ray.d.y, ray.d.z, ray.tmin);
+    if (!ANY) st_shared4(own + TRACE_HIT, 0.f, 0.f, 1.f, __uint_as_float(CRT_MISS));
+}
+
 // smem: the block's TRACE_SMEM bytes.  An any-hit traversal returns the slot only.
 template <bool ANY, bool COUNT>
 __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned char* smem, TravStats& st,
@@ -112,27 +224,8 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
     ray.tmax = not_neg0(ray.tmax);
     uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
     const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
-    // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
-    // -0.0 counts as negative, consistent with safe_rcp(-0.0) < 0
-    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
-                         ((__float_as_uint(ray.d.z) >> 31) << 2);
-    const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
-    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
-    // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative direction enters at hi)
-    // (byte offsets; the exit row is the entry row's partner, an exclusive or away)
-    const uint32_t rowx = (oct & 1u) ? 0x50u : 0x20u, rowy = (oct & 2u) ? 0x60u : 0x30u, rowz = (oct & 4u) ? 0x70u : 0x40u;
-    // the internal child to visit next is the pending one whose slot differs most from the octant: per
-    // slot bit, the slots that differ from the octant in it (in the group's top byte)
-    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
-                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
-    {
-        const TShear sh = make_shear(ray.d);
-        st_shared4(own + TRACE_RAY, sh.bx.x, sh.bx.y, sh.bx.z, shear_proj(ray.o, sh.bx));
-        st_shared4(own + TRACE_RAY + TRACE_ROW, sh.by.x, sh.by.y, sh.by.z, shear_proj(ray.o, sh.by));
-        st_shared4(own + TRACE_RAY + 2 * TRACE_ROW, ray.o.x, ray.o.y, ray.o.z, __uint_as_float(ray.skip));
-        st_shared4(own + TRACE_RAY + 3 * TRACE_ROW, ray.d.x, ray.d.y, ray.d.z, ray.tmin);
-        if (!ANY) st_shared4(own + TRACE_HIT, 0.f, 0.f, 1.f, __uint_as_float(CRT_MISS));
-    }
+    const NodeRay nr = node_ray(ray);
+    ray_to_shared<ANY>(ray, own);
     uint2 lstack[CRT_STACK_TOTAL - CRT_STACK_SMEM];
     int sp = 0;
     // root = slot 0 of a virtual parent whose children start at node 0
@@ -179,15 +272,7 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
             --sp;
             ngroup = sp < CRT_STACK_SMEM ? sstack[sp * CRT_TRACE_BLOCK] : lstack[sp - CRT_STACK_SMEM];
         }
-        uint32_t cb = ngroup.y & 0xFF000000u;   // pending children; ends as the one taken
-        uint32_t pr = cb & pick2;
-        cb = pr ? pr : cb;
-        pr = cb & pick1;
-        cb = pr ? pr : cb;
-        pr = cb & pick0;
-        cb = pr ? pr : cb;
-        const uint32_t node = ngroup.x + __popc(ngroup.y & ((cb >> 24) - 1u));
-        ngroup.y ^= cb;
+        const uint32_t node = next_child(ngroup, nr);
         if (ngroup.y > 0x00FFFFFFu) {
             if (sp < CRT_STACK_SMEM) sstack[sp * CRT_TRACE_BLOCK] = ngroup;
             else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
@@ -197,60 +282,8 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
             }
             ++sp;
         }
-        // ---- visit: test the 8 quantised child boxes
-        const uintptr_t np = reinterpret_cast<uintptr_t>(sv.nodes + node) ^ ((node & 7u) << 4);   // rows permuted
-        auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
-        const float4 w0 = row(0x00u), w1 = row(0x10u);
         if (COUNT) st.nodes++;
-        const uint32_t ew = __float_as_uint(w0.w);
-        const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
-        const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
-        const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
-        const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
-        const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
-        const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
-        const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
-        const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
-        // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
-        const float4 xn = row(rowx), xf = row(rowx ^ 0x70u), yn = row(rowy), yf = row(rowy ^ 0x50u), zn = row(rowz),
-                     zf = row(rowz ^ 0x30u);
-        // exit minus entry distance of each child: its sign bit is set where the ray misses the child
-        // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
-        // into `miss` in turn.
-        uint32_t miss = 0;
-#pragma unroll
-        for (int half = 1; half >= 0; --half) {   // children 4 half .. 4 half + 3: two words of each row
-            float2 gap[2];
-#pragma unroll
-            for (int odd = 1; odd >= 0; --odd) {
-                auto dist = [&](const float4& r, f32x2 s, f32x2 a) {
-                    return unpack2(fma2(half ? planes(r.z, r.w, odd) : planes(r.x, r.y, odd), s, a));
-                };
-                const float2 tx0 = dist(xn, sx2, ax2), tx1 = dist(xf, sx2, ax2);
-                const float2 ty0 = dist(yn, sy2, ay2), ty1 = dist(yf, sy2, ay2);
-                const float2 tz0 = dist(zn, sz2, az2), tz1 = dist(zf, sz2, az2);
-                gap[odd].x = fminf(fminf(tx1.x, ty1.x), fminf(tz1.x, ray.tmax)) -
-                             fmaxf(fmaxf(tx0.x, ty0.x), fmaxf(tz0.x, ray.tmin));
-                gap[odd].y = fminf(fminf(tx1.y, ty1.y), fminf(tz1.y, ray.tmax)) -
-                             fmaxf(fmaxf(tx0.y, ty0.y), fmaxf(tz0.y, ray.tmin));
-            }
-            miss = __funnelshift_l(__float_as_uint(gap[1].y), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[0].y), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[1].x), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[0].x), miss, 1);
-        }
-        // internal children that were hit, and the triangles of the leaf children that were hit: each
-        // child's bit spread to three, one per triangle of a leaf (ascending bits are ascending slots)
-        const uint32_t vm = __float_as_uint(w1.z);   // 24 bits of triangles, 8 of internal children
-        const uint32_t hits = ~miss;
-        uint32_t leaf3 = hits & 0xFFu;
-        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
-        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
-        leaf3 = (leaf3 * 0x5u) & 0x249249u;
-        tvalid = vm & 0x00FFFFFFu;
-        tmask = (leaf3 * 7u) & tvalid;
-        tbase = __float_as_uint(w1.y);
-        ngroup = make_uint2(__float_as_uint(w1.x), ((hits << 24) & vm) | (vm >> 24));
+        visit_node(sv.nodes, node, nr, ray.tmin, ray.tmax, ngroup, tmask, tvalid, tbase);
     }
     if (ANY) return hit;
     const float4 h = ld_shared4(own + TRACE_HIT);   // weights of p1 and p2, their sum with p0's, slot
@@ -309,27 +342,8 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
     ray.tmax = not_neg0(ray.tmax);
     uint2* const sstack = reinterpret_cast<uint2*>(smem) + threadIdx.x;
     const uint32_t own = (uint32_t)__cvta_generic_to_shared(smem) + 16u * threadIdx.x;
-    // octant from the sign bits, as NodeIntersector does with std::signbit (node_intersectors.hpp:25-30):
-    // -0.0 counts as negative, consistent with safe_rcp(-0.0) < 0
-    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
-                         ((__float_as_uint(ray.d.z) >> 31) << 2);
-    const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
-    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
-    // rows of the entry planes per axis (lo rows 2..4, hi rows 5..7; a negative direction enters at hi)
-    // (byte offsets; the exit row is the entry row's partner, an exclusive or away)
-    const uint32_t rowx = (oct & 1u) ? 0x50u : 0x20u, rowy = (oct & 2u) ? 0x60u : 0x30u, rowz = (oct & 4u) ? 0x70u : 0x40u;
-    // the internal child to visit next is the pending one whose slot differs most from the octant: per
-    // slot bit, the slots that differ from the octant in it (in the group's top byte)
-    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
-                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
-    {
-        const TShear sh = make_shear(ray.d);
-        st_shared4(own + TRACE_RAY, sh.bx.x, sh.bx.y, sh.bx.z, shear_proj(ray.o, sh.bx));
-        st_shared4(own + TRACE_RAY + TRACE_ROW, sh.by.x, sh.by.y, sh.by.z, shear_proj(ray.o, sh.by));
-        st_shared4(own + TRACE_RAY + 2 * TRACE_ROW, ray.o.x, ray.o.y, ray.o.z, __uint_as_float(ray.skip));
-        st_shared4(own + TRACE_RAY + 3 * TRACE_ROW, ray.d.x, ray.d.y, ray.d.z, ray.tmin);
-        if (!ANY) st_shared4(own + TRACE_HIT, 0.f, 0.f, 1.f, __uint_as_float(CRT_MISS));
-    }
+    const NodeRay nr = node_ray(ray);
+    ray_to_shared<ANY>(ray, own);
     // the nearest hit of a round is found in the first half of the owner's hit row
     auto best = [&](uint32_t thread) { return reinterpret_cast<unsigned long long*>(smem + TRACE_HIT + 16u * thread); };
     uint8_t* const s_owner = smem + COOP_OWNER + (threadIdx.x & ~31u);
@@ -489,80 +503,20 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
         if (!__any_sync(ALL, go)) break;
         tmask = 0;
         if (go) {
-        uint32_t cb = ngroup.y & 0xFF000000u;   // pending children; ends as the one taken
-        uint32_t pr = cb & pick2;
-        cb = pr ? pr : cb;
-        pr = cb & pick1;
-        cb = pr ? pr : cb;
-        pr = cb & pick0;
-        cb = pr ? pr : cb;
-        const uint32_t node = ngroup.x + __popc(ngroup.y & ((cb >> 24) - 1u));
-        ngroup.y ^= cb;
-        if (ngroup.y > 0x00FFFFFFu) {
-            if (sp < CRT_STACK_SMEM) sstack[sp * CRT_TRACE_BLOCK] = ngroup;
-            else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
-            else {
-                // reported, so the call fails; the ray goes on without what its stack held (to end it here takes
-                // a check after every visit, 0.4 % of 333 k any-hit rays)
-                atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
-                sp = -1;
+            const uint32_t node = next_child(ngroup, nr);
+            if (ngroup.y > 0x00FFFFFFu) {
+                if (sp < CRT_STACK_SMEM) sstack[sp * CRT_TRACE_BLOCK] = ngroup;
+                else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
+                else {
+                    // reported, so the call fails; the ray goes on without what its stack held (to end it here takes
+                    // a check after every visit, 0.4 % of 333 k any-hit rays)
+                    atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
+                    sp = -1;
+                }
+                ++sp;
             }
-            ++sp;
-        }
-        // ---- visit: test the 8 quantised child boxes
-        const uintptr_t np = reinterpret_cast<uintptr_t>(sv.nodes + node) ^ ((node & 7u) << 4);   // rows permuted
-        auto row = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(np ^ off)); };
-        const float4 w0 = row(0x00u), w1 = row(0x10u);
-        if (COUNT) st.nodes++;
-        const uint32_t ew = __float_as_uint(w0.w);
-        const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
-        const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
-        const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
-        const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
-        const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
-        const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
-        const f32x2 sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
-        const f32x2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
-        // entry / exit planes per axis by the ray octant: the lo / hi rows swap by address
-        const float4 xn = row(rowx), xf = row(rowx ^ 0x70u), yn = row(rowy), yf = row(rowy ^ 0x50u), zn = row(rowz),
-                     zf = row(rowz ^ 0x30u);
-        // exit minus entry distance of each child: its sign bit is set where the ray misses the child
-        // (the difference of two floats is zero only where they are equal).  Children 7 .. 0 are shifted
-        // into `miss` in turn.
-        uint32_t miss = 0;
-#pragma unroll
-        for (int half = 1; half >= 0; --half) {   // children 4 half .. 4 half + 3: two words of each row
-            float2 gap[2];
-#pragma unroll
-            for (int odd = 1; odd >= 0; --odd) {
-                auto dist = [&](const float4& r, f32x2 s, f32x2 a) {
-                    return unpack2(fma2(half ? planes(r.z, r.w, odd) : planes(r.x, r.y, odd), s, a));
-                };
-                const float2 tx0 = dist(xn, sx2, ax2), tx1 = dist(xf, sx2, ax2);
-                const float2 ty0 = dist(yn, sy2, ay2), ty1 = dist(yf, sy2, ay2);
-                const float2 tz0 = dist(zn, sz2, az2), tz1 = dist(zf, sz2, az2);
-                gap[odd].x = fminf(fminf(tx1.x, ty1.x), fminf(tz1.x, ray.tmax)) -
-                             fmaxf(fmaxf(tx0.x, ty0.x), fmaxf(tz0.x, ray.tmin));
-                gap[odd].y = fminf(fminf(tx1.y, ty1.y), fminf(tz1.y, ray.tmax)) -
-                             fmaxf(fmaxf(tx0.y, ty0.y), fmaxf(tz0.y, ray.tmin));
-            }
-            miss = __funnelshift_l(__float_as_uint(gap[1].y), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[0].y), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[1].x), miss, 1);
-            miss = __funnelshift_l(__float_as_uint(gap[0].x), miss, 1);
-        }
-        // internal children that were hit, and the triangles of the leaf children that were hit: each
-        // child's bit spread to three, one per triangle of a leaf (ascending bits are ascending slots)
-        const uint32_t vm = __float_as_uint(w1.z);   // 24 bits of triangles, 8 of internal children
-        const uint32_t hits = ~miss;
-        uint32_t leaf3 = hits & 0xFFu;
-        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
-        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
-        leaf3 = (leaf3 * 0x5u) & 0x249249u;
-        tvalid = vm & 0x00FFFFFFu;
-        tmask = (leaf3 * 7u) & tvalid;
-        tbase = __float_as_uint(w1.y);
-        ngroup = make_uint2(__float_as_uint(w1.x), ((hits << 24) & vm) | (vm >> 24));
+            if (COUNT) st.nodes++;
+            visit_node(sv.nodes, node, nr, ray.tmin, ray.tmax, ngroup, tmask, tvalid, tbase);
         }
     }
     if (ANY) return hit;
@@ -599,16 +553,10 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
     ray.tmax = not_neg0(ray.tmax);
     float det = 1.0f;
     uint2* const stack = reinterpret_cast<uint2*>(smem) + (threadIdx.x >> 3);
-    const uint32_t oct = (__float_as_uint(ray.d.x) >> 31) | ((__float_as_uint(ray.d.y) >> 31) << 1) |
-                         ((__float_as_uint(ray.d.z) >> 31) << 2);
-    const float3 idir = f3(safe_rcp(ray.d.x), safe_rcp(ray.d.y), safe_rcp(ray.d.z));
-    const float3 ood = f3(-ray.o.x * idir.x, -ray.o.y * idir.y, -ray.o.z * idir.z);
+    const NodeRay nr = node_ray(ray);
     // row of the near planes per axis, and the lane's word in it
     const uint32_t word = (sub >> 1) * 4u;
-    const uint32_t rowx = ((oct & 1u) ? 0x50u : 0x20u) + word, rowy = ((oct & 2u) ? 0x60u : 0x30u) + word,
-                   rowz = ((oct & 4u) ? 0x70u : 0x40u) + word;
-    const uint32_t pick2 = (oct & 4u) ? 0x0F000000u : 0xF0000000u, pick1 = (oct & 2u) ? 0x33000000u : 0xCC000000u,
-                   pick0 = (oct & 1u) ? 0x55000000u : 0xAA000000u;
+    const uint32_t rowx = nr.rowx + word, rowy = nr.rowy + word, rowz = nr.rowz + word;
     TShear shear = make_shear(ray.d);
     shear.ox = shear_proj(ray.o, shear.bx);
     shear.oy = shear_proj(ray.o, shear.by);
@@ -631,12 +579,12 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
                         zn = plane(rowz), zf = plane(rowz ^ 0x30u);
             if (COUNT) st.nodes += sub == 0;
             const uint32_t ew = __float_as_uint(w0.w);
-            const float sx = __uint_as_float(ew & 0x7F800000u) * idir.x;
-            const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * idir.y;
-            const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * idir.z;
-            const float ax = fmaf(-256.0f, sx, fmaf(w0.x, idir.x, ood.x));
-            const float ay = fmaf(-256.0f, sy, fmaf(w0.y, idir.y, ood.y));
-            const float az = fmaf(-256.0f, sz, fmaf(w0.z, idir.z, ood.z));
+            const float sx = __uint_as_float(ew & 0x7F800000u) * nr.idir.x;
+            const float sy = __uint_as_float((ew << 8) & 0x7F800000u) * nr.idir.y;
+            const float sz = __uint_as_float((ew << 16) & 0x7F800000u) * nr.idir.z;
+            const float ax = fmaf(-256.0f, sx, fmaf(w0.x, nr.idir.x, nr.ood.x));
+            const float ay = fmaf(-256.0f, sy, fmaf(w0.y, nr.idir.y, nr.ood.y));
+            const float az = fmaf(-256.0f, sz, fmaf(w0.z, nr.idir.z, nr.ood.z));
             const float gap = fminf(fminf(fmaf(xf, sx, ax), fmaf(yf, sy, ay)), fminf(fmaf(zf, sz, az), ray.tmax)) -
                               fmaxf(fmaxf(fmaf(xn, sx, ax), fmaf(yn, sy, ay)), fmaxf(fmaf(zn, sz, az), ray.tmin));
             in = !(__float_as_uint(gap) >> 31);
@@ -645,12 +593,8 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
             vm = __float_as_uint(w1.z);
         }
         const uint32_t hits = (__ballot_sync(ALL, in) >> oct0) & 0xFFu;
-        uint32_t leaf3 = hits;
-        leaf3 = (leaf3 * 0x101u) & 0x00F00Fu;
-        leaf3 = (leaf3 * 0x11u) & 0x0C30C3u;
-        leaf3 = (leaf3 * 0x5u) & 0x249249u;
         const uint32_t tvalid = vm & 0x00FFFFFFu;
-        uint32_t tmask = (leaf3 * 7u) & tvalid;
+        uint32_t tmask = leaf_bits(hits) & tvalid;
         // ---- next internal node (a nearer hit does not change which)
         uint2 group = make_uint2(cbase, ((hits << 24) & vm) | (vm >> 24));
         bool more = active;
@@ -660,15 +604,7 @@ __device__ __forceinline__ THit traverse_oct(const SceneView& sv, TRay ray, bool
         }
         __syncwarp();   // the entry has been read by the ray's lanes before it may be overwritten
         if (more) {
-            uint32_t cb = group.y & 0xFF000000u;
-            uint32_t pr = cb & pick2;
-            cb = pr ? pr : cb;
-            pr = cb & pick1;
-            cb = pr ? pr : cb;
-            pr = cb & pick0;
-            cb = pr ? pr : cb;
-            node = group.x + __popc(group.y & ((cb >> 24) - 1u));
-            group.y ^= cb;
+            node = next_child(group, nr);
             if (group.y > 0x00FFFFFFu) {
                 if (sp < CRT_STACK_TOTAL) {
                     if (sub == 0) stack[sp * OCT_RAYS] = group;
