@@ -1543,11 +1543,12 @@ struct WaveEngine {
     // of the same shape
     struct WaveGraph {
         int bounces, srp_nb;
-        const void *paths, *units, *bytes;
+        uint64_t layout;
         cudaGraphExec_t exec;
         uint64_t launches;
     };
     std::vector<WaveGraph> graphs;
+    uint64_t layout = 0;   // counts the allocations whose addresses a graph holds (a new one may get an old address)
 
     float4* pix() const { return (float4*)units_mem; }
     uint32_t* taken() const { return (uint32_t*)(units_mem + up256(units.cap() * 16)); }
@@ -1565,6 +1566,7 @@ void engine_alloc_units(WaveEngine* e, size_t cap) {
     e->units_mem = nullptr;
     e->units.reset(0);
     const size_t b = up256(cap * 16) + up256(cap * 4) + up256(cap);
+    ++e->layout;
     CRT_CUDA(cudaMalloc(&e->units_mem, b));
     e->units.reset(cap);
 }
@@ -1575,6 +1577,7 @@ void engine_alloc_bytes(WaveEngine* e, size_t cap) {
     e->bytes_mem = nullptr;
     e->bytes.reset(0);
     cap = up256(cap);
+    ++e->layout;
     CRT_CUDA(cudaMalloc(&e->bytes_mem, cap));
     e->bytes.reset(cap);
 }
@@ -1956,6 +1959,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
         if (e->paths) CRT_CUDA(cudaFree(e->paths));
         e->paths = nullptr;
         e->P = e->NL = 0;
+        ++e->layout;
         CRT_CUDA(cudaMalloc(&e->paths, WaveEngine::path_bytes(e->want_P, e->want_NL)));
         e->P = e->want_P;
         e->NL = e->want_NL;
@@ -2141,7 +2145,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
         WaveEngine::WaveGraph* g = nullptr;
         for (size_t k = 0; k < e->graphs.size();) {
             WaveEngine::WaveGraph& c = e->graphs[k];
-            if (c.paths != e->paths || c.units != e->units_mem || c.bytes != e->bytes_mem) {   // stale
+            if (c.layout != e->layout) {   // stale
                 cudaGraphExecDestroy(c.exec);
                 e->graphs.erase(e->graphs.begin() + (long)k);
                 continue;
@@ -2180,8 +2184,7 @@ void engine_step(WaveEngine* e, std::vector<uint64_t>& completed) {
             const cudaError_t ie = cudaGraphInstantiate(&ge, cg, 0);
             cudaGraphDestroy(cg);
             CRT_CUDA(ie);
-            e->graphs.push_back(WaveEngine::WaveGraph{max_bounces, srp_nb, e->paths, e->units_mem, e->bytes_mem, ge,
-                                                      ctx->launches - before});
+            e->graphs.push_back(WaveEngine::WaveGraph{max_bounces, srp_nb, e->layout, ge, ctx->launches - before});
             ctx->launches = before;
             g = &e->graphs.back();
         }
