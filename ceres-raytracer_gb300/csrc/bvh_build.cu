@@ -1025,10 +1025,9 @@ __global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, con
             q[3 + a] = 0u;
             if (!full) continue;
             const double iq = ldexp(1.0, -ex[a]);   // 1 / 2^ex, exact: the products equal the quotients
-            // an even child's planes read 0.71875 .. 0.75 quanta above the byte (WideNode)
             const bool even = !(sub & 1);
-            const double l = floor(((double)clo[a] - (double)p[a]) * iq - (even ? 1.75 : 1.0));
-            const double h = ceil(((double)chi[a] - (double)p[a]) * iq + (even ? 1.0 - 0.71875 : 1.0));
+            const double l = plane_below(((double)clo[a] - (double)p[a]) * iq, even);
+            const double h = plane_above(((double)chi[a] - (double)p[a]) * iq, even);
             if (l < 0 || h > 255) atomicOr(A.err, (uint32_t)DEVERR_QUANT_RANGE);
             q[a] = (uint32_t)fmax(0.0, fmin(255.0, l));
             q[3 + a] = (uint32_t)fmax(0.0, fmin(255.0, h));
@@ -1041,7 +1040,7 @@ __global__ void __launch_bounds__(COLLAPSE_BLOCK) k_collapse(CollapseArgs A, con
         };
         for (int r = 0; r < 6; ++r) {
             const uint32_t odd = __shfl_xor_sync(ALL, q[r], 1);
-            if (!(sub & 1)) put(2u + r, (uint32_t)sub >> 1, 0x43800000u | (q[r] << 15) | 0x5C00u | (odd << 2));
+            if (!(sub & 1)) put(2u + r, (uint32_t)sub >> 1, plane_word(q[r], odd));
         }
         const uint32_t eword = ((uint32_t)(ex[0] + 127) << 23) | ((uint32_t)(ex[1] + 127) << 15) |
                                ((uint32_t)(ex[2] + 127) << 7);

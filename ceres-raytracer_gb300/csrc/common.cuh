@@ -162,11 +162,18 @@ int crt_guard(crt_context* ctx, F&& f) {
 // node.  Spread over the banks: 12 % fewer data-pipe passes and 13 % less time on 3 M incoherent rays
 // (1742 -> 1519 us), 333 k any-hit rays 120 -> 105 us, a 2048^2 render 1625 -> 1554 us; the permutation
 // costs no instruction per row (the row's offset is xored to the address instead of added).
-// A leaf holds 1..3 triangles, stored contiguously from tri_base in slot order; internal children are stored contiguously from child_base in slot order; an empty slot has no bit and
-// its lo planes lie above its hi planes.
+// A leaf holds 1..3 triangles, stored contiguously from tri_base in slot order; internal children are stored
+// contiguously from child_base in slot order; an empty slot has no bit and its lo planes lie above its hi planes.
 struct WideNode {
     float4 w[8];
 };
+__host__ __device__ __forceinline__ uint32_t plane_word(uint32_t a, uint32_t b) {
+    return 0x43800000u | (a << 15) | 0x5C00u | (b << 2);
+}
+// The bytes of a child whose box side lies at x quanta: as the traversal reads them (an even child's 0.71875 ..
+// 0.75 above the byte), a lo plane one quantum or more below the side, a hi plane one or more above
+__host__ __device__ __forceinline__ double plane_below(double x, bool even) { return floor(x - (even ? 1.75 : 1.0)); }
+__host__ __device__ __forceinline__ double plane_above(double x, bool even) { return ceil(x + (even ? 1.0 - 0.71875 : 1.0)); }
 static_assert(sizeof(WideNode) == 128, "wide node must be 128 bytes");
 
 struct EntityDev {
@@ -332,7 +339,13 @@ inline FastDiv fast_div(uint32_t d) {
     if (d) f.m = (uint32_t)((((uint64_t)((1ull << f.s) - d)) << 32) / d) + 1u;
     return f;
 }
-__device__ __forceinline__ uint32_t div_by(uint32_t n, const FastDiv& f) { return (__umulhi(f.m, n) + n) >> f.s; }
+__host__ __device__ __forceinline__ uint32_t div_by(uint32_t n, const FastDiv& f) {
+#ifdef __CUDA_ARCH__
+    return (__umulhi(f.m, n) + n) >> f.s;
+#else
+    return ((uint32_t)((uint64_t)f.m * n >> 32) + n) >> f.s;
+#endif
+}
 
 // Pixel (px, py) of item i of a W x H grid in 8 x 4 tiles of 32 items (tiles: W / 8 rounded up); false outside.
 __device__ __forceinline__ bool tile_px(uint32_t i, const FastDiv& tiles, uint32_t W, uint32_t H, uint32_t& px, uint32_t& py) {
