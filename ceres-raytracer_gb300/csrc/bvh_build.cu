@@ -482,7 +482,7 @@ __device__ __forceinline__ void tl_better(float& best, uint32_t& bp, float c, ui
 }
 
 // One warp per treelet.  What bounds it: the chain of dependent loads that grows the treelet (each
-// opened node gives the next two boxes) and the dynamic program's 1,093 partitions, both of which one
+// opened node gives the next two boxes) and the dynamic program's 966 partitions, both of which one
 // lane walked before; now the leaves sit in lanes, and the partitions of a size are spread over lanes
 // (one lane a subset up to size 5, four lanes a subset of 6, all lanes for 7).  500 k triangles, seven
 // launches: 2516 -> 632 us.

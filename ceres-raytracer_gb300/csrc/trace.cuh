@@ -139,7 +139,8 @@ struct trace_oct<J, std::void_t<decltype(J::kOct)>> {
 
 // Jobs whose rays may be incoherent (kCoop) are traced with traverse_coop, unless the launch says that they
 // are not (first shadow rays: 2048^2 of them 3 % slower with it) or the scene is of fewer than SMALL_SCENE
-// triangles (a Cornell box's path-traced image: 563 us with it, 446 without).  A job over a buffer of rays
+// triangles (a Cornell box's path-traced image: 563 us with it, 446 without; few specular rays of a served wave do
+// not show it, srp_wave_stages_dev's caller in render.cu).  A job over a buffer of rays
 // (JobBase) asks per warp (rays_apart).  Camera, beam and sun rays are coherent.
 template <class J, class = void>
 struct trace_coop {

@@ -18,7 +18,8 @@
 // slot used per cycle on incoherent rays), so it runs as many warps as it can (8 blocks per SM, below).
 // Together, before / after: 3 M incoherent closest-hit rays on 2 M triangles 1942 / 1742 us, 333 k any-hit
 // rays on 100 k 125 / 120 us, a 1024^2 beam scan 236 / 211 us, a 2048^2 render 1860 / 1625 us, 12 x 2048^2
-// sun rays 3260 / 3070 us.
+// sun rays 3260 / 3070 us.  (Times of one workload differ between comments with the body's pose and the timing
+// loop; a pair is of one pose.)
 #pragma once
 
 #include "common.cuh"
@@ -310,7 +311,8 @@ __device__ __forceinline__ THit traverse(const SceneView& sv, TRay ray, unsigned
 // origins lie further apart than an eighth of the scene.  For buffers of rays, of which nothing is known:
 // with it 2048^2 camera rays in tiles take 3 - 6 % longer than in a kernel with traverse alone, against the 10
 // - 15 % (closest hits on 20 k / 500 k / 2 M triangles: 303 / 387 / 436 us alone, 314 / 399 / 449 with
-// both; any hits 213 / 272 / 329 and 228 / 288 / 347).
+// both; any hits 213 / 272 / 329 and 228 / 288 / 347).  Least is gained just above SMALL_SCENE: 45 k rays on
+// 1,100 triangles without / with both, random 28.7 / 26.9 us, coherent 21.9 / 23.1.
 __device__ __forceinline__ bool rays_apart(const SceneView& sv, const TRay& ray, bool active) {
     constexpr uint32_t ALL = 0xFFFFFFFFu;
     const uint32_t live = __ballot_sync(ALL, active);
@@ -509,7 +511,7 @@ __device__ __forceinline__ THit traverse_coop(const SceneView& sv, TRay ray, boo
                 else if (sp < CRT_STACK_TOTAL) lstack[sp - CRT_STACK_SMEM] = ngroup;
                 else {
                     // reported, so the call fails; the ray goes on without what its stack held (to end it here takes
-                    // a check after every visit, 0.4 % of 333 k any-hit rays)
+                    // a check after every visit, 0.4 - 0.9 % of 333 k any-hit rays)
                     atomicOr(err, (uint32_t)DEVERR_STACK_OVERFLOW);
                     sp = -1;
                 }

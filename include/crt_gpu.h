@@ -325,8 +325,7 @@ typedef struct {
  * beams (one shared ray queue), each wave carrying a range of one SRP request's items, and that
  * range's shade and specular segments follow in the same wave.  Render and LiDAR results equal
  * crt_batch's; force and torque equal crt_srp's bit for bit (partial sums are kept per block of the
- * request's items, whatever the waves).  Waves that carry SRP items are launched one by one (no
- * CUDA-graph replay). */
+ * request's items, whatever the waves). */
 int crt_batch_mixed(crt_context* ctx, const crt_server_request* requests, size_t n, crt_batch_stats* stats);
 
 typedef struct {
